@@ -13,6 +13,7 @@
 #include <chrono>
 #include <cmath>
 #include <cstdarg>
+#include <cstddef>
 #include <cstdio>
 #include <cstring>
 #include <map>
@@ -151,12 +152,32 @@ struct Arena {
 
 size_t al(size_t v) { return (v + 255) & ~(size_t)255; }
 
+}  // namespace
+
+// l = ceil(log2 d), mul = floor(2^32 (2^l - d) / d) + 1, shift = l - 1
+FastDiv make_fast_div(unsigned d) {
+  FastDiv f{0, 0};
+  if (d <= 1) return f;
+  unsigned l = 0;
+  while (l < 32 && (1ull << l) < d) l++;
+  f.mul = (unsigned)(((((1ull << l) - d) << 32) / d) + 1);
+  f.shift = l - 1;
+  return f;
+}
+
+namespace {
+
+// The first three members mirror the device block that one copy reads back.
 struct HostCounters {
   unsigned long long ctr[16];
-  unsigned err;
+  RoundCount rounds[AMS_ROUND_SLOTS];
+  unsigned err, pad;
+  int level[AMS_WIDE_LEVELS + 1];  // wide nodes per level, overflow flag
 };
 
 }  // namespace
+
+constexpr size_t kCounterBytes = offsetof(HostCounters, pad);
 
 struct ams_scene {
   int device = 0;
@@ -174,7 +195,10 @@ struct ams_scene {
   bool have_last = false;
   float ms_bvh_scene = 0.f;
   cudaEvent_t k2[2] = {nullptr, nullptr};
-  size_t tris_bytes = 0, mat_bytes = 0, mat_prop_bytes = 0, bvh_bytes = 0;
+  float *wide = nullptr;  // 32-wide nodes of bvh
+  float4 *attr = nullptr;  // trace_tri_attr
+  size_t tris_bytes = 0, mat_bytes = 0, mat_prop_bytes = 0, bvh_bytes = 0, wide_bytes = 0,
+         attr_bytes = 0;
   ~ams_scene() {
     for (auto &e : k2)
       if (e) cudaEventDestroy(e);
@@ -182,6 +206,8 @@ struct ams_scene {
     pool_free(mat, mat_bytes, device);
     pool_free(mat_prop, mat_prop_bytes, device);
     pool_free(bvh_out, bvh_bytes, device);
+    pool_free(wide, wide_bytes, device);
+    pool_free(attr, attr_bytes, device);
     pool_free_pinned(hc);
   }
 };
@@ -212,6 +238,36 @@ float elapsed_ms(cudaEvent_t a, cudaEvent_t b) {
 // elsewhere on this thread (its own launches are checked with
 // cudaGetLastError()).
 void clear_stale_error() { (void)cudaGetLastError(); }
+
+// The 32-wide form of the scene hierarchy for stage 2's beams.  The passes
+// that a balanced tree needs are enqueued at once, then the level counts are
+// read and any deeper level is added.  A hierarchy that does not fit the wide
+// nodes' memory goes without (stage 2 then traverses the binary nodes).
+cudaError_t build_wide(ams_scene *s, cudaStream_t st) {
+  const int n = s->n_tri;
+  s->wide_bytes = wide_bvh_bytes(n);
+  cudaError_t e = pool_malloc(reinterpret_cast<void **>(&s->wide), s->wide_bytes);
+  if (e != cudaSuccess) return e;
+  int levels = 2;
+  for (long long k = 32; k < n; k *= 16) levels++;
+  int *lv = s->hc->level, first = 0;
+  while (true) {
+    if ((e = wide_bvh_build(s->bvh, first, levels, s->wide, s->ws.base, st)) != cudaSuccess ||
+        (e = cudaMemcpyAsync(lv, s->ws.base, sizeof(s->hc->level), cudaMemcpyDeviceToHost, st)) !=
+            cudaSuccess ||
+        (e = cudaStreamSynchronize(st)) != cudaSuccess)
+      return e;
+    if (lv[AMS_WIDE_LEVELS]) return cudaSuccess;  // too many nodes
+    if (lv[levels] == 0) break;
+    if (levels >= AMS_WIDE_LEVELS - 1) return cudaSuccess;  // too deep
+    first = levels;
+    levels = std::min(levels + 4, AMS_WIDE_LEVELS - 1);
+  }
+  s->bvh.n_wide = 0;
+  for (int l = 0; l < levels; l++) s->bvh.n_wide += lv[l];
+  s->bvh.wide = s->wide;
+  return cudaSuccess;
+}
 }  // namespace
 
 extern "C" {
@@ -246,11 +302,13 @@ ams_status ams_scene_create(const float *tris, int n_tri, const int *mat, const 
   s->mat_bytes = sizeof(int) * (size_t)std::max(n_tri, 1);
   s->mat_prop_bytes = sizeof(float) * 19 * (size_t)std::max(n_mat, 1);
   s->bvh_bytes = lbvh_output_bytes(n_tri);
+  s->attr_bytes = 2 * sizeof(float4) * (size_t)std::max(n_tri, 1);
   if ((e = pool_malloc(reinterpret_cast<void **>(&s->tris), s->tris_bytes)) != cudaSuccess ||
       (e = pool_malloc(reinterpret_cast<void **>(&s->mat), s->mat_bytes)) != cudaSuccess ||
       (e = pool_malloc(reinterpret_cast<void **>(&s->mat_prop), s->mat_prop_bytes)) !=
           cudaSuccess ||
-      (e = pool_malloc(reinterpret_cast<void **>(&s->bvh_out), s->bvh_bytes)) != cudaSuccess) {
+      (e = pool_malloc(reinterpret_cast<void **>(&s->bvh_out), s->bvh_bytes)) != cudaSuccess ||
+      (e = pool_malloc(reinterpret_cast<void **>(&s->attr), s->attr_bytes)) != cudaSuccess) {
     set_err(errbuf, errlen, "scene allocation: %s", cudaGetErrorString(e));
     return fail(AMS_ERR_OOM);
   }
@@ -283,7 +341,8 @@ ams_status ams_scene_create(const float *tris, int n_tri, const int *mat, const 
     if ((e = cudaMemcpyAsync(s->tris, tris, sizeof(float) * 9 * (size_t)n_tri,
                              cudaMemcpyDeviceToDevice, st)) != cudaSuccess ||
         (e = cudaMemcpyAsync(s->mat, mat, sizeof(int) * (size_t)n_tri, cudaMemcpyDeviceToDevice,
-                             st)) != cudaSuccess) {
+                             st)) != cudaSuccess ||
+        (e = trace_tri_attr(s->tris, n_tri, s->attr, st)) != cudaSuccess) {
       set_err(errbuf, errlen, "copying the scene arrays: %s", cudaGetErrorString(e));
       return fail(AMS_ERR_CUDA);
     }
@@ -294,7 +353,8 @@ ams_status ams_scene_create(const float *tris, int n_tri, const int *mat, const 
     set_err(errbuf, errlen, "copying mat_prop: %s", cudaGetErrorString(e));
     return fail(AMS_ERR_CUDA);
   }
-  if ((e = s->ws.ensure(lbvh_scratch_bytes(n_tri) + 1024)) != cudaSuccess) {
+  if ((e = s->ws.ensure(std::max(lbvh_scratch_bytes(n_tri), wide_bvh_scratch_bytes(n_tri)) +
+                        1024)) != cudaSuccess) {
     set_err(errbuf, errlen, "BVH scratch: %s", cudaGetErrorString(e));
     return fail(AMS_ERR_OOM);
   }
@@ -320,6 +380,10 @@ ams_status ams_scene_create(const float *tris, int n_tri, const int *mat, const 
              (e = cudaStreamSynchronize(st)) != cudaSuccess) {
     set_err(errbuf, errlen, "triangle BVH build: %s", cudaGetErrorString(e));
     return fail(AMS_ERR_CUDA);
+  }
+  if (n_tri > 1 && (e = build_wide(s, st)) != cudaSuccess) {
+    set_err(errbuf, errlen, "wide triangle BVH build: %s", cudaGetErrorString(e));
+    return fail(e == cudaErrorMemoryAllocation ? AMS_ERR_OOM : AMS_ERR_CUDA);
   }
   s->ms_bvh_scene =
       std::chrono::duration<float, std::milli>(std::chrono::steady_clock::now() - t0).count();
@@ -402,7 +466,7 @@ ams_status trace_impl(ams_scene *S, const ams_trace_params *p, const float *src,
     need += 3 * al(4 * (size_t)ng * W);
     need += 2 * al(4 * ((size_t)ng + 1)) + al(4 * (size_t)ng) + 2 * al(4 * (size_t)tab_size);
     need += al(16 * (size_t)n_src * n_dst);
-    need += al(8 * 16) + al(4);
+    need += al(kCounterBytes) + al(4 * 16);
     need += 4096;
     CK(S->ws.ensure(need));
     S->ws.reset();
@@ -427,26 +491,41 @@ ams_status trace_impl(ams_scene *S, const ams_trace_params *p, const float *src,
     P.slot_of = S->ws.take<int>(tab_size);
     int *dense_of = S->ws.take<int>(tab_size);
     P.acc = S->ws.take<unsigned long long>(2 * (size_t)n_src * n_dst);
-    P.ctr = S->ws.take<unsigned long long>(16);
-    P.err = S->ws.take<unsigned>(1);
+    char *counters = S->ws.take<char>(kCounterBytes);
+    P.ctr = reinterpret_cast<unsigned long long *>(counters);
+    P.rounds = reinterpret_cast<RoundCount *>(counters + offsetof(HostCounters, rounds));
+    P.err = reinterpret_cast<unsigned *>(counters + offsetof(HostCounters, err));
+    P.round_slot = 0;
+    float *tx_info = S->ws.take<float>(16);
 
     if (!src_aabb) { CK(sphere_aabbs(src, n_src, p->src_r, sbox, st)); src_aabb = sbox; }
     if (!dst_aabb) { CK(sphere_aabbs(dst, n_dst, p->dst_r, dbox, st)); dst_aabb = dbox; }
     Lbvh tx, rx;
     CK(lbvh_build_spheres(tx, src, src_aabb, n_src, scratch, tx_out, st));
     CK(lbvh_build_spheres(rx, dst, dst_aabb, n_dst, scratch, rx_out, st));
+    CK(trace_tx_info(src, src_aabb, n_src, tx_info, st));
     CK(cudaEventRecord(ev[1], st));
 
     P.tris = S->tris;
     P.tri_nodes = S->bvh.nodes;
     P.tri_prims = S->bvh.prims;
     P.n_tri = S->n_tri;
+    P.tri_wide = S->bvh.wide;
+    P.n_tri_wide = S->bvh.n_wide;
+    P.tri_attr = S->attr;
     P.mat = S->mat;
     P.mat_prop = S->mat_prop;
     P.tx_nodes = tx.nodes; P.tx_prims = tx.prims; P.n_src = n_src; P.src = src; P.src_r = p->src_r;
+    P.src_aabb = src_aabb;
+    P.tx_info = reinterpret_cast<const float4 *>(tx_info);
     P.rx_nodes = rx.nodes; P.rx_prims = rx.prims; P.n_dst = n_dst; P.dst = dst; P.dst_r = p->dst_r;
     P.n0_dst = n0; P.n1_dst = n1; P.n0g = n0g; P.n1g = n1g; P.ng = ng; P.gs = gs;
     P.strict_grid = p->strict_grid;
+    P.s2_groups = (unsigned)(((long long)gs * gs * n_src + 31) / 32);
+    P.div_groups = make_fast_div(P.s2_groups);
+    P.div_src = make_fast_div((unsigned)n_src);
+    P.div_gs = make_fast_div((unsigned)gs);
+    P.div_n1g = make_fast_div((unsigned)n1g);
     P.L = p->max_reflection; P.reserve = p->reserve_size; P.spl = p->samples_per_launch;
     P.launch_x = p->launch_x; P.launch_y = p->launch_y;
     P.lam_f = (float)p->wave_len; P.lam_d = p->wave_len;
@@ -462,16 +541,17 @@ ams_status trace_impl(ams_scene *S, const ams_trace_params *p, const float *src,
     CK(cudaMemsetAsync(P.T, 0, 4 * (size_t)ng * W, st));
     CK(cudaMemsetAsync(P.S, 0, 4 * (size_t)ng * W, st));
     CK(cudaMemsetAsync(P.acc, 0, 16 * (size_t)n_src * n_dst, st));
-    CK(cudaMemsetAsync(P.ctr, 0, 8 * 16, st));
-    CK(cudaMemsetAsync(P.err, 0, 4, st));
+    CK(cudaMemsetAsync(counters, 0, kCounterBytes, st));
 
     // ---- stage 1
     CK(trace_stage1(P, st));
     CK(trace_count_bits(P, P.T, P.ctr + 6, st));
     CK(cudaEventRecord(ev[2], st));
-    CK(cudaMemcpyAsync(S->hc->ctr, P.ctr, 128, cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(&S->hc->err, P.err, 4, cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
+    auto read_counters = [&]() -> cudaError_t {
+      cudaError_t e = cudaMemcpyAsync(S->hc, counters, kCounterBytes, cudaMemcpyDeviceToHost, st);
+      return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
+    };
+    CK(read_counters());
     if (S->hc->err & AMS_DERR_PATH_TABLE) {
       if (S->tab_log2 >= 26) {
         set_err(errbuf, errlen, "path table would exceed 2^26 slots");
@@ -502,50 +582,84 @@ ams_status trace_impl(ams_scene *S, const ams_trace_params *p, const float *src,
       CK(cudaMemsetAsync(P.N, 0, 4 * dwords, st));
       CK(trace_dense_paths(P, P.T, W, dense_of, P.N, st));
       CK(cudaMemcpyAsync(P.T, P.N, 4 * dwords, cudaMemcpyDeviceToDevice, st));
-      CK(trace_count_tasks(P, P.N, st));
-      while (n_new > 0) {
-        // per task: its (path id, slot) and at most one chunk record
-        const size_t per_task = sizeof(int2) + sizeof(int4);
-        if (S->tasks.cap < n_new * per_task + 512) {
-          CK(cudaStreamSynchronize(st));
-          CK(S->tasks.ensure(std::max<size_t>(n_new * per_task * 2 + 512, 1 << 20)));
+      // two success bitmaps in turn (the dense ones fill half the memory)
+      P.S_next = P.S + dwords;
+      const size_t per_task = sizeof(int2) + sizeof(int4);
+      auto ensure_tasks = [&](unsigned long long n, unsigned long long want) -> cudaError_t {
+        if (S->tasks.cap < n * per_task + 512) {
+          cudaError_t e = cudaStreamSynchronize(st);
+          if (e == cudaSuccess)
+            e = S->tasks.ensure(std::max<size_t>(want * per_task + 512, (size_t)1 << 20));
+          if (e != cudaSuccess) return e;
         }
         P.task_cap = (S->tasks.cap - 512) / per_task;
         P.task_path = reinterpret_cast<int2 *>(S->tasks.base);
         P.chunk_at = reinterpret_cast<int4 *>(S->tasks.base + al(sizeof(int2) * P.task_cap));
-        P.kpi = records ? 1 : trace_paths_per_item(P, n_new);
-        CK(trace_make_tasks(P, P.N, st));
-        CK(cudaEventRecord(S->k2[0], st));
-        if (records) {
-          CK(trace_stage2_export(P, n_new, st));
-          P.rec_base += n_new * (unsigned long long)(gs * gs) * (unsigned long long)n_src;
+        return cudaSuccess;
+      };
+      // No round can list more than every path in every cell.  With memory
+      // for that, rounds whose stage 2 leaves the chip mostly idle run in
+      // batches without the host looking at their counts.
+      const unsigned long long most = (unsigned long long)ng * n_paths;
+      const bool batches = !records && most * per_task <= ((size_t)256 << 20);
+      constexpr int kBatch = 4;
+      if (batches) CK(ensure_tasks(most, most));
+      bool listed = false;
+      while (n_new > 0) {
+        if (listed && trace_round_is_small(P, n_new)) {
+          CK(cudaEventRecord(S->k2[0], st));
+          const unsigned first = P.round_slot;
+          for (int i = 0; i < kBatch; i++) {
+            CK(trace_stage2(P, 0, st));
+            P.round_slot++;
+            CK(trace_round(P, true, true, st));
+            std::swap(P.S, P.S_next);
+          }
+          CK(cudaEventRecord(S->k2[1], st));
+          CK(read_counters());
+          for (int i = 0; i < kBatch; i++) {
+            const unsigned long long n = S->hc->rounds[(first + i) & (AMS_ROUND_SLOTS - 1)].tasks;
+            if (i > 0 && n > 0) { rounds++; total_tasks += n; }
+          }
+          rounds++;
+          total_tasks += n_new;
         } else {
+          CK(ensure_tasks(n_new, 2 * n_new));
+          P.kpi = records || listed ? 1 : trace_paths_per_item(P, n_new);
+          if (records) CK(trace_list_ordered(P, st));
+          else if (!listed) CK(trace_round(P, false, true, st));
+          CK(cudaEventRecord(S->k2[0], st));
           CK(trace_stage2(P, n_new, st));
+          CK(cudaEventRecord(S->k2[1], st));
+          if (records)
+            P.rec_base += n_new * (unsigned long long)(gs * gs) * (unsigned long long)n_src;
+          rounds++;
+          total_tasks += n_new;
+          // a round of one path per item is followed by the next one's list at
+          // once; the others wait for its count to choose kpi
+          const unsigned slot = P.round_slot++;
+          const bool list = batches && P.kpi == 1;
+          CK(trace_round(P, true, list, st));
+          std::swap(P.S, P.S_next);
+          CK(read_counters());
+          if (!S->hc->err && !listed && S->hc->rounds[slot & (AMS_ROUND_SLOTS - 1)].listed != n_new) {
+            set_err(errbuf, errlen, "task count mismatch (%llu listed, %llu expected)",
+                    S->hc->rounds[slot & (AMS_ROUND_SLOTS - 1)].listed, n_new);
+            return AMS_ERR_INTERNAL;
+          }
+          listed = list;
         }
-        CK(cudaEventRecord(S->k2[1], st));
-        CK(trace_expand(P, st));
-        rounds++;
-        total_tasks += n_new;
-        CK(cudaMemcpyAsync(S->hc->ctr, P.ctr, 128, cudaMemcpyDeviceToHost, st));
-        CK(cudaMemcpyAsync(&S->hc->err, P.err, 4, cudaMemcpyDeviceToHost, st));
-        CK(cudaStreamSynchronize(st));
         if (S->hc->err) {
           set_err(errbuf, errlen, "stage 2 device error flags 0x%x", S->hc->err);
           return (S->hc->err & AMS_DERR_ACC_RANGE) ? AMS_ERR_NUMERIC : AMS_ERR_CAPACITY;
         }
         ms_k2 += elapsed_ms(S->k2[0], S->k2[1]);
-        if (S->hc->ctr[5] != n_new) {
-          set_err(errbuf, errlen, "task count mismatch (%llu listed, %llu expected)",
-                  S->hc->ctr[5], n_new);
-          return AMS_ERR_INTERNAL;
-        }
-        n_new = S->hc->ctr[7];
+        n_new = S->hc->rounds[P.round_slot & (AMS_ROUND_SLOTS - 1)].tasks;
       }
       CK(trace_finalize(P, result, st));
     }
     CK(cudaEventRecord(ev[3], st));
-    CK(cudaMemcpyAsync(S->hc->ctr, P.ctr, 128, cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
+    CK(read_counters());
     S->last = P;
     S->have_last = true;
     if (stats) {

@@ -16,6 +16,8 @@
 // four 16-byte loads), boxes widened outward so that node culling is
 // conservative.  Leaves hold one primitive; a child reference c < 0 is the
 // leaf of sorted primitive ~c.
+#include <algorithm>
+
 #include "ams_common.cuh"
 #include "lbvh.h"
 
@@ -312,9 +314,115 @@ __global__ void k_sphere_aabbs(const float *pos, int n, float r, float *aabb) {
   }
 }
 
+// One level of the collapse of a binary hierarchy into 32-wide nodes: a warp
+// per wide node.  The warp's list starts with the two children of the wide
+// node's binary root; every round replaces inner children by their own two
+// (all of them while they fit, else those with the largest surface) until the
+// list holds 32 or only leaves.  Wide nodes of level l + 1 are numbered after
+// those of level l through the level's counter.  Latency-bound (one dependent
+// node load per round, at most six full rounds).
+__global__ void __launch_bounds__(128) k_wide_pass(const BvhNode *nodes, int level, int cap,
+                                                   float *wide, int *src, int *cnt) {
+  __shared__ float box[4][6][32];
+  __shared__ int ref[4][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const unsigned lt = (1u << lane) - 1u;
+  int base = 0;
+  for (int l = 0; l < level; l++) base += cnt[l];
+  const int count = level == 0 ? 1 : cnt[level];
+  const int nbase = base + count;
+  if (nbase > cap) {  // a previous level did not fit
+    if (threadIdx.x == 0) cnt[AMS_WIDE_LEVELS] = 1;
+    return;
+  }
+  const int nwarp = (gridDim.x * blockDim.x) >> 5;
+  for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < count; i += nwarp) {
+    if (lane == 0) ref[w][0] = level == 0 ? 0 : src[base + i];
+    int c = 1;
+    __syncwarp();
+    while (true) {
+      const bool in = lane < c && ref[w][lane] >= 0;
+      const int ni = __popc(__ballot_sync(0xffffffffu, in)), room = 32 - c;
+      if (ni == 0 || room == 0) break;
+      bool ex = in;
+      if (ni > room) {  // only the largest fit
+        const float dx = box[w][1][lane] - box[w][0][lane], dy = box[w][3][lane] - box[w][2][lane],
+                    dz = box[w][5][lane] - box[w][4][lane];
+        const float area = in ? dx * dy + dy * dz + dz * dx : -1.0f;
+        int rank = 0;
+        for (int k = 0; k < 32; k++) {
+          const float o = __shfl_sync(0xffffffffu, area, k);
+          rank += (o > area || (o == area && k < lane)) ? 1 : 0;
+        }
+        ex = in && rank < room;
+      }
+      const unsigned me = __ballot_sync(0xffffffffu, ex);
+      const int at = c + __popc(me & lt);
+      const int node = ex ? ref[w][lane] : 0;
+      __syncwarp();
+      if (ex) {
+        const BvhNode nd = nodes[node];
+        box[w][0][lane] = nd.a.x; box[w][2][lane] = nd.a.y; box[w][4][lane] = nd.a.z;
+        box[w][1][lane] = nd.a.w; box[w][3][lane] = nd.b.x; box[w][5][lane] = nd.b.y;
+        box[w][0][at] = nd.b.z; box[w][2][at] = nd.b.w; box[w][4][at] = nd.c.x;
+        box[w][1][at] = nd.c.y; box[w][3][at] = nd.c.z; box[w][5][at] = nd.c.w;
+        ref[w][lane] = nd.d.x;
+        ref[w][at] = nd.d.y;
+      }
+      c += __popc(me);
+      __syncwarp();
+    }
+    const bool used = lane < c, inner = used && ref[w][lane] >= 0;
+    const unsigned mi = __ballot_sync(0xffffffffu, inner);
+    int first = 0;
+    if (lane == 0 && mi) first = nbase + atomicAdd(cnt + level + 1, __popc(mi));
+    first = __shfl_sync(0xffffffffu, first, 0);
+    const int id = first + __popc(mi & lt);
+    const bool fits = first + __popc(mi) <= cap;
+    if (!fits && lane == 0) cnt[AMS_WIDE_LEVELS] = 1;  // the caller drops the wide form
+    if (inner && fits) src[id] = ref[w][lane];
+    float *out = wide + (size_t)(base + i) * AMS_WIDE_WORDS + lane;
+#pragma unroll
+    for (int k = 0; k < 6; k++)
+      out[32 * k] = used ? box[w][k][lane] : ((k & 1) ? -3.0e38f : 3.0e38f);
+    reinterpret_cast<int *>(out)[32 * 6] =
+        !used ? (int)0x80000000 : (inner ? (fits ? id : (int)0x80000000) : ref[w][lane]);
+    __syncwarp();
+  }
+}
+
 inline int nblk(int n, int b) { return (n + b - 1) / b; }
 
 }  // namespace
+
+// A wide node with inner children is full, so the number of wide nodes is
+// at most n / 2 (every bottom node holding two leaves); a third covers any
+// hierarchy met in practice, and beyond it the wide form is not used.
+int wide_bvh_cap(int n) { return n / 3 + 64; }
+size_t wide_bvh_bytes(int n) {
+  return sizeof(float) * AMS_WIDE_WORDS * (size_t)wide_bvh_cap(n);
+}
+size_t wide_bvh_scratch_bytes(int n) {
+  return sizeof(int) * ((size_t)wide_bvh_cap(n) + AMS_WIDE_LEVELS + 1);
+}
+cudaError_t wide_bvh_build(const Lbvh &b, int first, int last, float *wide, char *scratch,
+                           cudaStream_t st) {
+  int *cnt = reinterpret_cast<int *>(scratch), *src = cnt + AMS_WIDE_LEVELS + 1;
+  if (first == 0) {
+    // level 0 is the root alone; its count is 1
+    cudaError_t e = cudaMemsetAsync(cnt, 0, sizeof(int) * (AMS_WIDE_LEVELS + 1), st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(cnt, 1, 1, st);  // little-endian int 1
+    if (e != cudaSuccess) return e;
+  }
+  const int cap = wide_bvh_cap(b.n);
+  for (int l = first; l < last && l < AMS_WIDE_LEVELS - 1; l++) {
+    // level l has at most 32^l nodes
+    const long long most = l < 4 ? (1ll << (5 * l)) : (1ll << 20);
+    const int blocks = (int)std::min<long long>((std::min<long long>(most, cap) + 3) / 4, 1216);
+    k_wide_pass<<<blocks, 128, 0, st>>>(b.nodes, l, cap, wide, src, cnt);
+  }
+  return cudaGetLastError();
+}
 
 size_t lbvh_scratch_bytes(int n) {
   size_t s = 0;

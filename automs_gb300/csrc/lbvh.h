@@ -15,7 +15,25 @@ struct Lbvh {
   BvhNode *nodes = nullptr;  // n-1 internal nodes, root = 0
   int *perm = nullptr;     // sorted position -> original primitive index
   float4 *prims = nullptr; // 3 float4 per sorted primitive (see lbvh.cu)
+  const float *wide = nullptr;  // 32-wide nodes (wide_bvh_build), root = 0
+  int n_wide = 0;
 };
+
+// 32-wide form of a binary hierarchy, one node per warp-wide visit: six
+// planes of 32 floats (lo.x, hi.x, lo.y, hi.y, lo.z, hi.z of each child) and
+// 32 child references (>= 0 wide node, < 0 leaf of sorted primitive ~c; an
+// unused slot has an inverted box).
+#define AMS_WIDE_WORDS (7 * 32)
+#define AMS_WIDE_LEVELS 64
+// device memory of the wide nodes of n primitives and of their build
+size_t wide_bvh_bytes(int n);
+size_t wide_bvh_scratch_bytes(int n);
+// enqueue the passes first .. last - 1 (one per level) of the collapse of
+// `b`; scratch starts with AMS_WIDE_LEVELS + 1 node counts (per level, then an
+// overflow flag), which the caller reads back to see whether a level is left
+cudaError_t wide_bvh_build(const Lbvh &b, int first, int last, float *wide, char *scratch,
+                           cudaStream_t st);
+int wide_bvh_cap(int n);
 
 size_t lbvh_scratch_bytes(int n);
 size_t lbvh_output_bytes(int n);

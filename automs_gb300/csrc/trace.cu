@@ -21,6 +21,8 @@
 //     bit-reproducible whatever the launch order.
 //   * this file is compiled with -fmad=false: the float arithmetic of every
 //     decision matches the CPU oracle bit for bit.
+#include <algorithm>
+
 #include "ams_common.cuh"
 #include "trace.h"
 
@@ -34,11 +36,20 @@ __constant__ unsigned c_theta_thr_bits[18] = {
     0x3f57e880u, 0x3f4b1934u, 0x3f3cbe35u, 0x3f2cf37au, 0x3f1bd7c9u, 0x3f098c77u,
     0x3eec6a50u, 0x3ec3ef15u, 0x3e99f61cu, 0x3e5da258u, 0x3e05a8a8u, 0x3d32aa3eu};
 
+// The bin of |c| is the number of edges not below it.  An estimate of the
+// angle (Abramowitz and Stegun 4.4.45, error below 7e-5 rad) gives the bin to
+// within one, and the exact edges on both sides of it decide.
 __device__ __forceinline__ int theta_id(float c) {
-  float a = fabsf(c);
-  int id = 0;
-#pragma unroll
-  for (int k = 0; k < 18; k++) id += (a <= __uint_as_float(c_theta_thr_bits[k])) ? 1 : 0;
+  const float a = fabsf(c);
+  const float x = fminf(a, 1.0f);
+  const float p = __fmaf_rn(x, __fmaf_rn(x, __fmaf_rn(x, -0.0187293f, 0.0742610f), -0.2121144f),
+                            1.5707288f);
+  const float th = __fsqrt_rn(1.0f - x) * p;  // acos
+  // edges lie at (2k - 1) pi / 72, bins are 5 degrees wide
+  int id = (int)__fmaf_rn(th, 36.0f / AMS_PIF, 0.5f);
+  id = max(0, min(18, id));
+  if (id > 0 && !(a <= __uint_as_float(c_theta_thr_bits[id - 1]))) id--;
+  else if (id < 18 && a <= __uint_as_float(c_theta_thr_bits[id])) id++;
   return id;
 }
 
@@ -111,9 +122,9 @@ __device__ __forceinline__ af3 rand_dir(uint32_t &seed, uint32_t ix, uint32_t iy
 // get_beampattern_factor, optixPathTracer.cu:107-136; branches on the float
 // cosine against cos(120 deg) and cos(75 deg), taper value in float.
 __device__ __forceinline__ float beampattern(af3 d1, af3 d2, int type) {
+  if (type == 0) return 1.0f;
   float c = dot3(d1, d2) / (len3(d1) * len3(d2));
   switch (type) {
-    case 0: return 1.0f;
     case 1: return c < 0.0f ? 0.0f : c * 2.4495f;
     case 2: {
       if ((double)c < -0.5) return 0.1f;
@@ -138,21 +149,10 @@ struct RayT {
   float Sx, Sy, Sz;
 };
 
-__device__ __forceinline__ void ray_setup(RayT &r, af3 o, af3 d) {
+// what the triangle test needs: the dominant axis and the shear
+__device__ __forceinline__ void ray_setup_tri(RayT &r, af3 o, af3 d) {
   r.o = o;
   r.d = d;
-  // The fused node test computes lo * inv - o * inv.  For an axis-parallel
-  // ray (a zero direction component) an infinite inverse would give
-  // inf - inf = NaN, or -inf for a box that reaches below 0, and cull nodes
-  // the ray is inside of.  The clamp keeps every term finite; node boxes are
-  // widened far beyond its rounding error.  prim_slab recovers the exact
-  // inverse where the clamp applies.
-  const float big = 1e30f;
-  r.inv = mk3(fminf(fmaxf(1.0f / d.x, -big), big), fminf(fmaxf(1.0f / d.y, -big), big),
-              fminf(fmaxf(1.0f / d.z, -big), big));
-  r.oix = o.x * r.inv.x;
-  r.oiy = o.y * r.inv.y;
-  r.oiz = o.z * r.inv.z;
   float ax = fabsf(d.x), ay = fabsf(d.y), az = fabsf(d.z);
   int kz = (ax > ay) ? ((ax > az) ? 0 : 2) : ((ay > az) ? 1 : 2);
   int kx = kz + 1; if (kx == 3) kx = 0;
@@ -163,6 +163,25 @@ __device__ __forceinline__ void ray_setup(RayT &r, af3 o, af3 d) {
   r.Sx = comp3(d, kx) / dz;
   r.Sy = comp3(d, ky) / dz;
   r.Sz = 1.0f / dz;
+}
+// what the box tests need (r.o and r.d are set)
+__device__ __forceinline__ void ray_setup_box(RayT &r) {
+  // The fused node test computes lo * inv - o * inv.  For an axis-parallel
+  // ray (a zero direction component) an infinite inverse would give
+  // inf - inf = NaN, or -inf for a box that reaches below 0, and cull nodes
+  // the ray is inside of.  The clamp keeps every term finite; node boxes are
+  // widened far beyond its rounding error.  prim_slab recovers the exact
+  // inverse where the clamp applies.
+  const float big = 1e30f;
+  r.inv = mk3(fminf(fmaxf(1.0f / r.d.x, -big), big), fminf(fmaxf(1.0f / r.d.y, -big), big),
+              fminf(fmaxf(1.0f / r.d.z, -big), big));
+  r.oix = r.o.x * r.inv.x;
+  r.oiy = r.o.y * r.inv.y;
+  r.oiz = r.o.z * r.inv.z;
+}
+__device__ __forceinline__ void ray_setup(RayT &r, af3 o, af3 d) {
+  ray_setup_tri(r, o, d);
+  ray_setup_box(r);
 }
 
 // Watertight ray/triangle test (Woop, Benthin, Wald, JCGT 2(1) 2013).
@@ -326,22 +345,325 @@ __device__ void traverse(const BvhNode *nodes, const float4 *prims, int n, const
   }
 }
 
-// Backward-ray query of stage 2: optixTrace with the visibility mask of the
-// scene and the Tx spheres (optixPathTracer.cpp:417-424).  On a path's last
-// segment the Tx sphere is the expected hit: finding it first bounds the
-// scene traversal to the segment before it instead of the wall behind the
-// Tx.  Other segments end on a triangle, so the scene goes first there.  The
-// result is the same lexicographic minimum in either order.
-__device__ __forceinline__ Hit closest_s2(const TraceDev &P, af3 o, af3 d, bool last) {
+// ------------------------------------------------------------------ beams
+// Stage 2 traces the rays of a warp together: from one Rx (or two
+// neighbours) to the images of neighbouring Tx elements, so they differ by
+// millimetres to centimetres.  A beam bounds them: at parameter t every
+// active ray lies in the box [omin + t dmin, omax + t dmax].  The 32 lanes
+// test the 32 children of one wide node against the beam at once, and each
+// triangle that survives is tested exactly by every lane's own ray, nearest
+// box first.  The closest hit is the lexicographic minimum over (t, instance,
+// primitive) of exact tests, so it is the one that a traversal ray by ray
+// finds; only the culling is shared.  Ray by ray, a query made 14 (2,172
+// triangles) to 25 dependent visits of binary nodes; a beam makes 2.6 to 6.5
+// visits of wide nodes and 4 to 5 triangle tests for 27 to 32 rays.  Stage-2
+// kernels: 3.05 -> 2.6 ms on coverage-128, 42 -> 33 ms on a 62k-triangle room
+// with 256 x 256 Rx, 90 -> 44 ms with 1,024 metasurface elements as Tx.
+// Bound by instruction issue (66% of the slots) and instruction fetch.
+constexpr unsigned kFullWarp = 0xffffffffu;
+
+// n / d by the multiplier of make_fast_div (Granlund and Montgomery 1994)
+__device__ __forceinline__ unsigned fdiv(unsigned n, const FastDiv &f) {
+  if (f.mul == 0u) return n;  // d = 1
+  const unsigned q = __umulhi(n, f.mul);
+  return (((n - q) >> 1) + q) >> f.shift;
+}
+__device__ __forceinline__ float warp_min(float v) {
+  float r;
+  asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
+}
+__device__ __forceinline__ float warp_max(float v) {
+  float r;
+  asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
+}
+
+struct BeamAxis { float o1, i1, o2, i2; };  // bounds on t from the near and the far box plane
+struct Beam {
+  BeamAxis x, y, z;
+  // per axis k: bit k, directions negative (the hi plane is the near one);
+  // bit 8 + k, directions of both signs (both planes bound t from below)
+  unsigned flags;
+  float spread;  // largest extent of the directions along an axis
+};
+
+// rcp.approx keeps the error (1 ulp) far inside the slack of the box test;
+// the clamp as in ray_setup_box
+__device__ __forceinline__ float beam_inv(float d) {
+  return fminf(fmaxf(__fdividef(1.0f, d), -1e30f), 1e30f);
+}
+__device__ __forceinline__ BeamAxis beam_axis(float o, float d, bool on, int axis, Beam &b) {
+  const float inf = 3.0e38f;
+  const float omin = warp_min(on ? o : inf), omax = warp_max(on ? o : -inf);
+  const float dmin = warp_min(on ? d : inf), dmax = warp_max(on ? d : -inf);
+  // hi plane: omin + t dmin <= hi; lo plane: omax + t dmax >= lo.  A positive
+  // dmin bounds t above by the first, a negative one below; and so on.
+  const float ihi = dmin == 0.0f ? 1e30f : beam_inv(dmin);
+  const float ilo = dmax == 0.0f ? (dmin < 0.0f ? -1e30f : 1e30f) : beam_inv(dmax);
+  BeamAxis a;
+  const bool neg = dmax <= 0.0f && dmin < 0.0f;
+  if (neg) b.flags |= 1u << axis;
+  if (dmin < 0.0f && dmax > 0.0f) b.flags |= 256u << axis;
+  b.spread = fmaxf(b.spread, dmax - dmin);
+  a.o1 = neg ? omin : omax; a.i1 = neg ? ihi : ilo;
+  a.o2 = neg ? omax : omin; a.i2 = neg ? ilo : ihi;
+  return a;
+}
+// bounds of the rays of the lanes with `on` (at least one)
+__device__ __forceinline__ Beam beam_of(af3 o, af3 d, bool on) {
+  Beam b;
+  b.flags = 0u;
+  b.spread = 0.0f;
+  b.x = beam_axis(o.x, d.x, on, 0, b);
+  b.y = beam_axis(o.y, d.y, on, 1, b);
+  b.z = beam_axis(o.z, d.z, on, 2, b);
+  return b;
+}
+__device__ __forceinline__ void beam_slab(const BeamAxis &a, bool mixed, float v1, float v2,
+                                          float &tn, float &tf) {
+  const float t1 = (v1 - a.o1) * a.i1, t2 = (v2 - a.o2) * a.i2;
+  tn = fmaxf(tn, mixed ? fmaxf(t1, t2) : t1);
+  tf = fminf(tf, mixed ? 3.0e38f : t2);
+}
+// the slack of child_test, which covers the same rounding
+__device__ __forceinline__ bool beam_in(float tn, float tf, float lim) {
+  return tn <= __fmaf_rn(tf, 1.0001f, 1e-5f) && tf >= -1e-5f && tn <= lim;
+}
+__device__ __forceinline__ float beam_limit(float best) { return __fmaf_rn(best, 1.0001f, 1e-4f); }
+
+// A lane's ray for the triangle tests of a beam: origin and shear in the
+// order (kx, ky, kz) of its dominant axis (ray_setup_tri), so that a test
+// reads the vertices' components in that order and selects nothing.
+struct RayB { float ox, oy, oz, Sx, Sy, Sz; int kx, ky, kz; };
+__device__ __forceinline__ RayB ray_b(af3 o, af3 d) {
+  RayT r;
+  ray_setup_tri(r, o, d);
+  RayB b;
+  b.kx = r.kx; b.ky = r.ky; b.kz = r.kz;
+  b.Sx = r.Sx; b.Sy = r.Sy; b.Sz = r.Sz;
+  b.ox = comp3(o, r.kx); b.oy = comp3(o, r.ky); b.oz = comp3(o, r.kz);
+  return b;
+}
+// tri_hit on packed triangle p (v0, index, v1, -, v2, -), the same operations
+__device__ __forceinline__ float tri_hit_b(const RayB &r, const float *p) {
+  const float *px = p + r.kx, *py = p + r.ky, *pz = p + r.kz;
+  const float Az_ = __ldg(pz) - r.oz, Bz_ = __ldg(pz + 4) - r.oz, Cz_ = __ldg(pz + 8) - r.oz;
+  const float Ax = (__ldg(px) - r.ox) - r.Sx * Az_, Ay = (__ldg(py) - r.oy) - r.Sy * Az_;
+  const float Bx = (__ldg(px + 4) - r.ox) - r.Sx * Bz_, By = (__ldg(py + 4) - r.oy) - r.Sy * Bz_;
+  const float Cx = (__ldg(px + 8) - r.ox) - r.Sx * Cz_, Cy = (__ldg(py + 8) - r.oy) - r.Sy * Cz_;
+  float U = Cx * By - Cy * Bx;
+  float V = Ax * Cy - Ay * Cx;
+  float W = Bx * Ay - By * Ax;
+  if (U == 0.0f || V == 0.0f || W == 0.0f) {
+    U = (float)((double)Cx * (double)By - (double)Cy * (double)Bx);
+    V = (float)((double)Ax * (double)Cy - (double)Ay * (double)Cx);
+    W = (float)((double)Bx * (double)Ay - (double)By * (double)Ax);
+  }
+  if ((U < 0.0f || V < 0.0f || W < 0.0f) && (U > 0.0f || V > 0.0f || W > 0.0f)) return -1.0f;
+  const float det = U + V + W;
+  if (det == 0.0f) return -1.0f;
+  const float Az = r.Sz * Az_, Bz = r.Sz * Bz_, Cz = r.Sz * Cz_;
+  const float T = U * Az + V * Bz + W * Cz;
+  return T / det;
+}
+
+// Wide-node stack of a warp: child reference and near distance (bits).
+#define AMS_BEAM_STACK 96
+// node visits + triangle tests after which a beam is given up; its lanes then
+// traverse the binary nodes one ray each
+#define AMS_BEAM_WORK 64
+// Directions further apart than this along an axis (rays that met different
+// surfaces) are taken as several beams of closer ones.
+#define AMS_BEAM_SPREAD 0.1f
+
+// Closest scene hit of every alive lane's ray, or with `any` whether there is
+// one at all before `best` (such a lane's `alive` becomes false).  Warp
+// collective; returns false when the beam was given up or the stack is full,
+// with `best` holding only hits that exist.
+__device__ __forceinline__ bool beam_scene(const TraceDev &P, const Beam &bm, const RayB &r,
+                                           Hit &best, bool &alive, bool any, int2 *stk) {
+  const int lane = threadIdx.x & 31;
+  int sp = 0, node = 0, work = 0;
+  float lim = beam_limit(warp_max(alive ? best.t : 0.0f));
+  while (true) {
+    if ((unsigned)node >= (unsigned)P.n_tri_wide) {
+      if (lane == 0) atomicOr(P.err, AMS_DERR_BVH);
+      return true;
+    }
+    const float *nd = P.tri_wide + (size_t)node * AMS_WIDE_WORDS + lane;
+    const int px = (bm.flags & 1u) << 5, py = (bm.flags & 2u) << 4, pz = (bm.flags & 4u) << 3;
+    const float x1 = __ldg(nd + px), x2 = __ldg(nd + (px ^ 32)), y1 = __ldg(nd + 64 + py),
+                y2 = __ldg(nd + 64 + (py ^ 32)), z1 = __ldg(nd + 128 + pz),
+                z2 = __ldg(nd + 128 + (pz ^ 32));
+    const int child = __float_as_int(__ldg(nd + 192));
+    float tn = -3.0e38f, tf = 3.0e38f;
+    beam_slab(bm.x, bm.flags & 256u, x1, x2, tn, tf);
+    beam_slab(bm.y, bm.flags & 512u, y1, y2, tn, tf);
+    beam_slab(bm.z, bm.flags & 1024u, z1, z2, tn, tf);
+    bool hit = beam_in(tn, tf, lim);
+    // near distance in the high bits, lane in the low five: the order of
+    // non-negative floats is that of their bits
+    const unsigned key = (__float_as_uint(fmaxf(tn, 0.0f)) & ~31u) | (unsigned)lane;
+    unsigned lk = hit && child < 0 ? key : 0xffffffffu;
+    while (true) {
+      const unsigned k = __reduce_min_sync(kFullWarp, lk);
+      if (k == 0xffffffffu || __uint_as_float(k & ~31u) > lim) break;
+      const int j = ~__shfl_sync(kFullWarp, child, (int)(k & 31u));
+      if ((unsigned)j >= (unsigned)P.n_tri) {
+        if (lane == 0) atomicOr(P.err, AMS_DERR_BVH);
+        return true;
+      }
+      bool closer = false;
+      if (alive) {
+        const float *pj = reinterpret_cast<const float *>(P.tri_prims + 3 * (size_t)j);
+        const float t = tri_hit_b(r, pj);
+        if (t > AMS_TMIN && t < AMS_TMAX && t <= best.t) {
+          const int orig = __float_as_int(__ldg(pj + 3));
+          closer = better(t, 0, orig, best);
+          if (closer) { best.t = t; best.inst = 0; best.prim = orig; alive = !any; }
+        }
+      }
+      if (__any_sync(kFullWarp, closer)) {
+        if (any && !__any_sync(kFullWarp, alive)) return true;
+        lim = beam_limit(warp_max(alive ? best.t : 0.0f));
+      }
+      if (lk == k) lk = 0xffffffffu;
+      work++;
+    }
+    hit = hit && child >= 0 && tn <= lim;
+    const unsigned m = __ballot_sync(kFullWarp, hit);
+    if (m) {
+      // the nearest child next, the others on the stack, nearer ones on top
+      int rank = 0;
+      if (m & (m - 1u)) {
+#pragma unroll 1
+        for (unsigned q = m; q; q &= q - 1u)
+          rank += __shfl_sync(kFullWarp, key, __ffs(q) - 1) < key ? 1 : 0;
+      }
+      const int more = __popc(m) - 1;
+      if (sp + more > AMS_BEAM_STACK) return false;
+      if (hit && rank > 0) stk[sp + more - rank] = make_int2(child, (int)(key & ~31u));
+      node = __shfl_sync(kFullWarp, child, __ffs(__ballot_sync(kFullWarp, hit && rank == 0)) - 1);
+      sp += more;
+      __syncwarp();
+    } else {
+      bool found = false;
+      while (sp > 0 && !found) {
+        const int2 e = stk[--sp];
+        found = __int_as_float(e.y) <= lim;
+        node = e.x;
+      }
+      __syncwarp();
+      if (!found) return true;
+    }
+    if (++work > AMS_BEAM_WORK) return false;
+  }
+}
+
+// whether a ray (r.inv set) meets the box of the whole Tx array, or with a
+// beam whether any of its rays may (tx_info words 8-10 and 12-14)
+__device__ __forceinline__ bool beam_near_tx(const TraceDev &P, const Beam &bm) {
+  const float4 lo = __ldg(P.tx_info + 2), hi = __ldg(P.tx_info + 3);
+  const bool nx = bm.flags & 1u, ny = bm.flags & 2u, nz = bm.flags & 4u;
+  float tn = -3.0e38f, tf = 3.0e38f;
+  beam_slab(bm.x, bm.flags & 256u, nx ? hi.x : lo.x, nx ? lo.x : hi.x, tn, tf);
+  beam_slab(bm.y, bm.flags & 512u, ny ? hi.y : lo.y, ny ? lo.y : hi.y, tn, tf);
+  beam_slab(bm.z, bm.flags & 1024u, nz ? hi.z : lo.z, nz ? lo.z : hi.z, tn, tf);
+  return beam_in(tn, tf, 3.0e38f);
+}
+__device__ __forceinline__ bool ray_near_tx(const TraceDev &P, const RayT &r) {
+  const float4 lo = __ldg(P.tx_info + 2), hi = __ldg(P.tx_info + 3);
+  float tn;
+  return child_test(r, lo.x, lo.y, lo.z, hi.x, hi.y, hi.z, AMS_TMAX, tn);
+}
+// The Tx spheres that a ray can meet besides the one it meets, without asking
+// the hierarchy.  A ray through the boxes of two Tx is nearly parallel to the
+// line between them, so one steep enough to the plane (or the line) of the
+// array meets only one: |D . n| > (eta + 2 rho) / (delta - 2 rho), with eta
+// the array's extent along n, rho the boxes' radius and delta the smallest
+// distance of two Tx (k_tx_info).
+__device__ __forceinline__ bool tx_alone(const TraceDev &P, af3 D) {
+  const float4 a = __ldg(P.tx_info), b = __ldg(P.tx_info + 1);
+  return fabsf(dot3(D, mk3(a.x, a.y, a.z))) > a.w || fabsf(dot3(D, mk3(b.x, b.y, b.z))) > b.w;
+}
+
+// the paths that are rarely taken, out of line: their code would push the
+// beam loop out of the instruction cache
+__device__ __noinline__ Hit traverse_tx(const TraceDev &P, af3 o, af3 d, Hit h) {
   RayT r;
   ray_setup(r, o, d);
+  traverse<1>(P.tx_nodes, P.tx_prims, P.n_src, r, h, P.src_r, P.err);
+  return h;
+}
+__device__ __noinline__ Hit traverse_scene(const TraceDev &P, af3 o, af3 d, Hit h) {
+  RayT r;
+  ray_setup(r, o, d);
+  traverse<0>(P.tri_nodes, P.tri_prims, P.n_tri, r, h, 0.0f, P.err);
+  return h;
+}
+
+// Backward-ray query of stage 2 for a warp: optixTrace with the visibility
+// mask of the scene and the Tx spheres (optixPathTracer.cpp:417-424), from
+// (o, d) of the lanes with `on` towards Tx s.  On a path's last segment a
+// triangle ends the ray wherever it is (optixPathTracer.cu:336-417), so there
+// the Tx spheres come first, Tx s itself before the others; a ray that meets
+// none has ended, and the scene is asked only for something in front of the
+// Tx hit.  Elsewhere the scene comes first.  Returns the closest hit; on the
+// last segment the triangle of an inst = 0 hit is any one in front, and
+// inst = 3 may stand for a triangle behind no Tx.
+__device__ __forceinline__ Hit closest_s2(const TraceDev &P, af3 o, af3 d, int s, bool last,
+                                          bool on, int2 *stk) {
   Hit h;
   h.t = AMS_TMAX; h.inst = 3; h.prim = 0x7fffffff;
-#pragma unroll 1
-  for (int ph = 0; ph < 2; ph++) {
-    if ((ph == 0) == last) traverse<1>(P.tx_nodes, P.tx_prims, P.n_src, r, h, P.src_r, P.err);
-    else traverse<0>(P.tri_nodes, P.tri_prims, P.n_tri, r, h, 0.0f, P.err);
+  if (last) {
+    bool others = false;
+    if (on) {
+      RayT r;
+      r.o = o;
+      r.d = d;
+      ray_setup_box(r);
+      const float *bx = P.src_aabb + 6 * (size_t)s;
+      const float4 lo = make_float4(__ldg(bx), __ldg(bx + 1), __ldg(bx + 2), 0.f),
+                   hi = make_float4(__ldg(bx + 3), __ldg(bx + 4), __ldg(bx + 5), 0.f);
+      if (prim_slab(r, lo, hi)) {
+        const af3 D = unit_dir(r);
+        const float t = sphere_hit(r, D, ld3(P.src + 3 * (size_t)s), P.src_r);
+        if (t >= 0.0f && better(t, 1, s, h)) {
+          h.t = t; h.inst = 1; h.prim = s;
+          others = P.n_src > 1 && !tx_alone(P, D);
+        }
+      }
+      if (h.inst != 1) others = P.n_src > 1 && ray_near_tx(P, r);
+    }
+    if (others) h = traverse_tx(P, o, d, h);
+    __syncwarp();
   }
+  // the rays that the scene is asked for, as beams of similar ones
+  bool ask = on && (!last || h.inst == 1), near_tx = false;
+  const RayB r = ray_b(o, d);
+  for (unsigned left = __ballot_sync(kFullWarp, ask); left;) {
+    bool in = (left >> (threadIdx.x & 31)) & 1u;
+    Beam bm = beam_of(o, d, in);
+    if (bm.spread > AMS_BEAM_SPREAD) {
+      const int lead = __ffs(left) - 1;
+      const float dx = __shfl_sync(kFullWarp, d.x, lead), dy = __shfl_sync(kFullWarp, d.y, lead),
+                  dz = __shfl_sync(kFullWarp, d.z, lead);
+      in = in && (lead == (int)(threadIdx.x & 31) ||
+                  fmaxf(fmaxf(fabsf(d.x - dx), fabsf(d.y - dy)), fabsf(d.z - dz)) <
+                      0.5f * AMS_BEAM_SPREAD);
+      bm = beam_of(o, d, in);
+    }
+    left &= ~__ballot_sync(kFullWarp, in);
+    if (!last && !near_tx) near_tx = beam_near_tx(P, bm);
+    bool alive = in;
+    bool given_up = P.n_tri_wide == 0;
+    if (!given_up) given_up = !beam_scene(P, bm, r, h, alive, last, stk);
+    if (given_up && alive) h = traverse_scene(P, o, d, h);
+    __syncwarp();
+  }
+  if (near_tx && on) h = traverse_tx(P, o, d, h);
+  __syncwarp();
   return h;
 }
 
@@ -457,12 +779,34 @@ __device__ int path_insert(const TraceDev &P, const int32_t *key) {
   return -1;
 }
 
-// scene triangle by original primitive index (optixPathTracer.cu:296-299)
-__device__ __forceinline__ void scene_tri(const TraceDev &P, int prim, af3 &v0, af3 &v1, af3 &v2) {
-  const float *v = P.tris + (size_t)prim * 9;
-  v0 = mk3(__ldg(v), __ldg(v + 1), __ldg(v + 2));
-  v1 = mk3(__ldg(v + 3), __ldg(v + 4), __ldg(v + 5));
-  v2 = mk3(__ldg(v + 6), __ldg(v + 7), __ldg(v + 8));
+// What the hit programs need of scene triangle `prim` (original index,
+// optixPathTracer.cu:296-299): computed once per scene by k_tri_attr with
+// the operations the programs would repeat at every hit.
+struct TriAttr {
+  af3 n;        // unit normal
+  float n_len;  // its length as computed
+  float max_d;  // longest edge
+  af3 v0;
+};
+__device__ __forceinline__ TriAttr scene_tri(const TraceDev &P, int prim) {
+  const float4 a = __ldg(P.tri_attr + 2 * (size_t)prim), b = __ldg(P.tri_attr + 2 * (size_t)prim + 1);
+  TriAttr r;
+  r.n = mk3(a.x, a.y, a.z);
+  r.n_len = a.w;
+  r.v0 = mk3(b.x, b.y, b.z);
+  r.max_d = b.w;
+  return r;
+}
+__global__ void k_tri_attr(const float *tris, int n, float4 *attr) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const float *v = tris + (size_t)i * 9;
+  const af3 v0 = ld3(v), v1 = ld3(v + 3), v2 = ld3(v + 6);
+  const af3 N0 = nrm3(cross3(sub3(v1, v0), sub3(v2, v0)));
+  const float max_d = fmaxf(fmaxf(len3(sub3(v0, v1)), len3(sub3(v1, v2))), len3(sub3(v2, v0)));
+  // a normal turned towards the ray has the same length: squares lose the sign
+  attr[2 * i] = make_float4(N0.x, N0.y, N0.z, len3(N0));
+  attr[2 * i + 1] = make_float4(v0.x, v0.y, v0.z, max_d);
 }
 
 // ---------------------------------------------------------------- stage 1
@@ -574,12 +918,11 @@ __device__ __forceinline__ void s1_hit(const TraceDev &P, S1Query &q, S1Ray &w, 
   const af3 o = add3(q.r.o, scl3(d, q.best.t));
   q.r.o = o;
   if (q.best.inst == 0 && w.ttl > 1) {
-    af3 v0, v1, v2;
-    scene_tri(P, q.best.prim, v0, v1, v2);
-    af3 N0 = nrm3(cross3(sub3(v1, v0), sub3(v2, v0)));
+    const TriAttr tri = scene_tri(P, q.best.prim);
+    const af3 v0 = tri.v0, N0 = tri.n;
     af3 N = faceforward3(N0, neg3(d), N0);
     int m = __ldg(P.mat + q.best.prim);
-    float ct = dot3(d, N) / (len3(N) * len3(d));
+    float ct = dot3(d, N) / (tri.n_len * len3(d));
     int tid = theta_id(ct);
     bool pen = __ldg(P.mat_prop + tid + m * AMS_NBINS) < 0.0f;
     w.ttl--;
@@ -836,6 +1179,107 @@ __global__ void __launch_bounds__(128, 8) k_stage1(TraceDev P) {
   }
 }
 
+// ------------------------------------------------------------- Tx array
+// tx_info of the Tx positions, 4 float4 (beam_near_tx, tx_alone): two
+// directions that the array is thin along (the normal of a planar array
+// twice, two normals of a linear one), each with the sine above which a ray
+// meets one Tx only; then the box of all Tx boxes, widened as a node's.  Word
+// 11 holds the square of the smallest distance of two Tx, word 15 counts the
+// CTAs that have done their share of the pairs (the memory is set to
+// 0x7f7f7f7f before); the last one, or CTA 0 alone beyond kTxPairs Tx where no
+// ray counts as steep enough, writes the rest.
+constexpr int kTxPairs = 4096;
+__global__ void __launch_bounds__(256) k_tx_info(const float *src, const float *aabb, int n,
+                                                 float *info) {
+  __shared__ float sv[8];
+  __shared__ int si[8];
+  __shared__ bool fit;
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+  if (n <= kTxPairs) {
+    float best = 3.0e38f;
+    for (int i = blockIdx.x; i < n; i += gridDim.x) {
+      const af3 a = ld3(src + 3 * i);
+      for (int j = i + 1 + t; j < n; j += blockDim.x) {
+        const af3 v = sub3(ld3(src + 3 * j), a);
+        best = fminf(best, dot3(v, v));
+      }
+    }
+    best = warp_min(best);
+    if (lane == 0) atomicMin(reinterpret_cast<int *>(info) + 11, __float_as_int(best));
+  }
+  __threadfence();
+  __syncthreads();
+  if (t == 0)
+    fit = atomicAdd(reinterpret_cast<int *>(info) + 15, 1) == 0x7f7f7f7f + (int)gridDim.x - 1;
+  __syncthreads();
+  if (!fit) return;
+  __threadfence();
+  // the largest f(i) over the Tx and its index
+  auto farthest = [&](auto f) {
+    float v = -3.0e38f;
+    int at = 0;
+    for (int i = t; i < n; i += blockDim.x) {
+      const float x = f(i);
+      if (x > v) { v = x; at = i; }
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      const float x = __shfl_xor_sync(kFullWarp, v, o);
+      const int i = __shfl_xor_sync(kFullWarp, at, o);
+      if (x > v) { v = x; at = i; }
+    }
+    __syncthreads();
+    if (lane == 0) { sv[w] = v; si[w] = at; }
+    __syncthreads();
+    v = sv[0]; at = si[0];
+    for (int i = 1; i < 8; i++)
+      if (sv[i] > v) { v = sv[i]; at = si[i]; }
+    return make_float2(v, __int_as_float(at));
+  };
+  const af3 a = ld3(src);
+  auto rel = [&](int i) { return sub3(ld3(src + 3 * i), a); };
+  const float2 f1 = farthest([&](int i) { const af3 v = rel(i); return dot3(v, v); });
+  const af3 v1 = rel(__float_as_int(f1.y));
+  const float len = sqrtf(fmaxf(f1.x, 0.0f));
+  const af3 u = len > 0.0f ? scl3(v1, 1.0f / len) : mk3(1.f, 0.f, 0.f);
+  const float2 f2 = farthest([&](int i) { const af3 c = cross3(rel(i), u); return dot3(c, c); });
+  af3 n1, n2;
+  if (f2.x > 1e-6f * len * len) {  // a plane
+    n1 = cross3(rel(__float_as_int(f2.y)), u);
+    n1 = scl3(n1, 1.0f / len3(n1));
+    n2 = n1;
+  } else {  // a line
+    const af3 e = fabsf(u.x) < 0.6f ? mk3(1.f, 0.f, 0.f) : mk3(0.f, 1.f, 0.f);
+    n1 = cross3(u, e);
+    n1 = scl3(n1, 1.0f / len3(n1));
+    n2 = cross3(u, n1);
+  }
+  const float e1 = farthest([&](int i) { return fabsf(dot3(rel(i), n1)); }).x;
+  const float e2 = farthest([&](int i) { return fabsf(dot3(rel(i), n2)); }).x;
+  const float rh = farthest([&](int i) {
+    const af3 c = ld3(src + 3 * i), lo = sub3(c, ld3(aabb + 6 * i)),
+              hi = sub3(ld3(aabb + 6 * i + 3), c);
+    return len3(mk3(fmaxf(fabsf(lo.x), fabsf(hi.x)), fmaxf(fabsf(lo.y), fabsf(hi.y)),
+                    fmaxf(fabsf(lo.z), fabsf(hi.z))));
+  }).x;
+  float bx[6];
+  for (int k = 0; k < 6; k++) {
+    const float sign = k < 3 ? -1.0f : 1.0f;
+    bx[k] = sign * farthest([&](int i) { return sign * aabb[6 * i + k]; }).x;
+    bx[k] += sign * (1e-5f + 2e-6f * fabsf(bx[k]));
+  }
+  if (t == 0) {
+    // two Tx may lie on either side of the first; 20 um of slack for the
+    // rounding of positions and box tests over a building
+    const float rho = 2.0f * (rh + 2e-5f);
+    const float gap = n <= kTxPairs ? sqrtf(__ldcg(info + 11)) - rho : 0.0f;
+    float4 *o = reinterpret_cast<float4 *>(info);
+    o[0] = make_float4(n1.x, n1.y, n1.z, gap > 0.0f ? (2.0f * e1 + rho) / gap + 1e-3f : 3.0e38f);
+    o[1] = make_float4(n2.x, n2.y, n2.z, gap > 0.0f ? (2.0f * e2 + rho) / gap + 1e-3f : 3.0e38f);
+    o[2] = make_float4(bx[0], bx[1], bx[2], 0.0f);
+    o[3] = make_float4(bx[3], bx[4], bx[5], 0.0f);
+  }
+}
+
 // --------------------------------------------------------------- tasks
 // Dense path ids: after stage 1 the path table is final, so stage 2 numbers
 // its paths 0 .. n_paths - 1 (slot_of maps back to the table) and keeps its
@@ -870,11 +1314,11 @@ __global__ void k_to_dense(TraceDev P, const unsigned *in, int w_in, const int *
   }
 }
 
-// The round's tasks, listed per cell: cell c's new paths (dense ids) are
+// With per-ray records (EXPORT) a round's tasks are listed in a fixed order,
+// cell by cell: cell c's new paths (dense ids) are
 // task_path[cell_off[c] .. cell_off[c + 1]) in increasing order, cut into
 // chunks of up to kpi paths: chunk_at[chunk_off[c] ..] = (cell, first
 // task).  A warp per cell counts, one CTA scans, a warp per cell fills.
-// tasks per cell of the first round (later rounds: k_expand counts them)
 __global__ void k_cell_counts(TraceDev P, const unsigned *bits) {
   const int lane = threadIdx.x & 31;
   const int nwarp = (gridDim.x * blockDim.x) >> 5;
@@ -887,9 +1331,8 @@ __global__ void k_cell_counts(TraceDev P, const unsigned *bits) {
   }
 }
 
-// exclusive scans of the task and chunk counts (cell_cnt, zeroed for the
-// next round's counts) into cell_off and chunk_off ([ng] = totals), and the
-// round's counters reset; one CTA of 1024 threads
+// exclusive scans of the task and chunk counts (cell_cnt) into cell_off and
+// chunk_off ([ng] = totals); one CTA of 1024 threads
 __global__ void __launch_bounds__(1024) k_cell_scan(TraceDev P) {
   __shared__ int wsum[32], wch[32];
   __shared__ int carry_s, ccarry_s;
@@ -899,7 +1342,6 @@ __global__ void __launch_bounds__(1024) k_cell_scan(TraceDev P) {
   for (int base = 0; base < P.ng; base += 1024) {
     const int i = base + t;
     const int v = i < P.ng ? P.cell_cnt[i] : 0;
-    if (i < P.ng) P.cell_cnt[i] = 0;
     const int ch = (v + P.kpi - 1) / P.kpi;
     int x = v, y = ch;
     for (int o = 1; o < 32; o <<= 1) {
@@ -928,8 +1370,9 @@ __global__ void __launch_bounds__(1024) k_cell_scan(TraceDev P) {
   if (t == 0) {
     P.cell_off[P.ng] = carry_s;
     P.chunk_off[P.ng] = ccarry_s;
-    P.ctr[5] = (unsigned long long)carry_s;
-    P.ctr[7] = 0ull;  // new tasks, counted by k_expand after this round's stage 2
+    RoundCount *rc = P.rounds + (P.round_slot & (AMS_ROUND_SLOTS - 1));
+    rc->listed = (unsigned long long)carry_s;
+    rc->chunks = (unsigned long long)ccarry_s;
   }
 }
 
@@ -969,28 +1412,113 @@ __global__ void k_cell_fill(TraceDev P, const unsigned *bits) {
       else atomicOr(P.err, AMS_DERR_TASKS);
     }
   }
-  // the success bits of the coming stage 2 start empty
-  const long long nw = (long long)P.ng * P.W;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nw;
-       i += (long long)gridDim.x * blockDim.x)
-    P.S[i] = 0u;
+}
+
+// Flood-fill step and task list of a round in one kernel, a warp per cell.
+// EXPAND: N = (S of the 4 neighbour cells) & ~T; T |= N (cpp:257-300; the
+// neighbours are linear cell indices +-1 and +-n1g with only the [0, ng)
+// check, exactly as the reference, so row ends wrap), and S_next, where the
+// coming stage 2 sets its success bits, is cleared.  Without EXPAND the new
+// tasks are the bits of N already.  LIST: the cell's new tasks in path order
+// go to a run of task_path that the warp claims, cut into chunks of up to kpi
+// paths in chunk_at.  The order of the runs differs from one execution to the
+// next; nothing computed depends on it.  The counts go to the round's slot of
+// the ring `rounds`, whose next slot is zeroed.  Replaces four kernels and two
+// copies a round (count, scan, fill, expand: 20 us of 33 us between the
+// stage-2 kernels of coverage-128's late rounds).
+template <bool EXPAND, bool LIST>
+__global__ void __launch_bounds__(256) k_round(const __grid_constant__ TraceDev P) {
+  const int lane = threadIdx.x & 31;
+  RoundCount *rc = P.rounds + (P.round_slot & (AMS_ROUND_SLOTS - 1));
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    RoundCount *nx = P.rounds + ((P.round_slot + 1) & (AMS_ROUND_SLOTS - 1));
+    nx->tasks = 0ull;
+    nx->listed = 0ull;
+    nx->chunks = 0ull;
+  }
+  const int nwarp = (gridDim.x * blockDim.x) >> 5;
+  for (int cell = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; cell < P.ng; cell += nwarp) {
+    const size_t row = (size_t)cell * P.W;
+    int cnt = 0;
+    for (int w = lane; w < P.W; w += 32) {
+      unsigned n;
+      if (EXPAND) {
+        unsigned s = 0;
+        const int nb[4] = {cell - 1, cell + 1, cell - P.n1g, cell + P.n1g};
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+          if (nb[k] >= 0 && nb[k] < P.ng) s |= __ldg(P.S + (size_t)nb[k] * P.W + w);
+        const unsigned t = P.T[row + w];
+        n = s & ~t;
+        if (n) P.T[row + w] = t | n;
+        P.N[row + w] = n;
+        P.S_next[row + w] = 0u;
+      } else {
+        n = P.N[row + w];
+      }
+      cnt += __popc(n);
+    }
+    cnt = __reduce_add_sync(kFullWarp, cnt);
+    if (cnt == 0) continue;
+    unsigned long long first = 0, c0 = 0;
+    const int nch = (cnt + P.kpi - 1) / P.kpi;
+    if (lane == 0) {
+      first = atomicAdd(EXPAND ? &rc->tasks : &rc->listed, (unsigned long long)cnt);
+      if (LIST) c0 = atomicAdd(&rc->chunks, (unsigned long long)nch);
+    }
+    if (!LIST) continue;
+    first = __shfl_sync(kFullWarp, first, 0);
+    c0 = __shfl_sync(kFullWarp, c0, 0);
+    if (first + cnt > P.task_cap) {
+      if (lane == 0) atomicOr(P.err, AMS_DERR_TASKS);
+      continue;
+    }
+    __syncwarp();
+    unsigned long long pos = first;
+    for (int w0 = 0; w0 < P.W; w0 += 32) {
+      const int w = w0 + lane;
+      unsigned b = w < P.W ? P.N[row + w] : 0u;
+      const int c = __popc(b);
+      int x = c;
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(kFullWarp, x, o);
+        if (lane >= o) x += y;
+      }
+      unsigned long long q = pos + x - c;
+      while (b) {
+        const int id = w * 32 + __ffs(b) - 1;
+        b &= b - 1u;
+        P.task_path[q++] = make_int2(id, id < P.n_paths ? P.slot_of[id] : -1);
+      }
+      pos += __shfl_sync(kFullWarp, x, 31);
+    }
+    for (int j = lane; j < nch; j += 32) {
+      const int t0 = (int)first + j * P.kpi;
+      P.chunk_at[c0 + j] = make_int4(cell, t0, min((int)first + cnt, t0 + P.kpi), 0);
+    }
+  }
 }
 
 // ---------------------------------------------------------------- stage 2
-// One backward ray (stage-2 raygen + closest-hit programs,
+// One backward ray per active lane (stage-2 raygen + closest-hit programs,
 // optixPathTracer.cu:191-273, :332-417): the image source of the path key in
-// `slot` seen from Rx position o, traced back to Tx `s`.  Returns true with
-// the contribution as 2^-56 fixed point when the ray arrives.
-template <bool EXPORT = false>
-__device__ __forceinline__ bool s2_ray(const TraceDev &P, int slot, int s, af3 o, af3 srcdir,
-                                       af3 dstdir, unsigned &segs, unsigned long long &cre,
-                                       unsigned long long &cim, ams_ray_record *rr = nullptr) {
+// `slot` (the same for the whole warp) seen from Rx position o, traced back to
+// Tx `s`.  Every scene hit lowers the remaining levels by one, so the warp's
+// rays stay at the same segment.  Returns true with the contribution as 2^-56
+// fixed point when the ray arrives.  Warp collective.
+template <bool EXPORT>
+__device__ __forceinline__ bool s2_ray(const TraceDev &P, int slot, int s, af3 o,
+                                       bool act, int2 *stk, unsigned &segs,
+                                       unsigned long long &cre, unsigned long long &cim,
+                                       ams_ray_record *rr) {
   const int32_t *key = P.tab_key + (size_t)slot * 14;
   Mat34 M;
 #pragma unroll
   for (int k = 0; k < 12; k++) M.m[k] = __int_as_float(key_word(key, k));
   const int hc = key_word(key, 12), mask = key_word(key, 13);
   const float lam = P.lam_f;
+  const af3 srcdir = mk3(P.src_dir[0], P.src_dir[1], P.src_dir[2]);
+  const af3 dstdir = mk3(P.dst_dir[0], P.dst_dir[1], P.dst_dir[2]);
   af3 d = nrm3(sub3(image_of(M, ld3(P.src + 3 * s)), o));
   float amp = beampattern(d, dstdir, P.dst_bp);
   float xloss = 1.0f;  // exported: free-space factors only
@@ -1000,31 +1528,45 @@ __device__ __forceinline__ bool s2_ray(const TraceDev &P, int slot, int s, af3 o
   }
   float far = 1e6f, dd = 0.0f, dres = 0.0f;
   double D = 0.0;
-  int ttl = hc + 1;
-  int guard = 0;
   bool ok = false;
-  while (ttl > 0) {
-    if (++guard > AMS_SEG_CAP) { atomicOr(P.err, AMS_DERR_LOOP); break; }
-    Hit h = closest_s2(P, o, d, ttl == 1);
-    segs++;
-    if (h.inst == 3) break;
-    const float t = h.t;
-    o = add3(o, scl3(d, t));
-    dd += t;
-    D += (double)t;
-    if (h.inst == 0) {
-      if (ttl == 1) break;
-      af3 v0, v1, v2;
-      scene_tri(P, h.prim, v0, v1, v2);
-      af3 N0 = nrm3(cross3(sub3(v1, v0), sub3(v2, v0)));
-      af3 N = faceforward3(N0, neg3(d), N0);
-      int m = __ldg(P.mat + h.prim);
-      float ct = dot3(d, N) / (len3(N) * len3(d));
+  for (int ttl = hc + 1; ttl > 0; ttl--) {
+    if (!__any_sync(kFullWarp, act)) break;
+    const bool last = ttl == 1;
+    // a ray that meets another Tx's sphere goes on behind it; the warp's other
+    // rays wait for it
+    bool todo = act;
+    int prim = 0;
+    for (int guard = 0; __any_sync(kFullWarp, todo); guard++) {
+      if (guard >= AMS_SEG_CAP) {
+        if (todo) { atomicOr(P.err, AMS_DERR_LOOP); act = false; }
+        break;
+      }
+      __syncwarp();
+      const Hit h = closest_s2(P, o, d, s, last, todo, stk);
+      if (todo) {
+        segs++;
+        const bool other = h.inst == 1 && h.prim != s;
+        if (h.inst != 3) {
+          o = add3(o, scl3(d, h.t));
+          dd += h.t;
+          D += (double)h.t;
+        }
+        prim = h.prim;
+        todo = other;
+        // the segment has to end on a triangle, the last one on Tx s
+        if (!other && h.inst != (last ? 1 : 0)) act = false;
+      }
+      __syncwarp();
+    }
+    if (act && !last) {
+      const TriAttr tri = scene_tri(P, prim);
+      const float max_d = tri.max_d;
+      const af3 N = faceforward3(tri.n, neg3(d), tri.n);
+      int m = __ldg(P.mat + prim);
+      float ct = dot3(d, N) / (tri.n_len * len3(d));
       float loss = fabsf(__ldg(P.mat_prop + theta_id(ct) + m * AMS_NBINS));
-      ttl--;
-      int hcb = hc + 1 - ttl;
+      int hcb = hc + 2 - ttl;
       int is_ref = (mask >> (hcb - 1)) & 1;
-      float max_d = fmaxf(fmaxf(len3(sub3(v0, v1)), len3(sub3(v1, v2))), len3(sub3(v2, v0)));
       float fspl = 1.0f;
       if (dd > far) { fspl = lam / ((4.0f * AMS_PIF) * dres); dres = 0.0f; }
       amp *= loss * fspl;
@@ -1047,21 +1589,19 @@ __device__ __forceinline__ bool s2_ray(const TraceDev &P, int slot, int s, af3 o
       far = far_next;
       dd = 0.0f;
       if (is_ref) d = sub3(d, scl3(N, 2.0f * dot3(d, N)));
-    } else if (h.inst == 1 && h.prim == s) {
-      if (ttl == 1) {
-        float bp = beampattern(neg3(d), srcdir, P.src_bp);
-        float af = lam / ((4.0f * AMS_PIF) * (dres + dd));
-        amp *= bp * af;
-        ok = true;
-        if (EXPORT) {
-          const af3 nd = neg3(d);
-          rr->launch_angle = dot3(nd, srcdir) / (len3(nd) * len3(srcdir));
-          rr->loss = xloss * af;
-          rr->phase = D * P.two_pi_over_lam;
-        }
+    } else if (act) {
+      float bp = beampattern(neg3(d), srcdir, P.src_bp);
+      float af = lam / ((4.0f * AMS_PIF) * (dres + dd));
+      amp *= bp * af;
+      ok = true;
+      if (EXPORT) {
+        const af3 nd = neg3(d);
+        rr->launch_angle = dot3(nd, srcdir) / (len3(nd) * len3(srcdir));
+        rr->loss = xloss * af;
+        rr->phase = D * P.two_pi_over_lam;
       }
-      break;
     }
+    __syncwarp();
   }
   if (ok) {
     // FP64 path length -> phase, reduced mod 2 pi in FP64 (products with
@@ -1085,47 +1625,58 @@ __device__ __forceinline__ bool s2_ray(const TraceDev &P, int slot, int s, af3 o
   return ok;
 }
 
-// Persistent stage 2: a warp takes an item = (a chunk of up to kpi of one
-// cell's new paths, 32 consecutive (Rx within the cell, Tx) pairs, Tx
-// fastest) and traces the chunk's paths one after the other; each
+// Stage 2: a warp takes an item = (a chunk of up to kpi of one cell's new
+// paths, 32 consecutive (Rx within the cell, Tx) pairs, Tx fastest) and traces
+// the chunk's paths one after the other, the 32 rays of a path as a beam; each
 // lane sums its pair's contributions over the chunk in registers (exact
 // 64-bit fixed point) and adds them once into the Rx-major accumulator
 // acc[dst][s], so a warp's adds cover one or a few contiguous runs of Tx
 // (coalesced), one atomic add per (Tx, Rx) and chunk instead of two per
-// verified ray.  The lanes of an item trace the same path key from the same
-// Rx to neighbouring Tx elements: nearly identical rays.  One warp per item,
-// 8 per CTA: the block scheduler balances items of uneven cost (fixed
-// strides over persistent warps and a fetch counter both measured slower);
-// kpi is chosen per round by the host so that a round keeps several items
-// per resident warp.
-__global__ void __launch_bounds__(256, 5) k_stage2(TraceDev P) {
-  const int S = P.n_src;
-  const long long pairs = (long long)P.gs * P.gs * S;
-  const long long G = (pairs + 31) / 32;
-  const long long n_items = (long long)P.chunk_off[P.ng] * G;
+// verified ray.  One warp per item, 8 per CTA: the block scheduler balances
+// items of uneven cost (fixed strides over persistent warps and a fetch
+// counter both measured slower); kpi is chosen per round by the host so that a
+// round keeps several items per resident warp.  The launch covers the items
+// when the host knows their number, else (late rounds, whose list the host has
+// not seen) the resident warps stride over them.  With EXPORT (kpi = 1) every
+// ray's record is written.
+template <bool EXPORT>
+__global__ void __launch_bounds__(256, 4) k_stage2(const __grid_constant__ TraceDev P) {
+  __shared__ int2 stack[8][AMS_BEAM_STACK];
   const int lane = threadIdx.x & 31;
-  const af3 srcdir = mk3(P.src_dir[0], P.src_dir[1], P.src_dir[2]);
-  const af3 dstdir = mk3(P.dst_dir[0], P.dst_dir[1], P.dst_dir[2]);
+  const unsigned n_chunks = (unsigned)P.rounds[P.round_slot & (AMS_ROUND_SLOTS - 1)].chunks;
+  const long long n_items = (long long)n_chunks * P.s2_groups;
   unsigned n_ok = 0, n_fail = 0, n_segs = 0, n_adds = 0;  // n_adds: warp total
-  if (blockIdx.x == 0 && threadIdx.x == 0 && n_items > (long long)gridDim.x * (blockDim.x >> 5))
-    atomicOr(P.err, AMS_DERR_TASKS);  // the launch must cover every item
-  {
-    const long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (item >= n_items) return;
-    const int4 chunk = __ldg(P.chunk_at + item / G);
+  long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (item >= n_items) return;
+  for (; item < n_items; item += (long long)gridDim.x * (blockDim.x >> 5)) {
+    unsigned ck, grp;  // chunk and group of 32 pairs
+    if (n_items <= 0xffffffffll) {
+      ck = fdiv((unsigned)item, P.div_groups);
+      grp = (unsigned)item - ck * P.s2_groups;
+    } else {
+      ck = (unsigned)(item / P.s2_groups);
+      grp = (unsigned)(item % P.s2_groups);
+    }
+    const int4 chunk = __ldg(P.chunk_at + ck);
     const int cell = chunk.x, t0 = chunk.y, t1 = chunk.z;
     if ((unsigned)cell >= (unsigned)P.ng || t0 < 0 || t1 < t0 ||
         (unsigned long long)t1 > P.task_cap) {
       if (lane == 0) atomicOr(P.err, AMS_DERR_TASKS);
-      return;
+      break;
     }
-    const long long pr = (long long)(item % G) * 32 + lane;
-    bool act = pr < pairs;
-    const int inner = act ? (int)(pr / S) : 0, s = act ? (int)(pr % S) : 0;
-    const int gi = cell / P.n1g, gj = cell % P.n1g;
-    const int di = inner / P.gs + gi * P.gs, dj = inner % P.gs + gj * P.gs;
+    const long long pairs = (long long)P.gs * P.gs * P.n_src;
+    const long long pr = (long long)grp * 32 + lane;
+    const bool pair = pr < pairs;
+    const unsigned inner = !pair ? 0u : pr <= 0xffffffffll ? fdiv((unsigned)pr, P.div_src)
+                                                          : (unsigned)(pr / P.n_src);
+    const int s = pair ? (int)(pr - (long long)inner * P.n_src) : 0;
+    const int ir = (int)fdiv(inner, P.div_gs), gi = (int)fdiv((unsigned)cell, P.div_n1g);
+    const int di = ir + gi * P.gs, dj = (int)inner - ir * P.gs + (cell - gi * P.n1g) * P.gs;
     const int dst = di * P.n1_dst + dj;
-    if (dst >= P.n_dst || (P.strict_grid && (di >= P.n0_dst || dj >= P.n1_dst))) act = false;
+    const bool act = pair && !(dst >= P.n_dst ||
+                               (P.strict_grid && (di >= P.n0_dst || dj >= P.n1_dst)));
+    const af3 o = act ? ld3(P.dst + 3 * (size_t)dst) : mk3(0.f, 0.f, 0.f);
+    bool any_ok = false;
     unsigned long long sre = 0, sim = 0;
     for (int t = t0; t < t1; t++) {
       const int2 task = __ldg(P.task_path + t);
@@ -1134,146 +1685,45 @@ __global__ void __launch_bounds__(256, 5) k_stage2(TraceDev P) {
         if (lane == 0) atomicOr(P.err, AMS_DERR_TASKS);
         break;
       }
-      bool ok = false;
-      if (act) {
-        unsigned long long cre = 0, cim = 0;
-        ok = s2_ray(P, slot, s, ld3(P.dst + 3 * dst), srcdir, dstdir, n_segs, cre, cim);
-        if (ok) { sre += cre; sim += cim; n_ok++; } else { n_fail++; }
+      ams_ray_record rr;
+      if (EXPORT) {
+        rr.src = s; rr.dst = pair ? dst : -1; rr.path = path; rr.traced = act ? 1 : 0;
+        rr.successful = 0; rr.hit_cnt = 0;
+        rr.launch_angle = 0.f; rr.receive_angle = 0.f; rr.loss = 0.f; rr.pad0 = 0.f;
+        rr.phase = 0.0; rr.pad1 = 0;
+#pragma unroll
+        for (int i = 0; i < 5; i++) rr.hit_loss_idx[i] = -1;
       }
-      if (__any_sync(0xffffffffu, ok) && lane == 0)
+      unsigned long long cre = 0, cim = 0;
+      const bool ok = s2_ray<EXPORT>(P, slot, s, o, act, stack[threadIdx.x >> 5], n_segs, cre, cim,
+                                     &rr);
+      if (ok) { sre += cre; sim += cim; n_ok++; any_ok = true; } else if (act) { n_fail++; }
+      if (EXPORT && pair) {
+        if (!act) rr.receive_angle = 0.f;  // not traced
+        rr.successful = ok ? 1 : 0;
+        const unsigned long long at = P.rec_base + (unsigned long long)t * pairs + pr;
+        if (at < P.rec_cap) P.rec[at] = rr;
+      }
+      if (__any_sync(kFullWarp, ok) && lane == 0)
         atomicOr(P.S + (size_t)cell * P.W + (path >> 5), 1u << (path & 31));
     }
-    const bool add = act && (sre | sim);
+    const bool add = P.kpi == 1 ? any_ok : act && (sre | sim);
     if (add) {
-      unsigned long long *acc = P.acc + ((size_t)dst * S + s) * 2;
+      unsigned long long *acc = P.acc + ((size_t)dst * P.n_src + s) * 2;
       atomicAdd(acc, sre);
       atomicAdd(acc + 1, sim);
     }
-    n_adds += 2u * (unsigned)__popc(__ballot_sync(0xffffffffu, add));
+    n_adds += 2u * (unsigned)__popc(__ballot_sync(kFullWarp, add));
   }
-  for (int off = 16; off > 0; off >>= 1) {
-    n_ok += __shfl_xor_sync(0xffffffffu, n_ok, off);
-    n_fail += __shfl_xor_sync(0xffffffffu, n_fail, off);
-    n_segs += __shfl_xor_sync(0xffffffffu, n_segs, off);
-  }
+  n_ok = __reduce_add_sync(kFullWarp, n_ok);
+  n_fail = __reduce_add_sync(kFullWarp, n_fail);
+  n_segs = __reduce_add_sync(kFullWarp, n_segs);
   if (lane == 0) {
     if (n_adds) atomicAdd(P.ctr + 13, (unsigned long long)n_adds);
     if (n_segs) atomicAdd(P.ctr + 9, (unsigned long long)n_segs);
     if (n_ok) atomicAdd(P.ctr + 3, (unsigned long long)n_ok);
     if (n_fail) atomicAdd(P.ctr + 4, (unsigned long long)n_fail);
   }
-}
-
-// Stage 2 for rounds whose items hold one path each (kpi == 1, where the
-// per-lane sums above have nothing to add up): one thread per backward ray,
-// rays of all tasks laid out back to back (task-major, then Rx within the
-// cell, then Tx), so no warp idles on the padding of a task's last item.
-// Each verified ray adds its contribution to the Rx-major accumulator.
-template <bool EXPORT>
-__global__ void __launch_bounds__(256, 5) k_stage2_rays(TraceDev P) {
-  const int S = P.n_src;
-  const long long pairs = (long long)P.gs * P.gs * S;
-  const long long n_rays = (long long)P.cell_off[P.ng] * pairs;
-  const long long ray = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const int lane = threadIdx.x & 31;
-  if (blockIdx.x == 0 && threadIdx.x == 0 && n_rays > (long long)gridDim.x * blockDim.x)
-    atomicOr(P.err, AMS_DERR_TASKS);  // the launch must cover every ray
-  if (ray - lane >= n_rays) return;   // the whole warp is past the last ray
-  bool valid = ray < n_rays;
-  const long long t = valid ? ray / pairs : -1;
-  int cell = 0, path = 0, slot = 0, inner = 0, s = 0;
-  if (valid) {
-    const int4 chunk = __ldg(P.chunk_at + t);
-    const int2 task = __ldg(P.task_path + t);
-    cell = chunk.x;
-    path = task.x;
-    slot = task.y;
-    const long long pr = ray % pairs;
-    inner = (int)(pr / S);
-    s = (int)(pr % S);
-    if ((unsigned)cell >= (unsigned)P.ng || (unsigned)path >= (unsigned)P.n_paths ||
-        (unsigned)slot > P.tab_mask || (unsigned long long)t >= P.task_cap) {
-      atomicOr(P.err, AMS_DERR_TASKS);
-      valid = false;
-    }
-  }
-  bool ok = false, traced = false;
-  unsigned segs = 0;
-  ams_ray_record rr;
-  if (EXPORT) {
-    rr.src = s; rr.dst = -1; rr.path = path; rr.traced = 0; rr.successful = 0; rr.hit_cnt = 0;
-    rr.launch_angle = 0.f; rr.receive_angle = 0.f; rr.loss = 0.f; rr.pad0 = 0.f;
-    rr.phase = 0.0; rr.pad1 = 0;
-#pragma unroll
-    for (int i = 0; i < 5; i++) rr.hit_loss_idx[i] = -1;
-  }
-  if (valid) {
-    const int gi = cell / P.n1g, gj = cell % P.n1g;
-    const int di = inner / P.gs + gi * P.gs, dj = inner % P.gs + gj * P.gs;
-    const int dst = di * P.n1_dst + dj;
-    if (EXPORT) rr.dst = dst;
-    if (!(dst >= P.n_dst || (P.strict_grid && (di >= P.n0_dst || dj >= P.n1_dst)))) {
-      traced = true;
-      unsigned long long cre = 0, cim = 0;
-      const af3 srcdir = mk3(P.src_dir[0], P.src_dir[1], P.src_dir[2]);
-      const af3 dstdir = mk3(P.dst_dir[0], P.dst_dir[1], P.dst_dir[2]);
-      ok = s2_ray<EXPORT>(P, slot, s, ld3(P.dst + 3 * dst), srcdir, dstdir, segs, cre, cim, &rr);
-      if (ok) {
-        unsigned long long *acc = P.acc + ((size_t)dst * S + s) * 2;
-        atomicAdd(acc, cre);
-        atomicAdd(acc + 1, cim);
-      }
-    }
-  }
-  if (EXPORT && valid) {
-    rr.traced = traced ? 1 : 0;
-    rr.successful = ok ? 1 : 0;
-    const unsigned long long at = P.rec_base + (unsigned long long)ray;
-    if (at < P.rec_cap) P.rec[at] = rr;
-  }
-  // counters and each task's success bit, one atomic per warp / task
-  const unsigned okb = __ballot_sync(0xffffffffu, ok);
-  const unsigned trb = __ballot_sync(0xffffffffu, traced);
-  for (int off = 16; off > 0; off >>= 1) segs += __shfl_xor_sync(0xffffffffu, segs, off);
-  if (lane == 0) {
-    if (segs) atomicAdd(P.ctr + 9, (unsigned long long)segs);
-    if (okb) {
-      atomicAdd(P.ctr + 3, (unsigned long long)__popc(okb));
-      atomicAdd(P.ctr + 13, 2ull * (unsigned long long)__popc(okb));  // two adds per ray
-    }
-    if (trb & ~okb) atomicAdd(P.ctr + 4, (unsigned long long)__popc(trb & ~okb));
-  }
-  const unsigned same = __match_any_sync(0xffffffffu, t);
-  if (valid && (okb & same) && lane == __ffs(same) - 1)
-    atomicOr(P.S + (size_t)cell * P.W + (path >> 5), 1u << (path & 31));
-}
-
-// N = (S of the 4 neighbour cells) & ~T; T |= N; S = 0 (cpp:257-300).  The
-// neighbours are linear cell indices +-1 and +-n1g with only the [0, ng)
-// check, exactly as the reference (so row ends wrap).
-__global__ void k_expand(TraceDev P) {
-  const long long nwords = (long long)P.ng * P.W;
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  unsigned long long cnt = 0;
-  for (long long wi = (long long)blockIdx.x * blockDim.x + threadIdx.x; wi < nwords; wi += stride) {
-    const int cell = (int)(wi / P.W);
-    const int w = (int)(wi % P.W);
-    unsigned s = 0;
-    const int nb[4] = {cell - 1, cell + 1, cell - P.n1g, cell + P.n1g};
-#pragma unroll
-    for (int k = 0; k < 4; k++)
-      if (nb[k] >= 0 && nb[k] < P.ng) s |= P.S[(size_t)nb[k] * P.W + w];
-    unsigned t = P.T[wi];
-    unsigned n = s & ~t;
-    P.N[wi] = n;
-    if (n) {
-      P.T[wi] = t | n;
-      atomicAdd(P.cell_cnt + cell, __popc(n));
-    }
-    cnt += __popc(n);
-  }
-  for (int off = 16; off > 0; off >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, off);
-  if ((threadIdx.x & 31) == 0 && cnt) atomicAdd(P.ctr + 7, cnt);
 }
 
 __global__ void k_popcount(const unsigned *bits, long long n, unsigned long long *out) {
@@ -1336,6 +1786,20 @@ int grid_for(long long n, int block) {
 
 }  // namespace
 
+cudaError_t trace_tri_attr(const float *tris, int n, float4 *attr, cudaStream_t st) {
+  if (n > 0) k_tri_attr<<<(n + 255) / 256, 256, 0, st>>>(tris, n, attr);
+  return cudaGetLastError();
+}
+
+cudaError_t trace_tx_info(const float *src, const float *aabb, int n, float *info,
+                          cudaStream_t st) {
+  cudaError_t e = cudaMemsetAsync(info, 0x7f, 4 * 16, st);
+  if (e != cudaSuccess) return e;
+  const int blocks = n > kTxPairs ? 1 : std::min(n, 304);
+  k_tx_info<<<blocks, 256, 0, st>>>(src, aabb, n, info);
+  return cudaGetLastError();
+}
+
 cudaError_t trace_stage1(const TraceDev &P, cudaStream_t st) {
   // persistent: as many CTAs as are resident at once (lanes fetch launch
   // indices from ctr[10], zeroed with the other counters)
@@ -1367,7 +1831,7 @@ int stage2_per_sm() {
   if (dev < 0) return 1;
   if (per_sm[dev] == 0) {
     int b = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_stage2, 256, 0) != cudaSuccess) b = 1;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_stage2<false>, 256, 0) != cudaSuccess) b = 1;
     per_sm[dev] = b > 0 ? b : 1;
   }
   return per_sm[dev];
@@ -1396,53 +1860,47 @@ cudaError_t trace_dense_paths(const TraceDev &P, const unsigned *T_slots, int w_
   return cudaGetLastError();
 }
 
-cudaError_t trace_count_tasks(const TraceDev &P, const unsigned *bits, cudaStream_t st) {
-  k_cell_counts<<<grid_for((long long)P.ng * 32, 256), 256, 0, st>>>(P, bits);
+cudaError_t trace_round(const TraceDev &P, bool expand, bool list, cudaStream_t st) {
+  const int blocks = grid_for((long long)P.ng * 32, 256);
+  if (expand && list) k_round<true, true><<<blocks, 256, 0, st>>>(P);
+  else if (expand) k_round<true, false><<<blocks, 256, 0, st>>>(P);
+  else if (list) k_round<false, true><<<blocks, 256, 0, st>>>(P);
   return cudaGetLastError();
 }
 
-cudaError_t trace_make_tasks(const TraceDev &P, const unsigned *bits, cudaStream_t st) {
-  const long long threads = (long long)P.ng * 32;
+cudaError_t trace_list_ordered(const TraceDev &P, cudaStream_t st) {
+  const int blocks = grid_for((long long)P.ng * 32, 256);
+  k_cell_counts<<<blocks, 256, 0, st>>>(P, P.N);
   k_cell_scan<<<1, 1024, 0, st>>>(P);
-  k_cell_fill<<<grid_for(threads, 256), 256, 0, st>>>(P, bits);
+  k_cell_fill<<<blocks, 256, 0, st>>>(P, P.N);
   return cudaGetLastError();
 }
 
 cudaError_t trace_stage2(const TraceDev &P, unsigned long long n_tasks, cudaStream_t st) {
-  if (n_tasks == 0) return cudaSuccess;
   // one warp per item; the chunks number at most n_tasks / kpi + one per
-  // cell (the exact count is on the device, warps beyond it return)
-  const unsigned long long pairs = (unsigned long long)(P.gs * P.gs) * P.n_src;
-  const unsigned long long k = (unsigned long long)P.kpi;
-  unsigned long long chunks = (n_tasks + k - 1) / k + (unsigned long long)P.ng;
-  if (chunks > n_tasks) chunks = n_tasks;
-  if (P.kpi == 1) {  // one path per item: one thread per ray
-    const unsigned long long blocks = (n_tasks * pairs + 255) / 256;
+  // cell (the exact count is on the device, warps beyond it return); with no
+  // n_tasks, the warps that are resident at once
+  unsigned long long blocks = (unsigned long long)stage2_per_sm() * ams_device_sms();
+  if (n_tasks > 0) {
+    const unsigned long long k = (unsigned long long)P.kpi;
+    unsigned long long chunks = (n_tasks + k - 1) / k + (unsigned long long)P.ng;
+    if (chunks > n_tasks) chunks = n_tasks;
+    blocks = (chunks * P.s2_groups + 7) / 8;
     if (blocks > 0x7fffffffull) return cudaErrorInvalidConfiguration;
-    k_stage2_rays<false><<<(unsigned)blocks, 256, 0, st>>>(P);
-    return cudaGetLastError();
   }
-  const unsigned long long items_max = chunks * ((pairs + 31) / 32);
-  const unsigned long long blocks = (items_max + 7) / 8;
-  if (blocks > 0x7fffffffull) return cudaErrorInvalidConfiguration;
-  k_stage2<<<(unsigned)blocks, 256, 0, st>>>(P);
+  if (P.rec) {
+    if (P.kpi != 1) return cudaErrorInvalidValue;
+    k_stage2<true><<<(unsigned)blocks, 256, 0, st>>>(P);
+  } else {
+    k_stage2<false><<<(unsigned)blocks, 256, 0, st>>>(P);
+  }
   return cudaGetLastError();
 }
 
-cudaError_t trace_stage2_export(const TraceDev &P, unsigned long long n_tasks, cudaStream_t st) {
-  if (n_tasks == 0) return cudaSuccess;
-  if (P.kpi != 1) return cudaErrorInvalidValue;
-  const unsigned long long pairs = (unsigned long long)(P.gs * P.gs) * P.n_src;
-  const unsigned long long blocks = (n_tasks * pairs + 255) / 256;
-  if (blocks > 0x7fffffffull) return cudaErrorInvalidConfiguration;
-  k_stage2_rays<true><<<(unsigned)blocks, 256, 0, st>>>(P);
-  return cudaGetLastError();
-}
-
-cudaError_t trace_expand(const TraceDev &P, cudaStream_t st) {
-  long long n = (long long)P.ng * P.W;
-  k_expand<<<grid_for(n, 256), 256, 0, st>>>(P);
-  return cudaGetLastError();
+bool trace_round_is_small(const TraceDev &P, unsigned long long n_tasks) {
+  // up to four items per resident warp
+  const unsigned long long warps = (unsigned long long)stage2_per_sm() * ams_device_sms() * 8;
+  return n_tasks * P.s2_groups <= 4 * warps;
 }
 
 cudaError_t trace_count_bits(const TraceDev &P, const unsigned *bits, unsigned long long *out,
