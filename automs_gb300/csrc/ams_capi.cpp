@@ -466,7 +466,7 @@ ams_status trace_impl(ams_scene *S, const ams_trace_params *p, const float *src,
     need += 3 * al(4 * (size_t)ng * W);
     need += 2 * al(4 * ((size_t)ng + 1)) + al(4 * (size_t)ng) + 2 * al(4 * (size_t)tab_size);
     need += al(16 * (size_t)n_src * n_dst);
-    need += al(kCounterBytes) + al(4 * 16);
+    need += al(kCounterBytes) + al(4 * 16) + al(4 * 8);
     need += 4096;
     CK(S->ws.ensure(need));
     S->ws.reset();
@@ -497,6 +497,7 @@ ams_status trace_impl(ams_scene *S, const ams_trace_params *p, const float *src,
     P.err = reinterpret_cast<unsigned *>(counters + offsetof(HostCounters, err));
     P.round_slot = 0;
     float *tx_info = S->ws.take<float>(16);
+    float *rx_grid = S->ws.take<float>(8);
 
     if (!src_aabb) { CK(sphere_aabbs(src, n_src, p->src_r, sbox, st)); src_aabb = sbox; }
     if (!dst_aabb) { CK(sphere_aabbs(dst, n_dst, p->dst_r, dbox, st)); dst_aabb = dbox; }
@@ -504,6 +505,7 @@ ams_status trace_impl(ams_scene *S, const ams_trace_params *p, const float *src,
     CK(lbvh_build_spheres(tx, src, src_aabb, n_src, scratch, tx_out, st));
     CK(lbvh_build_spheres(rx, dst, dst_aabb, n_dst, scratch, rx_out, st));
     CK(trace_tx_info(src, src_aabb, n_src, tx_info, st));
+    CK(trace_rx_grid(dst, dst_aabb, n0, n1, rx_grid, st));
     CK(cudaEventRecord(ev[1], st));
 
     P.tris = S->tris;
@@ -517,6 +519,8 @@ ams_status trace_impl(ams_scene *S, const ams_trace_params *p, const float *src,
     P.mat_prop = S->mat_prop;
     P.tx_nodes = tx.nodes; P.tx_prims = tx.prims; P.n_src = n_src; P.src = src; P.src_r = p->src_r;
     P.src_aabb = src_aabb;
+    P.dst_aabb = dst_aabb;
+    P.rx_grid = rx_grid;
     P.tx_info = reinterpret_cast<const float4 *>(tx_info);
     P.rx_nodes = rx.nodes; P.rx_prims = rx.prims; P.n_dst = n_dst; P.dst = dst; P.dst_r = p->dst_r;
     P.n0_dst = n0; P.n1_dst = n1; P.n0g = n0g; P.n1g = n1g; P.ng = ng; P.gs = gs;

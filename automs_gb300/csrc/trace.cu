@@ -603,6 +603,13 @@ __device__ __noinline__ Hit traverse_scene(const TraceDev &P, af3 o, af3 d, Hit 
   return h;
 }
 
+__device__ __noinline__ Hit traverse_rx(const TraceDev &P, af3 o, af3 d, Hit h) {
+  RayT r;
+  ray_setup(r, o, d);
+  traverse<2>(P.rx_nodes, P.rx_prims, P.n_dst, r, h, P.dst_r, P.err);
+  return h;
+}
+
 // Backward-ray query of stage 2 for a warp: optixTrace with the visibility
 // mask of the scene and the Tx spheres (optixPathTracer.cpp:417-424), from
 // (o, d) of the lanes with `on` towards Tx s.  On a path's last segment a
@@ -745,6 +752,7 @@ __device__ int path_insert(const TraceDev &P, const int32_t *key) {
 #pragma unroll
   for (int i = 0; i < 14; i++) enc[i] = (uint32_t)key[i] ^ AMS_KEY_FLIP;
   uint32_t slot = (uint32_t)h & P.tab_mask;
+#pragma unroll 1
   for (uint32_t probe = 0; probe <= P.tab_mask; probe++) {
     unsigned long long old = __ldcg(P.tab_h + slot);
     uint32_t *sk = reinterpret_cast<uint32_t *>(P.tab_key) + (size_t)slot * 14;
@@ -844,22 +852,28 @@ struct CurMatrix {
 
 // Stage 1 runs as a persistent loop per warp with dynamic fetching (after
 // Aila & Laine, "Understanding the efficiency of ray traversal on GPUs",
-// HPG 2009).  All lanes visit BVH nodes of their own closest-hit queries
-// (Rx spheres, then the scene pruned at the sphere hit) in one loop whose
-// body is a single node visit, until every lane's query has ended; then all
-// lanes handle their hits together and set up their next queries (the next
-// segment, the next pending slot, the next sub-launch, or a launch index
-// fetched from a global counter), and the next round of node visits starts.
-// Lanes that finish a short ray take new work instead of idling behind the
-// warp's longest ray, and the hit code runs once per round for the whole
-// warp.  (Handling the hits of a subset of lanes while the others still
-// traverse measured slower at every threshold tried: the hit code is long.)
+// HPG 2009).  A round answers one closest-hit query of every lane: the Rx
+// spheres (by their grid, or by their hierarchy where they form none), then
+// the scene pruned at the sphere hit, visiting BVH nodes until every lane's
+// query has ended; then all lanes handle their hits together and set up their
+// next queries (the next segment, the next pending slot, the next sub-launch,
+// or a launch index fetched from a global counter).  Lanes that finish a
+// short ray take new work instead of idling behind the warp's longest ray, and
+// the hit code runs once per round for the whole warp.  (Handling the hits
+// of a subset of lanes while the others still traverse measured slower at
+// every threshold tried: the hit code is long.)
 // Per launch index the queries, hits and records come in the order of the
 // sequential trace (slots in increasing index, which is the order
 // __ffs(pending) gives because a spawned slot always has a higher index than
 // its parent), so the per-thread min_hc dedup and the reserve cap see
 // exactly what they see in the reference.
-enum { PH_RX = 0, PH_SCENE = 1, PH_HIT = 2 };
+//
+// Half of the node visits were spent on the Rx spheres (13 per query in a tree
+// of 16,384); the grid needs a row or two.  Bound by instruction fetch: 12 of
+// 32 lanes are active, and short loops run rolled up (unrolled by the
+// compiler they cost 3.1 instead of 2.6 ms on coverage-128).  k_stage1:
+// coverage-128 3.84 -> 2.56 ms, 62k triangles and 256 x 256 Rx 14.8 -> 8.8 ms,
+// the same scene and a 32 x 32 metasurface as Rx 9.6 -> 4.8 ms.
 
 // warp-aggregated fetch of one launch index per calling lane
 __device__ __forceinline__ long long fetch_launch(unsigned long long *ctr) {
@@ -876,21 +890,151 @@ struct S1Query {
   RayT r;
   af3 Dq;  // unit direction for the sphere tests
   Hit best;
-  int phase, node, sp;
 };
 
-// first node of the query's next instance, or PH_HIT; one-primitive
-// instances are tested here (they have no nodes)
-__device__ __forceinline__ void s1_enter(const TraceDev &P, S1Query &q, int phase) {
-  q.node = 0;
-  q.sp = 0;
-  if (phase == PH_RX) {
-    if (P.n_dst > 1) { q.phase = PH_RX; return; }
-    if (P.n_dst == 1) test_prim<2>(P.rx_prims, 0, q.r, q.best, P.dst_r, q.Dq);
+// ------------------------------------------------------------- Rx grid
+// Rx sets are mostly axis-aligned planar grids (gen_pos_from_endpoint,
+// go.py:248-300): index i runs along axis ua, j along va, and axis wa is
+// constant.  A ray crosses the slab of all Rx boxes over a short stretch, whose
+// u and v intervals give the few Rx that it can meet; they are tested one by
+// one with the tests that the hierarchy's leaves get.  rx_grid words: 0-2 the
+// largest deviation of an Rx from its place in the grid along u, v, w; 3-5 the
+// largest extent of a box from its Rx.
+struct RxGrid {
+  int ok, ua, va, wa;
+  float u0, su, iu, v0, sv, iv, w0;  // steps and their inverses, 0 where there is one row
+  float bu, bv, bw;          // reach of a box, with the deviation and a margin
+};
+// axes, origin and steps from three corners of the set
+__device__ __forceinline__ RxGrid rx_grid_axes(const float *dst, int n0, int n1, float &du,
+                                               float &dv) {
+  RxGrid g;
+  const af3 a = ld3(dst), e = sub3(ld3(dst + 3 * (size_t)(n0 - 1) * n1), a),
+            f = sub3(ld3(dst + 3 * (size_t)(n1 - 1)), a);
+  auto main_axis = [](af3 v) {
+    const float x = fabsf(v.x), y = fabsf(v.y), z = fabsf(v.z);
+    return x >= y ? (x >= z ? 0 : 2) : (y >= z ? 1 : 2);
+  };
+  g.ua = main_axis(e);
+  g.va = main_axis(f);
+  if (n0 == 1) g.ua = (g.va + 1) % 3;
+  if (n1 == 1) g.va = (g.ua + 1) % 3;
+  g.wa = 3 - g.ua - g.va;
+  g.ok = g.ua != g.va && n0 * n1 > 1;
+  if (!g.ok) g.wa = 0;
+  du = n0 > 1 ? comp3(e, g.ua) / (float)(n0 - 1) : 0.0f;
+  dv = n1 > 1 ? comp3(f, g.va) / (float)(n1 - 1) : 0.0f;
+  g.u0 = comp3(a, g.ua);
+  g.v0 = comp3(a, g.va);
+  g.w0 = comp3(a, g.wa);
+  return g;
+}
+__global__ void __launch_bounds__(256) k_rx_grid(const float *dst, const float *aabb, int n0, int n1,
+                                                 float *out) {
+  float du, dv;
+  const RxGrid g = rx_grid_axes(dst, n0, n1, du, dv);
+  float m[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  const int ax[3] = {g.ua, g.va, g.wa};
+  for (int d = blockIdx.x * blockDim.x + threadIdx.x; d < n0 * n1; d += gridDim.x * blockDim.x) {
+    const int i = d / n1, j = d % n1;
+    const af3 p = ld3(dst + 3 * (size_t)d), lo = ld3(aabb + 6 * (size_t)d),
+              hi = ld3(aabb + 6 * (size_t)d + 3);
+    const float at[3] = {g.u0 + (float)i * du, g.v0 + (float)j * dv, g.w0};
+    for (int k = 0; k < 3; k++) {
+      const float x = comp3(p, ax[k]);
+      const float dev = fabsf(x - at[k]);
+      m[k] = dev < 3.0e38f ? fmaxf(m[k], dev) : 3.0e38f;  // a NaN too
+      m[3 + k] = fmaxf(m[3 + k], fmaxf(fabsf(comp3(hi, ax[k]) - x), fabsf(x - comp3(lo, ax[k]))));
+    }
   }
-  if (P.n_tri > 1) { q.phase = PH_SCENE; return; }
-  if (P.n_tri == 1) test_prim<0>(P.tri_prims, 0, q.r, q.best, 0.0f, q.Dq);
-  q.phase = PH_HIT;
+  for (int k = 0; k < 6; k++) {
+    const float v = warp_max(m[k]);
+    if ((threadIdx.x & 31) == 0)
+      atomicMax(reinterpret_cast<int *>(out) + k, __float_as_int(v));
+  }
+}
+__device__ __forceinline__ RxGrid rx_grid(const TraceDev &P) {
+  float du, dv;
+  RxGrid g = rx_grid_axes(P.dst, P.n0_dst, P.n1_dst, du, dv);
+  const float *m = P.rx_grid;
+  // (NaN compares false)
+  g.ok = g.ok && P.n0_dst > 0 && (P.n0_dst == 1 || m[0] <= 0.25f * fabsf(du)) &&
+         (P.n1_dst == 1 || m[1] <= 0.25f * fabsf(dv)) && m[2] <= m[5] && m[3] < 1e6f &&
+         m[4] < 1e6f && m[5] < 1e6f;
+  g.su = du;
+  g.sv = dv;
+  g.iu = du != 0.0f ? 1.0f / du : 0.0f;
+  g.iv = dv != 0.0f ? 1.0f / dv : 0.0f;
+  // 0.1 mm and 10 ppm of the place for rounding
+  g.bu = m[3] + m[0] + 1e-4f + 1e-5f * fabsf(g.u0);
+  g.bv = m[4] + m[1] + 1e-4f + 1e-5f * fabsf(g.v0);
+  g.bw = m[5] + m[2] + 1e-4f + 1e-5f * fabsf(g.w0);
+  return g;
+}
+// index range along one axis whose boxes the ray meets for t in [tn, tf]
+__device__ __forceinline__ void grid_range(float o, float d, float tn, float tf, float u0, float iu,
+                                           float b, int n, int &i0, int &i1) {
+  const float a0 = __fmaf_rn(tn, d, o), a1 = __fmaf_rn(tf, d, o);
+  // 20 ppm of the far end for its rounding
+  const float e = b + 2e-5f * fmaxf(fabsf(a0), fabsf(a1));
+  const float lo = fminf(a0, a1) - e - u0, hi = fmaxf(a0, a1) + e - u0;
+  if (iu == 0.0f) {  // one row
+    i0 = 0;
+    i1 = lo <= 0.0f && hi >= 0.0f ? 0 : -1;
+    return;
+  }
+  const float x = lo * iu, y = hi * iu;
+  i0 = (int)fminf(fmaxf(ceilf(fminf(x, y) - 1e-3f), 0.0f), (float)n);
+  i1 = (int)fmaxf(fminf(floorf(fmaxf(x, y) + 1e-3f), (float)(n - 1)), -1.0f);
+}
+// Closest Rx sphere by the grid: rows of the axis that the ray crosses more of,
+// in the order in which it meets them, until they lie behind the best hit.
+__device__ __forceinline__ void rx_by_grid(const TraceDev &P, const RxGrid &g, S1Query &q) {
+  const float ow = comp3(q.r.o, g.wa), iw = comp3(q.r.inv, g.wa);
+  const float t1 = (g.w0 - g.bw - ow) * iw, t2 = (g.w0 + g.bw - ow) * iw;
+  const float tn = fmaxf(__fmaf_rn(fminf(t1, t2), 0.9999f, -1e-4f), 0.0f);
+  // (a ray in the plane of the Rx stays in it: 1000 km stand for ever)
+  const float tf = fminf(__fmaf_rn(fmaxf(t1, t2), 1.0001f, 1e-4f), 1e6f);
+  if (!(tn <= tf)) return;
+  const float ou = comp3(q.r.o, g.ua), du = comp3(q.r.d, g.ua), ov = comp3(q.r.o, g.va),
+              dv = comp3(q.r.d, g.va);
+  int i0, i1, j0, j1;
+  grid_range(ou, du, tn, tf, g.u0, g.iu, g.bu, P.n0_dst, i0, i1);
+  grid_range(ov, dv, tn, tf, g.v0, g.iv, g.bv, P.n1_dst, j0, j1);
+  if (i1 < i0 || j1 < j0) return;
+  const bool by_u = i1 - i0 >= j1 - j0;  // rows of constant u or of constant v
+  const float oo = by_u ? ou : ov, io = comp3(q.r.inv, by_u ? g.ua : g.va),
+              o0 = by_u ? g.u0 : g.v0, so = by_u ? g.su : g.sv, bo = by_u ? g.bu : g.bv;
+  const float on = by_u ? ov : ou, dn = by_u ? dv : du, n0 = by_u ? g.v0 : g.u0,
+              in = by_u ? g.iv : g.iu, bn = by_u ? g.bv : g.bu;
+  const int nn = by_u ? P.n1_dst : P.n0_dst, step = by_u ? 1 : P.n1_dst,
+            row_step = by_u ? P.n1_dst : 1;
+  const int first = by_u ? i0 : j0, last = by_u ? i1 : j1;
+  const bool up = (io < 0.0f) == (so < 0.0f);
+#pragma unroll 1
+  for (int k = 0; k <= last - first; k++) {
+    const int row = up ? first + k : last - k;
+    const float c = o0 + (float)row * so - oo, ta = (c - bo) * io, tb = (c + bo) * io;
+    const float r0 = fmaxf(__fmaf_rn(fminf(ta, tb), 0.9999f, -1e-4f), tn),
+                r1 = fminf(__fmaf_rn(fmaxf(ta, tb), 1.0001f, 1e-4f), tf);
+    if (r0 > __fmaf_rn(q.best.t, 1.0001f, 1e-4f)) break;
+    if (!(r0 <= r1)) continue;
+    int a, b;
+    grid_range(on, dn, r0, r1, n0, in, bn, nn, a, b);
+#pragma unroll 1
+    for (; a <= b; a++) {
+      const int d = row * row_step + a * step;
+      const float *x = P.dst + 3 * (size_t)d;
+      const float t = sphere_hit(q.r, q.Dq, mk3(__ldg(x), __ldg(x + 1), __ldg(x + 2)), P.dst_r);
+      if (t >= 0.0f && better(t, 2, d, q.best)) {
+        const float *y = P.dst_aabb + 6 * (size_t)d;
+        if (prim_slab(q.r, make_float4(__ldg(y), __ldg(y + 1), __ldg(y + 2), 0.f),
+                      make_float4(__ldg(y + 3), __ldg(y + 4), __ldg(y + 5), 0.f))) {
+          q.best.t = t; q.best.inst = 2; q.best.prim = d;
+        }
+      }
+    }
+  }
 }
 
 struct S1Ray {
@@ -955,6 +1099,7 @@ __device__ __forceinline__ void s1_hit(const TraceDev &P, S1Query &q, S1Ray &w, 
       int cell = (d0 / P.gs) * P.n1g + d1 / P.gs;
       int hc = L + 1 - w.ttl;
       int mhc = 0;
+#pragma unroll 1
       for (int k = w.res_cnt - 1; k >= 0; k--)
         if ((rec[k] >> 3) == cell) { mhc = (rec[k] & 7) + 1; break; }
       if (mhc <= hc) {
@@ -1000,10 +1145,6 @@ __device__ __forceinline__ bool s1_next(const TraceDev &P, S1Query &q, S1Ray &w,
         w.ttl = 0;
         continue;
       }
-      ray_setup(q.r, q.r.o, q.r.d);
-      q.Dq = unit_dir(q.r);
-      q.best.t = AMS_TMAX; q.best.inst = 3; q.best.prim = 0x7fffffff;
-      s1_enter(P, q, PH_RX);
       return true;
     }
     if (w.pending) {
@@ -1065,7 +1206,7 @@ __device__ __forceinline__ bool s1_next(const TraceDev &P, S1Query &q, S1Ray &w,
 // LMAX bounds max_reflection: 2^LMAX branch slots (slot indices hold one bit
 // per hit count below L).
 template <int LMAX>
-__global__ void __launch_bounds__(128, 8) k_stage1(TraceDev P) {
+__global__ void __launch_bounds__(128, 8) k_stage1(const __grid_constant__ TraceDev P) {
   const long long tiles_y = (P.launch_y + 7) / 8;
   const long long n_fetch = (long long)((P.launch_x + 3) / 4) * tiles_y * 32;
   unsigned long long my_records = 0, my_segs = 0, my_capped = 0;
@@ -1073,93 +1214,90 @@ __global__ void __launch_bounds__(128, 8) k_stage1(TraceDev P) {
   const CurMatrix cm{curm};
   // path-table slot of the primary ray's key per hit count (-1: not known)
   __shared__ int s_los[AMS_MAX_L + 2];
+  __shared__ RxGrid s_grid;
   if (threadIdx.x < AMS_MAX_L + 2) s_los[threadIdx.x] = -1;
+  if (threadIdx.x == 32) s_grid = rx_grid(P);
   __syncthreads();
   int rec[AMS_MAX_RESERVE];  // cell * 8 + hit_cnt of the records kept so far
   Slot slots[1 << LMAX];     // deferred branch slots
-  int st_node[AMS_STACK];
-  float st_t[AMS_STACK];
+  int2 stack[AMS_STACK];     // node, its near distance
 
   S1Ray w;
   w.li = -1; w.ix = 0; w.iy = 0; w.launch = 0; w.res_cnt = 0; w.seed = 0u; w.capped = false;
   w.spos = mk3(0.f, 0.f, 0.f); w.pending = 0u; w.cur = 0; w.ttl = 0; w.guard = 0;
   w.key_cur = -1; w.key_ttl = 0; w.key_slot = -1;
   S1Query q;
-  ray_setup(q.r, mk3(0.f, 0.f, 0.f), mk3(0.f, 0.f, 1.f));
-  q.Dq = mk3(0.f, 0.f, 1.f);
-  q.best.t = AMS_TMAX; q.best.inst = 3; q.best.prim = 0x7fffffff;
-  q.phase = PH_HIT; q.node = 0; q.sp = 0;
+  q.r.o = mk3(0.f, 0.f, 0.f);
+  q.r.d = mk3(0.f, 0.f, 1.f);
   bool live = s1_next(P, q, w, slots, cm, n_fetch, tiles_y, my_capped);
 
-  while (__any_sync(0xffffffffu, live)) {
-    // ---- traversal: node visits until every lane's query has ended
-    while (true) {
-      const bool trav = live && q.phase != PH_HIT;
-      if (__ballot_sync(0xffffffffu, trav) == 0u) break;
-      if (trav) {
-        const bool rx = q.phase == PH_RX;
-        const BvhNode *nodes = rx ? P.rx_nodes : P.tri_nodes;
-        const float4 *prims = rx ? P.rx_prims : P.tri_prims;
-        const int n = rx ? P.n_dst : P.n_tri;
-        bool more = true;
-        if ((unsigned)q.node >= (unsigned)(n - 1)) {
-          atomicOr(P.err, AMS_DERR_BVH);
-          more = false;
-        } else {
-          const float4 *np = reinterpret_cast<const float4 *>(nodes + q.node);
-          const float4 a = __ldg(np), b = __ldg(np + 1), c = __ldg(np + 2);
-          const int4 d = __ldg(reinterpret_cast<const int4 *>(np + 3));
-          float tn0, tn1;
-          bool h0 = child_test(q.r, a.x, a.y, a.z, a.w, b.x, b.y, q.best.t, tn0);
-          bool h1 = child_test(q.r, b.z, b.w, c.x, c.y, c.z, c.w, q.best.t, tn1);
-          // leaves: one test site for both children
-          int lf0 = (h0 && d.x < 0) ? ~d.x : -1;
-          int lf1 = (h1 && d.y < 0) ? ~d.y : -1;
-          if (lf0 >= 0) h0 = false;
-          if (lf1 >= 0) h1 = false;
-          if (lf0 >= n || lf1 >= n) {
-            atomicOr(P.err, AMS_DERR_BVH);
-            more = false;
-          } else {
+  while (__any_sync(kFullWarp, live)) {
+    __syncwarp();
+    ray_setup(q.r, q.r.o, q.r.d);
+    q.Dq = unit_dir(q.r);
+    q.best.t = AMS_TMAX; q.best.inst = 3; q.best.prim = 0x7fffffff;
+    // ---- Rx spheres
+    if (s_grid.ok) {
+      if (live) rx_by_grid(P, s_grid, q);
+    } else if (live) {
+      q.best = traverse_rx(P, q.r.o, q.r.d, q.best);
+    }
+    __syncwarp();
+    // ---- scene, pruned at the sphere hit: node visits until every lane's
+    // query has ended
+    if (live && P.n_tri == 1) test_prim<0>(P.tri_prims, 0, q.r, q.best, 0.0f, q.Dq);
+    bool trav = live && P.n_tri > 1;
+    int node = 0, sp = 0;
+    while (trav) {
+      if ((unsigned)node >= (unsigned)(P.n_tri - 1)) {
+        atomicOr(P.err, AMS_DERR_BVH);
+        break;
+      }
+      const float4 *np = reinterpret_cast<const float4 *>(P.tri_nodes + node);
+      const float4 a = __ldg(np), b = __ldg(np + 1), c = __ldg(np + 2);
+      const int2 d = __ldg(reinterpret_cast<const int2 *>(np + 3));
+      float tn0, tn1;
+      bool h0 = child_test(q.r, a.x, a.y, a.z, a.w, b.x, b.y, q.best.t, tn0);
+      bool h1 = child_test(q.r, b.z, b.w, c.x, c.y, c.z, c.w, q.best.t, tn1);
+      // leaves: one test site for both children
+      const int lf0 = (h0 && d.x < 0) ? ~d.x : -1;
+      const int lf1 = (h1 && d.y < 0) ? ~d.y : -1;
+      if (lf0 >= 0) h0 = false;
+      if (lf1 >= 0) h1 = false;
+      if (lf0 >= P.n_tri || lf1 >= P.n_tri) {
+        atomicOr(P.err, AMS_DERR_BVH);
+        break;
+      }
 #pragma unroll 1
-            for (int k = 0; k < 2; k++) {
-              const int lf = k == 0 ? lf0 : lf1;
-              if (lf < 0) continue;
-              if (rx) test_prim<2>(prims, lf, q.r, q.best, P.dst_r, q.Dq);
-              else test_prim<0>(prims, lf, q.r, q.best, 0.0f, q.Dq);
-            }
-            if (h0 && h1) {
-              int nearn = d.x, farn = d.y;
-              float tfar = tn1;
-              if (tn1 < tn0) { nearn = d.y; farn = d.x; tfar = tn0; }
-              if (q.sp < AMS_STACK) {
-                st_node[q.sp] = farn; st_t[q.sp] = tfar; q.sp++;
-              } else {
-                atomicOr(P.err, AMS_DERR_STACK);
-              }
-              q.node = nearn;
-            } else if (h0) {
-              q.node = d.x;
-            } else if (h1) {
-              q.node = d.y;
-            } else {
-              more = false;
-              const float lim = __fmaf_rn(q.best.t, 1.0001f, 1e-4f);
-              while (q.sp > 0) {
-                q.sp--;
-                if (st_t[q.sp] <= lim) { q.node = st_node[q.sp]; more = true; break; }
-              }
-            }
-          }
+      for (int k = 0; k < 2; k++) {
+        const int lf = k == 0 ? lf0 : lf1;
+        if (lf >= 0) test_prim<0>(P.tri_prims, lf, q.r, q.best, 0.0f, q.Dq);
+      }
+      if (h0 && h1) {
+        const bool swap = tn1 < tn0;
+        if (sp < AMS_STACK) {
+          stack[sp++] = make_int2(swap ? d.x : d.y, __float_as_int(swap ? tn0 : tn1));
+        } else {
+          atomicOr(P.err, AMS_DERR_STACK);
         }
-        if (!more) {
-          if (rx) s1_enter(P, q, PH_SCENE);
-          else q.phase = PH_HIT;
+        node = swap ? d.y : d.x;
+      } else if (h0) {
+        node = d.x;
+      } else if (h1) {
+        node = d.y;
+      } else {
+        trav = false;
+        const float lim = __fmaf_rn(q.best.t, 1.0001f, 1e-4f);
+#pragma unroll 1
+        while (sp > 0) {
+          const int2 e = stack[--sp];
+          if (__int_as_float(e.y) <= lim) { node = e.x; trav = true; break; }
         }
       }
     }
-    // ---- hits of the waiting lanes, then their next queries
-    if (live && q.phase == PH_HIT) {
+    __syncwarp();
+    // ---- hits of all lanes, then their next queries
+    if (live) {
       my_segs++;
       s1_hit(P, q, w, slots, cm, s_los, rec, my_records);
       live = s1_next(P, q, w, slots, cm, n_fetch, tiles_y, my_capped);
@@ -1797,6 +1935,14 @@ cudaError_t trace_tx_info(const float *src, const float *aabb, int n, float *inf
   if (e != cudaSuccess) return e;
   const int blocks = n > kTxPairs ? 1 : std::min(n, 304);
   k_tx_info<<<blocks, 256, 0, st>>>(src, aabb, n, info);
+  return cudaGetLastError();
+}
+
+cudaError_t trace_rx_grid(const float *dst, const float *aabb, int n0, int n1, float *out,
+                          cudaStream_t st) {
+  cudaError_t e = cudaMemsetAsync(out, 0, 4 * 8, st);
+  if (e != cudaSuccess) return e;
+  k_rx_grid<<<grid_for((long long)n0 * n1, 256), 256, 0, st>>>(dst, aabb, n0, n1, out);
   return cudaGetLastError();
 }
 

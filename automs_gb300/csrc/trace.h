@@ -47,6 +47,8 @@ struct TraceDev {
   const float4 *rx_prims;
   int n_dst;
   const float *dst;  // original order [n_dst, 3]
+  const float *dst_aabb;  // original order [n_dst, 6]
+  const float *rx_grid;   // trace_rx_grid
   float dst_r;
   // Rx grid and cells
   int n0_dst, n1_dst, n0g, n1g, ng, gs;
@@ -106,6 +108,9 @@ struct TraceDev {
 cudaError_t trace_tri_attr(const float *tris, int n, float4 *attr, cudaStream_t st);
 // shape of the Tx array, 16 floats (k_tx_info in trace.cu)
 cudaError_t trace_tx_info(const float *src, const float *aabb, int n, float *info,
+                          cudaStream_t st);
+// how the Rx set fits an axis-aligned grid, 8 floats (RxGrid in trace.cu)
+cudaError_t trace_rx_grid(const float *dst, const float *aabb, int n0, int n1, float *out,
                           cudaStream_t st);
 cudaError_t trace_stage1(const TraceDev &P, cudaStream_t st);
 // dense path ids (dense_of [slots], P.slot_of) and the stage-1 bitmap
