@@ -480,32 +480,37 @@ ams_status trace_impl(ams_scene *S, const ams_trace_params *p, const float *src,
     P.rec = records;
     P.rec_cap = records ? max_records : 0;
     P.rec_base = 0;
-    P.tab_h = S->ws.take<unsigned long long>(tab_size);
-    P.tab_key = S->ws.take<int32_t>(14 * (size_t)tab_size);
-    P.T = S->ws.take<unsigned>((size_t)ng * W);
     P.N = S->ws.take<unsigned>((size_t)ng * W);
-    P.S = S->ws.take<unsigned>((size_t)ng * W);
     P.cell_off = S->ws.take<int>((size_t)ng + 1);
     P.chunk_off = S->ws.take<int>((size_t)ng + 1);
     P.cell_cnt = S->ws.take<int>((size_t)ng);
     P.slot_of = S->ws.take<int>(tab_size);
     int *dense_of = S->ws.take<int>(tab_size);
-    P.acc = S->ws.take<unsigned long long>(2 * (size_t)n_src * n_dst);
+    // what starts at zero, in one block
+    char *zero = S->ws.take<char>(0);
     char *counters = S->ws.take<char>(kCounterBytes);
+    float *tx_info = S->ws.take<float>(16);
+    float *rx_grid = S->ws.take<float>(8);
+    P.tab_h = S->ws.take<unsigned long long>(tab_size);
+    P.tab_key = S->ws.take<int32_t>(14 * (size_t)tab_size);  // 0 = word not written
+    P.T = S->ws.take<unsigned>((size_t)ng * W);
+    P.S = S->ws.take<unsigned>((size_t)ng * W);
+    P.acc = S->ws.take<unsigned long long>(2 * (size_t)n_src * n_dst);
+    const size_t zero_bytes = (size_t)(S->ws.take<char>(0) - zero);
     P.ctr = reinterpret_cast<unsigned long long *>(counters);
     P.rounds = reinterpret_cast<RoundCount *>(counters + offsetof(HostCounters, rounds));
     P.err = reinterpret_cast<unsigned *>(counters + offsetof(HostCounters, err));
     P.round_slot = 0;
-    float *tx_info = S->ws.take<float>(16);
-    float *rx_grid = S->ws.take<float>(8);
 
+    CK(cudaMemsetAsync(zero, 0, zero_bytes, st));
     if (!src_aabb) { CK(sphere_aabbs(src, n_src, p->src_r, sbox, st)); src_aabb = sbox; }
     if (!dst_aabb) { CK(sphere_aabbs(dst, n_dst, p->dst_r, dbox, st)); dst_aabb = dbox; }
     Lbvh tx, rx;
-    CK(lbvh_build_spheres(tx, src, src_aabb, n_src, scratch, tx_out, st));
-    CK(lbvh_build_spheres(rx, dst, dst_aabb, n_dst, scratch, rx_out, st));
+    CK(lbvh_build_spheres(tx, src, src_aabb, n_src, scratch, tx_out, nullptr, st));
     CK(trace_tx_info(src, src_aabb, n_src, tx_info, st));
     CK(trace_rx_grid(dst, dst_aabb, n0, n1, rx_grid, st));
+    CK(lbvh_build_spheres(rx, dst, dst_aabb, n_dst, scratch, rx_out,
+                          reinterpret_cast<const int *>(rx_grid) + 7, st));
     CK(cudaEventRecord(ev[1], st));
 
     P.tris = S->tris;
@@ -539,13 +544,6 @@ ams_status trace_impl(ams_scene *S, const ams_trace_params *p, const float *src,
     P.tab_mask = tab_size - 1;
     P.tab_limit = tab_size / 2;
     P.W = W;
-
-    CK(cudaMemsetAsync(P.tab_h, 0, 8 * (size_t)tab_size, st));
-    CK(cudaMemsetAsync(P.tab_key, 0, 56 * (size_t)tab_size, st));  // 0 = word not written
-    CK(cudaMemsetAsync(P.T, 0, 4 * (size_t)ng * W, st));
-    CK(cudaMemsetAsync(P.S, 0, 4 * (size_t)ng * W, st));
-    CK(cudaMemsetAsync(P.acc, 0, 16 * (size_t)n_src * n_dst, st));
-    CK(cudaMemsetAsync(counters, 0, kCounterBytes, st));
 
     // ---- stage 1
     CK(trace_stage1(P, st));

@@ -30,7 +30,8 @@ __device__ __forceinline__ float widen_hi(float v) {
   return nextafterf(v + (1e-6f + 1e-6f * fabsf(v)), 3.0e38f);
 }
 
-__global__ void k_bounds(const PrimBox *boxes, int n, float *out6) {
+// centroid bounds of the boxes, by one CTA of up to 1024 threads
+__device__ __forceinline__ void centroid_bounds(const PrimBox *boxes, int n, float *out6) {
   __shared__ float s[6][32];
   float lo[3] = {3.0e38f, 3.0e38f, 3.0e38f}, hi[3] = {-3.0e38f, -3.0e38f, -3.0e38f};
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
@@ -64,6 +65,11 @@ __global__ void k_bounds(const PrimBox *boxes, int n, float *out6) {
   }
 }
 
+__global__ void k_bounds(const PrimBox *boxes, int n, float *out6, const int *skip) {
+  if (skip && *skip) return;
+  centroid_bounds(boxes, n, out6);
+}
+
 __device__ __forceinline__ uint32_t expand10(uint32_t v) {
   v = (v * 0x00010001u) & 0xFF0000FFu;
   v = (v * 0x00000101u) & 0x0F00F00Fu;
@@ -72,10 +78,7 @@ __device__ __forceinline__ uint32_t expand10(uint32_t v) {
   return v;
 }
 
-__global__ void k_morton(const PrimBox *boxes, int n, const float *b6, uint64_t *keys) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const PrimBox b = boxes[i];
+__device__ __forceinline__ uint64_t morton_key(const PrimBox &b, int i, const float *b6) {
   uint32_t q[3];
   // one scale for all axes (the largest centroid extent): a flat room or
   // building gets its first splits across its long sides instead of cutting
@@ -98,12 +101,19 @@ __global__ void k_morton(const PrimBox *boxes, int n, const float *b6, uint64_t 
     sext = fmaxf(sext, b6[3 + k] - b6[k]);
   }
   if (sext > 0.0f && bext > 0.25f * sext) m |= 1u << 30;
-  keys[i] = ((uint64_t)m << 32) | (uint32_t)i;
+  return ((uint64_t)m << 32) | (uint32_t)i;
+}
+__global__ void k_morton(const PrimBox *boxes, int n, const float *b6, uint64_t *keys,
+                         const int *skip) {
+  if (skip && *skip) return;
+  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) keys[i] = morton_key(boxes[i], i, b6);
 }
 
 // Stable LSD radix sort of 64-bit items on their upper 32 bits (30 used),
 // one CTA of 1024 threads, tiles of 1024 items in order.
-__global__ void __launch_bounds__(1024) k_sort(uint64_t *a, uint64_t *b, int n) {
+__global__ void __launch_bounds__(1024) k_sort(uint64_t *a, uint64_t *b, int n, const int *skip) {
+  if (skip && *skip) return;
   __shared__ int hist[16];
   __shared__ int base[16];
   __shared__ int wcnt[32][16];
@@ -150,17 +160,8 @@ __global__ void __launch_bounds__(1024) k_sort(uint64_t *a, uint64_t *b, int n) 
   // 8 passes: the sorted data is back in `a`
 }
 
-// Up to kSmemSortMax keys: bitonic sort in shared memory, one CTA of 1024
-// threads (log2(n) (log2(n) + 1) / 2 compare-exchange steps).  The keys are
-// unique (primitive index in the low word), so the order equals the stable
-// radix sort's.  Padding slots hold ~0, which sorts last.
-constexpr int kSmemSortMax = 16384;
-__global__ void __launch_bounds__(1024) k_sort_smem(uint64_t *a, int n) {
-  extern __shared__ uint64_t sk[];
-  int np = 1;
-  while (np < n) np <<= 1;
-  for (int i = threadIdx.x; i < np; i += blockDim.x) sk[i] = i < n ? a[i] : ~0ull;
-  __syncthreads();
+// ascending bitonic sort of np (a power of two) keys in shared memory
+__device__ __forceinline__ void bitonic_sort(uint64_t *sk, int np) {
   // each step visits its np / 2 compare-exchange pairs (i, i + j) directly
   for (int k = 2; k <= np; k <<= 1) {
     for (int j = k >> 1; j > 0; j >>= 1) {
@@ -174,6 +175,20 @@ __global__ void __launch_bounds__(1024) k_sort_smem(uint64_t *a, int n) {
       __syncthreads();
     }
   }
+}
+// Up to kSmemSortMax keys: bitonic sort in shared memory, one CTA of 1024
+// threads (log2(n) (log2(n) + 1) / 2 compare-exchange steps).  The keys are
+// unique (primitive index in the low word), so the order equals the stable
+// radix sort's.  Padding slots hold ~0, which sorts last.
+constexpr int kSmemSortMax = 16384;
+__global__ void __launch_bounds__(1024) k_sort_smem(uint64_t *a, int n, const int *skip) {
+  if (skip && *skip) return;
+  extern __shared__ uint64_t sk[];
+  int np = 1;
+  while (np < n) np <<= 1;
+  for (int i = threadIdx.x; i < np; i += blockDim.x) sk[i] = i < n ? a[i] : ~0ull;
+  __syncthreads();
+  bitonic_sort(sk, np);
   for (int i = threadIdx.x; i < n; i += blockDim.x) a[i] = sk[i];
 }
 
@@ -182,10 +197,10 @@ __device__ __forceinline__ int delta(const uint64_t *k, int n, int i, int j) {
   return __clzll(k[i] ^ k[j]);  // keys are unique (index in the low word)
 }
 
-__global__ void k_karras(const uint64_t *keys, int n, BvhNode *nodes, int *parent) {
+// internal node i of the hierarchy over the sorted keys
+__device__ __forceinline__ void karras_node(const uint64_t *keys, int n, int i, BvhNode *nodes,
+                                            int *parent) {
   // parent[0 .. n-2]: internal nodes, parent[n-1 .. 2n-2]: leaves
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n - 1) return;
   int d = (delta(keys, n, i, i + 1) - delta(keys, n, i, i - 1)) >= 0 ? 1 : -1;
   int dmin = delta(keys, n, i, i - d);
   int lmax = 2;
@@ -212,6 +227,12 @@ __global__ void k_karras(const uint64_t *keys, int n, BvhNode *nodes, int *paren
   if (right >= 0) parent[right] = i; else parent[(n - 1) + ~right] = i;
   if (i == 0) parent[0] = -1;
 }
+__global__ void k_karras(const uint64_t *keys, int n, BvhNode *nodes, int *parent,
+                         const int *skip) {
+  if (skip && *skip) return;
+  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n - 1) karras_node(keys, n, i, nodes, parent);
+}
 
 __device__ __forceinline__ void store_child(BvhNode &nd, int which, const float lo[3],
                                             const float hi[3]) {
@@ -226,10 +247,10 @@ __device__ __forceinline__ void store_child(BvhNode &nd, int which, const float 
   }
 }
 
-__global__ void k_refit(const uint64_t *keys, const PrimBox *boxes, int n, BvhNode *nodes,
-                        const int *parent, int *flags, float *node_box, int *perm) {
-  int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= n) return;
+// boxes from sorted leaf j upwards, as far as it is the second to arrive
+__device__ __forceinline__ void refit_from(const uint64_t *keys, const PrimBox *boxes, int n, int j,
+                                           BvhNode *nodes, const int *parent, int *flags,
+                                           float *node_box, int *perm) {
   int orig = (int)(keys[j] & 0xffffffffu);
   perm[j] = orig;
   if (n == 1) return;
@@ -262,47 +283,100 @@ __global__ void k_refit(const uint64_t *keys, const PrimBox *boxes, int n, BvhNo
     p = parent[p];
   }
 }
+__global__ void k_refit(const uint64_t *keys, const PrimBox *boxes, int n, BvhNode *nodes,
+                        const int *parent, int *flags, float *node_box, int *perm,
+                        const int *skip) {
+  if (skip && *skip) return;
+  int j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j < n) refit_from(keys, boxes, n, j, nodes, parent, flags, node_box, perm);
+}
 
-__global__ void k_tri_boxes(const float *tris, int n, PrimBox *boxes) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+__device__ __forceinline__ PrimBox tri_box(const float *tris, int i) {
   const float *v = tris + (size_t)i * 9;
   PrimBox b;
   for (int k = 0; k < 3; k++) {
     b.lo[k] = fminf(fminf(v[k], v[3 + k]), v[6 + k]);
     b.hi[k] = fmaxf(fmaxf(v[k], v[3 + k]), v[6 + k]);
   }
-  boxes[i] = b;
+  return b;
+}
+__global__ void k_tri_boxes(const float *tris, int n, PrimBox *boxes) {
+  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) boxes[i] = tri_box(tris, i);
 }
 
-__global__ void k_aabb_boxes(const float *aabb, int n, PrimBox *boxes) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+__device__ __forceinline__ PrimBox aabb_box(const float *aabb, int i) {
   PrimBox b;
   for (int k = 0; k < 3; k++) { b.lo[k] = aabb[6 * i + k]; b.hi[k] = aabb[6 * i + 3 + k]; }
-  boxes[i] = b;
+  return b;
+}
+__global__ void k_aabb_boxes(const float *aabb, int n, PrimBox *boxes, const int *skip) {
+  if (skip && *skip) return;
+  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) boxes[i] = aabb_box(aabb, i);
 }
 
 // sorted triangle data: v0 (w = original index), v1, v2
-__global__ void k_pack_tris(const float *tris, const int *perm, int n, float4 *out) {
-  int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= n) return;
-  int o = perm[j];
+__device__ __forceinline__ void pack_tri(const float *tris, int o, int j, float4 *out) {
   const float *v = tris + (size_t)o * 9;
   out[3 * j + 0] = make_float4(v[0], v[1], v[2], __int_as_float(o));
   out[3 * j + 1] = make_float4(v[3], v[4], v[5], 0.0f);
   out[3 * j + 2] = make_float4(v[6], v[7], v[8], 0.0f);
 }
+__global__ void k_pack_tris(const float *tris, const int *perm, int n, float4 *out) {
+  int j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j < n) pack_tri(tris, perm[j], j, out);
+}
 
 // sorted sphere data: centre (w = original index), box lo, box hi
-__global__ void k_pack_spheres(const float *pos, const float *aabb, const int *perm, int n,
-                               float4 *out) {
-  int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= n) return;
-  int o = perm[j];
+__device__ __forceinline__ void pack_sphere(const float *pos, const float *aabb, int o, int j,
+                                            float4 *out) {
   out[3 * j + 0] = make_float4(pos[3 * o], pos[3 * o + 1], pos[3 * o + 2], __int_as_float(o));
   out[3 * j + 1] = make_float4(aabb[6 * o], aabb[6 * o + 1], aabb[6 * o + 2], 0.0f);
   out[3 * j + 2] = make_float4(aabb[6 * o + 3], aabb[6 * o + 4], aabb[6 * o + 5], 0.0f);
+}
+__global__ void k_pack_spheres(const float *pos, const float *aabb, const int *perm, int n,
+                               float4 *out, const int *skip) {
+  if (skip && *skip) return;
+  int j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j < n) pack_sphere(pos, aabb, perm[j], j, out);
+}
+
+// The whole build for up to kSmallMax primitives in one CTA: every step above
+// with barriers between (a Tx array took seven launches and a memset, 20 us of
+// launch gaps and 60 us of host time for both sphere sets).  TRI: pos holds
+// the triangles, aabb nothing.
+constexpr int kSmallMax = 2048;
+template <bool TRI>
+__global__ void __launch_bounds__(1024) k_lbvh_small(const float *pos, const float *aabb, int n,
+                                                     PrimBox *boxes, int *parent, int *flags,
+                                                     float *node_box, BvhNode *nodes, int *perm,
+                                                     float4 *prims, const int *skip) {
+  if (skip && *skip) return;
+  __shared__ uint64_t key[kSmallMax];
+  __shared__ float b6[6];
+  const int t = threadIdx.x;
+  for (int i = t; i < n; i += blockDim.x) {
+    boxes[i] = TRI ? tri_box(pos, i) : aabb_box(aabb, i);
+    flags[i] = 0;
+  }
+  __syncthreads();
+  centroid_bounds(boxes, n, b6);
+  __syncthreads();
+  int np = 1;
+  while (np < n) np <<= 1;
+  for (int i = t; i < np; i += blockDim.x) key[i] = i < n ? morton_key(boxes[i], i, b6) : ~0ull;
+  __syncthreads();
+  bitonic_sort(key, np);
+  for (int i = t; i < n - 1; i += blockDim.x) karras_node(key, n, i, nodes, parent);
+  __syncthreads();
+  for (int i = t; i < n; i += blockDim.x)
+    refit_from(key, boxes, n, i, nodes, parent, flags, node_box, perm);
+  for (int i = t; i < n; i += blockDim.x) {
+    const int o = (int)(key[i] & 0xffffffffu);
+    if (TRI) pack_tri(pos, o, i, prims);
+    else pack_sphere(pos, aabb, o, i, prims);
+  }
 }
 
 __global__ void k_sphere_aabbs(const float *pos, int n, float r, float *aabb) {
@@ -442,8 +516,10 @@ size_t lbvh_output_bytes(int n) {
          al(sizeof(float4) * 3 * (size_t)n);
 }
 
-static cudaError_t build_common(Lbvh &out, int n, char *scratch, char *outbuf,
-                                cudaStream_t st) {
+// pos / aabb as k_lbvh_small takes them; beyond kSmallMax primitives the boxes
+// are in scratch already
+static cudaError_t build_common(Lbvh &out, const float *pos, const float *aabb, int n,
+                                char *scratch, char *outbuf, const int *skip, cudaStream_t st) {
   auto al = [](size_t v) { return (v + 255) & ~(size_t)255; };
   PrimBox *boxes = (PrimBox *)scratch;
   char *p = scratch + al(sizeof(PrimBox) * (size_t)n);
@@ -458,41 +534,52 @@ static cudaError_t build_common(Lbvh &out, int n, char *scratch, char *outbuf,
   out.perm = (int *)(outbuf + al(sizeof(BvhNode) * (size_t)(n > 1 ? n - 1 : 1)));
   out.prims = (float4 *)((char *)out.perm + al(sizeof(int) * (size_t)n));
   if (n == 0) return cudaSuccess;
-  k_bounds<<<1, 1024, 0, st>>>(boxes, n, b6);
-  k_morton<<<nblk(n, 256), 256, 0, st>>>(boxes, n, b6, ka);
+  if (n <= kSmallMax) {
+    if (aabb)
+      k_lbvh_small<false><<<1, 1024, 0, st>>>(pos, aabb, n, boxes, parent, flags, nbox, out.nodes,
+                                              out.perm, out.prims, skip);
+    else
+      k_lbvh_small<true><<<1, 1024, 0, st>>>(pos, aabb, n, boxes, parent, flags, nbox, out.nodes,
+                                             out.perm, out.prims, skip);
+    return cudaGetLastError();
+  }
+  k_bounds<<<1, 1024, 0, st>>>(boxes, n, b6, skip);
+  k_morton<<<nblk(n, 256), 256, 0, st>>>(boxes, n, b6, ka, skip);
   if (n <= kSmemSortMax) {
     static size_t attr_set[AMS_MAX_DEVICES] = {0};
     cudaError_t e = ams_set_smem_atleast(attr_set, k_sort_smem, kSmemSortMax * sizeof(uint64_t));
     if (e != cudaSuccess) return e;
     int np = 1;
     while (np < n) np <<= 1;
-    k_sort_smem<<<1, 1024, np * sizeof(uint64_t), st>>>(ka, n);
+    k_sort_smem<<<1, 1024, np * sizeof(uint64_t), st>>>(ka, n, skip);
   } else {
-    k_sort<<<1, 1024, 0, st>>>(ka, kb, n);
+    k_sort<<<1, 1024, 0, st>>>(ka, kb, n, skip);
   }
   if (n > 1) {
-    k_karras<<<nblk(n - 1, 256), 256, 0, st>>>(ka, n, out.nodes, parent);
+    k_karras<<<nblk(n - 1, 256), 256, 0, st>>>(ka, n, out.nodes, parent, skip);
     cudaMemsetAsync(flags, 0, sizeof(int) * (size_t)n, st);
   }
-  k_refit<<<nblk(n, 256), 256, 0, st>>>(ka, boxes, n, out.nodes, parent, flags, nbox, out.perm);
+  k_refit<<<nblk(n, 256), 256, 0, st>>>(ka, boxes, n, out.nodes, parent, flags, nbox, out.perm,
+                                        skip);
   return cudaGetLastError();
 }
 
 cudaError_t lbvh_build_triangles(Lbvh &out, const float *tris, int n, char *scratch,
                                  char *outbuf, cudaStream_t st) {
-  if (n > 0) k_tri_boxes<<<nblk(n, 256), 256, 0, st>>>(tris, n, (PrimBox *)scratch);
-  cudaError_t e = build_common(out, n, scratch, outbuf, st);
-  if (e != cudaSuccess || n == 0) return e;
+  if (n > kSmallMax) k_tri_boxes<<<nblk(n, 256), 256, 0, st>>>(tris, n, (PrimBox *)scratch);
+  cudaError_t e = build_common(out, tris, nullptr, n, scratch, outbuf, nullptr, st);
+  if (e != cudaSuccess || n <= kSmallMax) return e;
   k_pack_tris<<<nblk(n, 256), 256, 0, st>>>(tris, out.perm, n, out.prims);
   return cudaGetLastError();
 }
 
 cudaError_t lbvh_build_spheres(Lbvh &out, const float *pos, const float *aabb, int n,
-                               char *scratch, char *outbuf, cudaStream_t st) {
-  if (n > 0) k_aabb_boxes<<<nblk(n, 256), 256, 0, st>>>(aabb, n, (PrimBox *)scratch);
-  cudaError_t e = build_common(out, n, scratch, outbuf, st);
-  if (e != cudaSuccess || n == 0) return e;
-  k_pack_spheres<<<nblk(n, 256), 256, 0, st>>>(pos, aabb, out.perm, n, out.prims);
+                               char *scratch, char *outbuf, const int *skip, cudaStream_t st) {
+  if (n > kSmallMax)
+    k_aabb_boxes<<<nblk(n, 256), 256, 0, st>>>(aabb, n, (PrimBox *)scratch, skip);
+  cudaError_t e = build_common(out, pos, aabb, n, scratch, outbuf, skip, st);
+  if (e != cudaSuccess || n <= kSmallMax) return e;
+  k_pack_spheres<<<nblk(n, 256), 256, 0, st>>>(pos, aabb, out.perm, n, out.prims, skip);
   return cudaGetLastError();
 }
 

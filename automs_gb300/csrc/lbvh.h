@@ -39,8 +39,9 @@ size_t lbvh_scratch_bytes(int n);
 size_t lbvh_output_bytes(int n);
 cudaError_t lbvh_build_triangles(Lbvh &out, const float *tris, int n, char *scratch,
                                  char *outbuf, cudaStream_t st);
+// with `skip` (device) and a value other than 0 there, nothing is built
 cudaError_t lbvh_build_spheres(Lbvh &out, const float *pos, const float *aabb, int n,
-                               char *scratch, char *outbuf, cudaStream_t st);
+                               char *scratch, char *outbuf, const int *skip, cudaStream_t st);
 // adopts a hierarchy built on the host (bvh_sah.h) for triangles already on
 // the device: copies nodes and perm into outbuf (the caller keeps the host
 // arrays alive until the stream has run) and packs the sorted triangles

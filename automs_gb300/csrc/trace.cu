@@ -899,7 +899,9 @@ struct S1Query {
 // u and v intervals give the few Rx that it can meet; they are tested one by
 // one with the tests that the hierarchy's leaves get.  rx_grid words: 0-2 the
 // largest deviation of an Rx from its place in the grid along u, v, w; 3-5 the
-// largest extent of a box from its Rx.
+// largest extent of a box from its Rx; 6 counts the CTAs of k_rx_grid that are
+// done, whose last one writes 7: 1 where the grid can be used (the hierarchy
+// of the Rx is not built then).
 struct RxGrid {
   int ok, ua, va, wa;
   float u0, su, iu, v0, sv, iv, w0;  // steps and their inverses, 0 where there is one row
@@ -952,15 +954,24 @@ __global__ void __launch_bounds__(256) k_rx_grid(const float *dst, const float *
     if ((threadIdx.x & 31) == 0)
       atomicMax(reinterpret_cast<int *>(out) + k, __float_as_int(v));
   }
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x != 0 ||
+      atomicAdd(reinterpret_cast<int *>(out) + 6, 1) != (int)gridDim.x - 1)
+    return;
+  __threadfence();
+  for (int k = 0; k < 6; k++) m[k] = __ldcg(out + k);
+  // (NaN compares false)
+  const bool ok = g.ok && (n0 == 1 || m[0] <= 0.25f * fabsf(du)) &&
+                  (n1 == 1 || m[1] <= 0.25f * fabsf(dv)) && m[2] <= m[5] && m[3] < 1e6f &&
+                  m[4] < 1e6f && m[5] < 1e6f;
+  reinterpret_cast<int *>(out)[7] = ok ? 1 : 0;
 }
 __device__ __forceinline__ RxGrid rx_grid(const TraceDev &P) {
   float du, dv;
   RxGrid g = rx_grid_axes(P.dst, P.n0_dst, P.n1_dst, du, dv);
   const float *m = P.rx_grid;
-  // (NaN compares false)
-  g.ok = g.ok && P.n0_dst > 0 && (P.n0_dst == 1 || m[0] <= 0.25f * fabsf(du)) &&
-         (P.n1_dst == 1 || m[1] <= 0.25f * fabsf(dv)) && m[2] <= m[5] && m[3] < 1e6f &&
-         m[4] < 1e6f && m[5] < 1e6f;
+  g.ok = reinterpret_cast<const int *>(m)[7];
   g.su = du;
   g.sv = dv;
   g.iu = du != 0.0f ? 1.0f / du : 0.0f;
@@ -1322,9 +1333,9 @@ __global__ void __launch_bounds__(128, 8) k_stage1(const __grid_constant__ Trace
 // directions that the array is thin along (the normal of a planar array
 // twice, two normals of a linear one), each with the sine above which a ray
 // meets one Tx only; then the box of all Tx boxes, widened as a node's.  Word
-// 11 holds the square of the smallest distance of two Tx, word 15 counts the
-// CTAs that have done their share of the pairs (the memory is set to
-// 0x7f7f7f7f before); the last one, or CTA 0 alone beyond kTxPairs Tx where no
+// 11 holds the square of the smallest distance of two Tx (the bits of the
+// largest float less its own, so that 0 stands for the largest), word 15 counts
+// the CTAs that have done their share of the pairs; the last one, or CTA 0 alone beyond kTxPairs Tx where no
 // ray counts as steep enough, writes the rest.
 constexpr int kTxPairs = 4096;
 __global__ void __launch_bounds__(256) k_tx_info(const float *src, const float *aabb, int n,
@@ -1343,12 +1354,13 @@ __global__ void __launch_bounds__(256) k_tx_info(const float *src, const float *
       }
     }
     best = warp_min(best);
-    if (lane == 0) atomicMin(reinterpret_cast<int *>(info) + 11, __float_as_int(best));
+    if (lane == 0)
+      atomicMax(reinterpret_cast<int *>(info) + 11, 0x7f7fffff - __float_as_int(best));
   }
   __threadfence();
   __syncthreads();
   if (t == 0)
-    fit = atomicAdd(reinterpret_cast<int *>(info) + 15, 1) == 0x7f7f7f7f + (int)gridDim.x - 1;
+    fit = atomicAdd(reinterpret_cast<int *>(info) + 15, 1) == (int)gridDim.x - 1;
   __syncthreads();
   if (!fit) return;
   __threadfence();
@@ -1409,7 +1421,8 @@ __global__ void __launch_bounds__(256) k_tx_info(const float *src, const float *
     // two Tx may lie on either side of the first; 20 um of slack for the
     // rounding of positions and box tests over a building
     const float rho = 2.0f * (rh + 2e-5f);
-    const float gap = n <= kTxPairs ? sqrtf(__ldcg(info + 11)) - rho : 0.0f;
+    const float d2 = __int_as_float(0x7f7fffff - __ldcg(reinterpret_cast<int *>(info) + 11));
+    const float gap = n <= kTxPairs ? sqrtf(d2) - rho : 0.0f;
     float4 *o = reinterpret_cast<float4 *>(info);
     o[0] = make_float4(n1.x, n1.y, n1.z, gap > 0.0f ? (2.0f * e1 + rho) / gap + 1e-3f : 3.0e38f);
     o[1] = make_float4(n2.x, n2.y, n2.z, gap > 0.0f ? (2.0f * e2 + rho) / gap + 1e-3f : 3.0e38f);
@@ -1931,8 +1944,6 @@ cudaError_t trace_tri_attr(const float *tris, int n, float4 *attr, cudaStream_t 
 
 cudaError_t trace_tx_info(const float *src, const float *aabb, int n, float *info,
                           cudaStream_t st) {
-  cudaError_t e = cudaMemsetAsync(info, 0x7f, 4 * 16, st);
-  if (e != cudaSuccess) return e;
   const int blocks = n > kTxPairs ? 1 : std::min(n, 304);
   k_tx_info<<<blocks, 256, 0, st>>>(src, aabb, n, info);
   return cudaGetLastError();
@@ -1940,8 +1951,6 @@ cudaError_t trace_tx_info(const float *src, const float *aabb, int n, float *inf
 
 cudaError_t trace_rx_grid(const float *dst, const float *aabb, int n0, int n1, float *out,
                           cudaStream_t st) {
-  cudaError_t e = cudaMemsetAsync(out, 0, 4 * 8, st);
-  if (e != cudaSuccess) return e;
   k_rx_grid<<<grid_for((long long)n0 * n1, 256), 256, 0, st>>>(dst, aabb, n0, n1, out);
   return cudaGetLastError();
 }
