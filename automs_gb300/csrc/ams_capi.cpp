@@ -1126,23 +1126,25 @@ unsigned long long ams_scratch_bytes(void) {
 struct ams_mlp {
   MlpDev dev;
   char *arena = nullptr;
+  unsigned *flags = nullptr;  // dev.err as the host sees it
   ~ams_mlp() {
     if (arena) cudaFree(arena);
+    if (flags) cudaFreeHost(flags);
   }
 };
 
 namespace {
 ams_status mlp_check_err(ams_mlp *m, cudaStream_t st, char *errbuf, size_t errlen) {
-  unsigned e = 0;
-  cudaError_t ce = cudaMemcpyAsync(&e, m->dev.err, 4, cudaMemcpyDeviceToHost, st);
-  if (ce == cudaSuccess) ce = cudaStreamSynchronize(st);
+  // the kernels set the flags in mapped host memory: nothing to copy
+  const cudaError_t ce = cudaStreamSynchronize(st);
   if (ce != cudaSuccess) {
     set_err(errbuf, errlen, "MLP: %s", cudaGetErrorString(ce));
     return AMS_ERR_CUDA;
   }
+  const unsigned e = *(volatile unsigned *)m->flags;
   if (e) {
     set_err(errbuf, errlen, "tensor-core GEMM timed out waiting (flags 0x%x)", e);
-    cudaMemsetAsync(m->dev.err, 0, 4, st);
+    *m->flags = 0;
     return AMS_ERR_INTERNAL;
   }
   return AMS_OK;
@@ -1220,8 +1222,8 @@ ams_status ams_mlp_create(const int *dims, int n_dims, int max_batch, unsigned l
   size_t off_W[kMlpMaxLayers + 1], off_b[kMlpMaxLayers + 1], off_mW[kMlpMaxLayers + 1],
       off_vW[kMlpMaxLayers + 1], off_mb[kMlpMaxLayers + 1], off_vb[kMlpMaxLayers + 1],
       off_gW[kMlpMaxLayers + 1], off_gb[kMlpMaxLayers + 1], off_Wb[kMlpMaxLayers + 1],
-      off_Wt[kMlpMaxLayers + 1], off_H[kMlpMaxLayers + 1], off_dZ[kMlpMaxLayers + 1];
-  size_t maxw = 0;
+      off_Wt[kMlpMaxLayers + 1], off_H[kMlpMaxLayers + 1], off_dZ[kMlpMaxLayers + 1],
+      off_Ht[kMlpMaxLayers + 1], off_dZt[kMlpMaxLayers + 1];
   for (int l = 1; l <= d.L; l++) {
     size_t n = (size_t)d.d[l] * d.dp[l - 1];
     off_W[l] = add(4 * n); off_mW[l] = add(4 * n); off_vW[l] = add(4 * n); off_gW[l] = add(4 * n);
@@ -1229,13 +1231,19 @@ ams_status ams_mlp_create(const int *dims, int n_dims, int max_batch, unsigned l
     off_gb[l] = add(4 * d.d[l]);
     off_Wb[l] = add(2 * n); off_Wt[l] = add(2 * n);
     off_dZ[l] = add(2 * (size_t)d.max_bp * d.dp[l]);
-    maxw = std::max(maxw, (size_t)std::max(d.dp[l], d.dp[l - 1]));
+    off_dZt[l] = add(2 * (size_t)d.max_bp * d.dp[l]);
   }
-  for (int l = 0; l < d.L; l++) off_H[l] = add(2 * (size_t)d.max_bp * d.dp[l]);
-  size_t off_tA = add(2 * (size_t)d.max_bp * maxw), off_tB = add(2 * (size_t)d.max_bp * maxw);
+  for (int l = 0; l < d.L; l++) {
+    off_H[l] = add(2 * (size_t)d.max_bp * d.dp[l]);
+    off_Ht[l] = add(2 * (size_t)d.max_bp * d.dp[l]);
+  }
   size_t off_Y = add(4 * (size_t)d.max_bp * d.dp[d.L]);
-  size_t off_part = add(8 * (size_t)kMlpLossParts), off_err = add(4);
+  size_t off_part = add(8 * ((size_t)d.max_bp / kMlpLossRows) * (d.dp[d.L] / kMlpLossCols));
+  size_t off_done = add(4);
   cudaError_t e = cudaMalloc(&m->arena, total);
+  if (e == cudaSuccess)
+    e = cudaHostAlloc((void **)&m->flags, 4, cudaHostAllocMapped | cudaHostAllocPortable);
+  if (e == cudaSuccess) e = cudaHostGetDevicePointer((void **)&d.err, m->flags, 0);
   if (e != cudaSuccess) {
     set_err(errbuf, errlen, "MLP arena (%zu bytes): %s", total, cudaGetErrorString(e));
     delete m;
@@ -1249,15 +1257,17 @@ ams_status ams_mlp_create(const int *dims, int n_dims, int max_batch, unsigned l
     d.vb[l] = (float *)(a + off_vb[l]); d.gb[l] = (float *)(a + off_gb[l]);
     d.Wb[l] = (__nv_bfloat16 *)(a + off_Wb[l]); d.Wt[l] = (__nv_bfloat16 *)(a + off_Wt[l]);
     d.dZ[l] = (__nv_bfloat16 *)(a + off_dZ[l]);
+    d.dZt[l] = (__nv_bfloat16 *)(a + off_dZt[l]);
   }
-  for (int l = 0; l < d.L; l++) d.H[l] = (__nv_bfloat16 *)(a + off_H[l]);
-  d.tA = (__nv_bfloat16 *)(a + off_tA);
-  d.tB = (__nv_bfloat16 *)(a + off_tB);
+  for (int l = 0; l < d.L; l++) {
+    d.H[l] = (__nv_bfloat16 *)(a + off_H[l]);
+    d.Ht[l] = (__nv_bfloat16 *)(a + off_Ht[l]);
+  }
   d.Y = (float *)(a + off_Y);
   d.part = (double *)(a + off_part);
-  d.err = (unsigned *)(a + off_err);
+  d.done = (unsigned *)(a + off_done);
+  *m->flags = 0;
   cudaStream_t st = (cudaStream_t)stream;
-  cudaMemsetAsync(d.err, 0, 4, st);
   if ((e = mlp_init(d, (uint32_t)(seed ^ (seed >> 32)), st)) != cudaSuccess ||
       (e = cudaStreamSynchronize(st)) != cudaSuccess) {
     set_err(errbuf, errlen, "MLP init: %s", cudaGetErrorString(e));
@@ -1295,28 +1305,6 @@ ams_status ams_mlp_train_step(ams_mlp *m, const float *X, const float *T, int B,
   return mlp_check_err(m, st, errbuf, errlen);
 }
 
-// which: 0 parameters, 1 gradients, 2 Adam first moments, 3 second moments
-static void mlp_param_copy(MlpDev &d, float *flat, bool to_flat, int which, cudaStream_t st) {
-  size_t o = 0;
-  for (int l = 1; l <= d.L; l++) {
-    float *const Ws[4] = {d.W[l], d.gW[l], d.mW[l], d.vW[l]};
-    float *const bs[4] = {d.b[l], d.gb[l], d.mb[l], d.vb[l]};
-    float *W = Ws[which];
-    float *b = bs[which];
-    const size_t dp = sizeof(float) * d.dp[l - 1], dl = sizeof(float) * d.d[l - 1];
-    if (to_flat)
-      cudaMemcpy2DAsync(flat + o, dl, W, dp, dl, d.d[l], cudaMemcpyDeviceToDevice, st);
-    else
-      cudaMemcpy2DAsync(W, dp, flat + o, dl, dl, d.d[l], cudaMemcpyDeviceToDevice, st);
-    o += (size_t)d.d[l] * d.d[l - 1];
-    if (to_flat)
-      cudaMemcpyAsync(flat + o, b, sizeof(float) * d.d[l], cudaMemcpyDeviceToDevice, st);
-    else
-      cudaMemcpyAsync(b, flat + o, sizeof(float) * d.d[l], cudaMemcpyDeviceToDevice, st);
-    o += d.d[l];
-  }
-}
-
 ams_status ams_mlp_gradients(ams_mlp *m, const float *X, const float *T, int B, float *loss,
                              float *grads, void *stream, char *errbuf, size_t errlen) {
   clear_stale_error();
@@ -1327,8 +1315,7 @@ ams_status ams_mlp_gradients(ams_mlp *m, const float *X, const float *T, int B, 
   cudaStream_t st = (cudaStream_t)stream;
   CK(mlp_forward(m->dev, X, B, nullptr, st));
   CK(mlp_backward(m->dev, T, B, loss, st));
-  mlp_param_copy(m->dev, grads, true, 1, st);
-  CK(cudaGetLastError());
+  CK(mlp_flat_copy(m->dev, grads, true, 1, st));
   return mlp_check_err(m, st, errbuf, errlen);
 }
 
@@ -1343,7 +1330,7 @@ ams_status ams_mlp_params(ams_mlp *m, float *params, int direction, long long *c
   if (count) *count = n;
   if (!params) return AMS_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  mlp_param_copy(m->dev, params, direction == 0, 0, st);
+  CK(mlp_flat_copy(m->dev, params, direction == 0, 0, st));
   if (direction == 1) CK(mlp_refresh_bf16(m->dev, st));
   CK(cudaStreamSynchronize(st));
   return AMS_OK;
@@ -1361,9 +1348,8 @@ ams_status ams_mlp_adam_state(ams_mlp *m, float *m1, float *m2, long long *step,
     return AMS_ERR_ARG;
   }
   cudaStream_t st = (cudaStream_t)stream;
-  mlp_param_copy(m->dev, m1, direction == 0, 2, st);
-  mlp_param_copy(m->dev, m2, direction == 0, 3, st);
-  CK(cudaGetLastError());
+  CK(mlp_flat_copy(m->dev, m1, direction == 0, 2, st));
+  CK(mlp_flat_copy(m->dev, m2, direction == 0, 3, st));
   if (direction == 0) *step = m->dev.step;
   else m->dev.step = (int)*step;
   CK(cudaStreamSynchronize(st));

@@ -76,7 +76,7 @@ class MLP:
             Y = torch.empty(Xi.shape[0], self.dims[-1], device="cuda")
             call("ams_mlp_forward", self._h, _ptr(Xi), Xi.shape[0], _ptr(Y), _stream())
             outs.append(Y)
-        return torch.cat(outs, 0)
+        return outs[0] if len(outs) == 1 else torch.cat(outs, 0)
 
     __call__ = forward
 
