@@ -1092,15 +1092,19 @@ cudaError_t run_cb(const ObjArgs &a, const Split &sp, int M, float *U, float *Yp
 // ------------------------------------------------------------------
 // Single-pass streaming path (one HBM read of H_r and H_d).
 //
-// A persistent CTA per SM walks column tiles of TR Rx.  For each tile the
-// TMA engine copies the (M + S) x TR complex block of [H_r; H_d] into a
-// 2-stage shared-memory ring (cp.async.bulk.tensor, mbarrier completion);
-// the CTA then (A) forms Y for the TR columns, (B) evaluates the per-Rx
-// capacity, max and mask and the two gradient parts, and (C) accumulates
-// P1[c,k] += sum_col G1[c,col] conj(H[k,col]) (and P2 for the norm term)
-// from the same shared-memory tile.  The per-CTA P1/P2 and loss partials are
-// reduced by k_stream_gu; k_tc_dphi and k_tc_dw_part / k_tc_dw_sum then form
-// dphi and dL/dW.
+// A cluster of CTAs walks column tiles of TR = 16 (or 8) Rx: the K = M + S rows
+// of [H_r; H_d] are split among the cluster's CTAs, so that a row's piece of a
+// tile is a whole 128-byte line (64 bytes) and a CTA's part of a tile still
+// fits its shared memory several times.  TMA copies (cp.async.bulk.tensor,
+// swizzled, mbarrier completion) fill a ring of stages.  For each tile a CTA
+// (A) forms its rows' part of Y, which the cluster's CTAs send each other through
+// distributed shared memory, then (B) evaluates the per-Rx capacity, max and
+// mask and the two gradient parts, and (C) accumulates P1[c,k] += sum_col
+// G1[c,col] conj(H[k,col]) (and P2 for the norm term) from the same
+// shared-memory tile.  Two warps do B while the others run A of later tiles: B
+// is a chain of 800 cycles for 16 columns, and done by every warp it took half
+// of the kernel's instructions.  The clusters' P1 / P2 and loss partials are
+// reduced by k_stream_tail.
 
 __device__ __forceinline__ uint32_t smem_addr(const void *p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
@@ -1110,6 +1114,372 @@ __device__ __forceinline__ uint32_t smem_addr(const void *p) {
 // from the other CTA on the SM; false after 2 s
 __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t parity) {
   return tc::mbar_wait(bar, parity);
+}
+// the same for a whole warp, one answer for all lanes
+__device__ __forceinline__ bool warp_wait(uint64_t *bar, uint32_t parity) {
+  return __all_sync(0xffffffffu, tc::mbar_wait(bar, parity));
+}
+__device__ __forceinline__ void cluster_arrive() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() {
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// store into CTA `rank` of the cluster; its mbarrier counts the 8 bytes (no fence
+// and no barrier on either side: a cluster barrier with its release cost about
+// 4 us a tile here)
+__device__ __forceinline__ void cluster_store(uint32_t addr, uint32_t bar, int rank, c2 v) {
+  uint32_t a, b;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(b) : "r"(bar), "r"(rank));
+  asm volatile(
+      "st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [%0], {%1, %2}, [%3];" ::"r"(a),
+      "f"(v.x), "f"(v.y), "r"(b)
+      : "memory");
+}
+
+// per-Rx capacity of one column: the gradient parts ga (max term) and gb (norm
+// term, before 1 / ||masked||) of every code, the max over codes, the squares
+// of the masked capacities and the amplitudes
+template <int CB>
+__device__ __forceinline__ void stream_column(const ObjArgs &a, const c2 (&y)[CB], c2 (&ga)[CB],
+                                              c2 (&gb)[CB], float &mx, float &sq,
+                                              float (&amp)[CB]) {
+  float cap[CB];
+  int arg = 0;
+  mx = -1.f;
+  sq = 0.f;
+#pragma unroll
+  for (int c = 0; c < CB; c++) {
+    if (c >= a.C) { cap[c] = 0.f; amp[c] = 0.f; continue; }
+    amp[c] = sqrtf(y[c].x * y[c].x + y[c].y * y[c].y);
+    const float aa = amp[c] + kEps;
+    float v = log2f(1.0f + aa * aa / kN0);
+    if (a.drop && a.drop[c]) v = 0.f;
+    cap[c] = v;
+    if (v > mx) { mx = v; arg = c; }
+  }
+#pragma unroll
+  for (int c = 0; c < CB; c++) {
+    ga[c] = {0.f, 0.f};
+    gb[c] = {0.f, 0.f};
+    if (c >= a.C) continue;
+    const bool dropped = a.drop && a.drop[c];
+    const float msk = (cap[c] != mx) ? cap[c] : 0.f;
+    sq += msk * msk;
+    const float aa = amp[c] + kEps;
+    const float dcap = (2.0f * aa / kN0) / (1.0f + aa * aa / kN0) * kInvLn2;
+    float g1 = (c == arg) ? -a.w : 0.f, g2 = msk;
+    if (dropped) { g1 = 0.f; g2 = 0.f; }
+    const float sc = amp[c] > 0.f ? dcap / amp[c] : 0.f;
+    ga[c] = {g1 * sc * y[c].x, g1 * sc * y[c].y};
+    gb[c] = {g2 * sc * y[c].x, g2 * sc * y[c].y};
+  }
+}
+
+// The split of a problem over clusters (stream_plan).
+struct StreamShape {
+  int M, K, S, Kc;   // rows of a CTA: virtual rows rank * Kc on
+  int boxR;          // rows of an H_r box (divides Kc)
+  int rows;          // rows of a stage: Kc and the room for padded H_d rows
+  int CL, stages, ntiles;
+};
+constexpr int kHdBox = 8;   // rows of an H_d box
+// Tiles between A and C of a compute warp, and epilogue warps (tile i goes to
+// warp i mod kLag): the exchange and B of a tile take about two tiles' time.
+constexpr int kLag = 2;
+constexpr int kNC = 16;  // compute warps
+constexpr int kMaxClusters = 512;  // partials the scratch holds
+// Buffers of what passes between the roles.  A compute warp that works on tile i
+// has read G of tile i - kLag - 1, so every CTA of the cluster had reached that
+// tile's A: what is older than 2 kLag + 2 tiles has been read everywhere, what
+// is older than kLag + 1 in this CTA.
+constexpr int kSlots = 8, kBufs = 4;
+static_assert(kSlots >= 2 * kLag + 3 && kBufs >= kLag + 2, "buffers");
+
+// Warps 0 .. NC - 1 compute (A and C), warps NC .. NC + kLag - 1 form G (the
+// exchange and B), the last warp copies.  The roles meet on mbarriers only, all
+// waits bounded; a wait that ran out ends its role, the others' waits run out
+// in turn, and the CTAs of the cluster leave together.
+// 16-byte chunk ch of row s in a stage, as the copy's swizzle places it
+template <int TR>
+__device__ __forceinline__ uint32_t tile_chunk(int s, int ch) {
+  return TR == 16 ? (uint32_t)s * 128u + (uint32_t)((ch ^ (s & 7)) << 4)
+                  : (uint32_t)s * 64u + (uint32_t)((ch ^ ((s >> 1) & 3)) << 4);
+}
+
+template <int CB, int TR, int RPT>
+__global__ void __launch_bounds__(32 * (kNC + kLag + 1), 1)
+    k_obj_stream(const __grid_constant__ ObjArgs a, const __grid_constant__ CUtensorMap mapR,
+                 const __grid_constant__ CUtensorMap mapD, const StreamShape sh, const float *U,
+                 float *Ppart, double *lpart, unsigned *err) {
+  constexpr int NC = kNC, NT = 32 * NC, CH = TR / 2;  // chunks of a row
+  extern __shared__ unsigned char smem_dyn[];
+  unsigned char *base = reinterpret_cast<unsigned char *>(
+      (reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~(uintptr_t)1023);
+  const uint32_t stage_bytes = (uint32_t)sh.rows * (TR * 8u);
+  c2 *coef = reinterpret_cast<c2 *>(base + (size_t)sh.stages * stage_bytes);  // [rows][CB]
+  c2 *ybuf = coef + (size_t)sh.rows * CB;              // [kSlots][CL][CB][TR]
+  __shared__ __align__(16) c2 red[kBufs][NC][CB][TR];
+  __shared__ __align__(16) c2 gbuf[kBufs][2 * CB][TR];
+  __shared__ __align__(8) uint64_t full[8], empty[8], redf[kBufs], gf[kBufs], got[kSlots];
+  __shared__ c2 sums[kLag];
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int rank = (int)blockIdx.x % sh.CL, cluster = (int)blockIdx.x / sh.CL,
+            nclusters = (int)gridDim.x / sh.CL;
+  // this CTA's virtual rows [k0, k1): nr rows of H_r at stage rows 0 on, nd
+  // rows of H_d from d0 on at stage rows hd on
+  const int k0 = rank * sh.Kc, k1 = min(sh.K, k0 + sh.Kc);
+  const int nr = max(0, min(k1, sh.M) - k0), nd = max(0, k1 - max(k0, sh.M)),
+            d0 = max(k0 - sh.M, 0);
+  const int hd = (nr + sh.boxR - 1) / sh.boxR * sh.boxR;
+  const int used = nd > 0 ? hd + nd : nr;  // stage rows that hold anything
+  const int n = cluster < sh.ntiles ? (sh.ntiles - cluster + nclusters - 1) / nclusters : 0;
+  if (t == 0) {
+    for (int i = 0; i < sh.stages; i++) { tc::mbar_init(&full[i], 1); tc::mbar_init(&empty[i], NC); }
+    for (int i = 0; i < kBufs; i++) { tc::mbar_init(&redf[i], NC); tc::mbar_init(&gf[i], 1); }
+    for (int i = 0; i < kSlots; i++) tc::mbar_init(&got[i], 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  // every CTA of the cluster runs, its barriers set, before anyone stores into
+  // its memory
+  __syncthreads();
+  cluster_arrive();
+  cluster_wait();
+
+  if (warp == NC + kLag) {
+    // ---- copies
+    if (lane == 0) {
+      const int n_box = hd / sh.boxR, d_box = (nd + kHdBox - 1) / kHdBox;
+      const uint32_t tx = (uint32_t)(hd + d_box * kHdBox) * (TR * 8u);
+      int it = 0;
+      bool ok = true;
+      for (; it < n; it++) {
+        const int stg = it % sh.stages;
+        if (it >= sh.stages &&
+            !mbar_wait_bounded(&empty[stg], (uint32_t)(it / sh.stages - 1) & 1u)) {
+          ok = false;
+          break;
+        }
+        unsigned char *dst = base + (size_t)stg * stage_bytes;
+        const int x = (cluster + it * nclusters) * TR * 2;
+        tc::mbar_expect_tx(&full[stg], tx);
+        for (int i = 0; i < n_box; i++)
+          tc::tma_load_2d(dst + (size_t)i * sh.boxR * (TR * 8), &mapR, x, k0 + i * sh.boxR, &full[stg]);
+        for (int i = 0; i < d_box; i++)
+          tc::tma_load_2d(dst + (size_t)(hd + i * kHdBox) * (TR * 8), &mapD, x, d0 + i * kHdBox,
+                          &full[stg]);
+      }
+      if (!ok) atomicOr(err, 1u);
+      // the copies issued land before the CTA exits (in a good run the compute
+      // warps have seen them land; the last ones are looked at again)
+      for (int i = max(0, it - sh.stages); i < it; i++)
+        mbar_wait_bounded(&full[i % sh.stages], (uint32_t)(i / sh.stages) & 1u);
+    }
+  } else if (warp >= NC) {
+    // ---- G of tiles warp - NC, warp - NC + kLag, ...
+    float sum_max = 0.f, sum_sq = 0.f;  // FP32 within a warp, FP64 across warps
+    const int col = lane & (TR - 1), cs = lane / TR;
+    for (int it = warp - NC; it < n; it += kLag) {
+      const int bi = it % kBufs, si = it % kSlots;
+      if (!warp_wait(&redf[bi], (uint32_t)(it / kBufs) & 1u)) { atomicOr(err, 1u); break; }
+      if (lane == 0)
+        tc::mbar_expect_tx(&got[si], (uint32_t)(sh.CL * CB * TR * sizeof(c2)));
+      __syncwarp();
+      if (cs < CB) {  // the CTA's part of Y, to every CTA of the cluster
+        c2 v = {0.f, 0.f};
+#pragma unroll
+        for (int w = 0; w < NC; w++) { v.x += red[bi][w][cs][col].x; v.y += red[bi][w][cs][col].y; }
+        const uint32_t at =
+            smem_addr(ybuf + ((size_t)(si * sh.CL + rank) * CB + cs) * TR + col);
+        const uint32_t bar = smem_addr(&got[si]);
+        for (int r = 0; r < sh.CL; r++) cluster_store(at, bar, r, v);
+      }
+      if (!warp_wait(&got[si], (uint32_t)(it / kSlots) & 1u)) { atomicOr(err, 1u); break; }
+      const c2 *yb = ybuf + (size_t)si * sh.CL * CB * TR;
+      c2 y[CB], ga[CB], gb[CB];
+#pragma unroll
+      for (int c = 0; c < CB; c++) {
+        y[c] = {0.f, 0.f};
+        for (int r = 0; r < sh.CL; r++) {
+          const c2 v = yb[(r * CB + c) * TR + col];
+          y[c].x += v.x;
+          y[c].y += v.y;
+        }
+      }
+      float mx, sq, amp[CB];
+      stream_column<CB>(a, y, ga, gb, mx, sq, amp);
+      const int r = (cluster + it * nclusters) * TR + col;
+      const bool live = r < a.R;
+      if (lane < TR) {
+#pragma unroll
+        for (int c = 0; c < CB; c++) {
+          gbuf[bi][c][col] = live ? ga[c] : c2{0.f, 0.f};
+          if (CB > 1) gbuf[bi][CB + c][col] = live ? gb[c] : c2{0.f, 0.f};
+        }
+        if (rank == 0 && live) {
+          sum_max += mx;
+          sum_sq += sq;
+          if (a.recv_amp)
+#pragma unroll
+            for (int c = 0; c < CB; c++)
+              if (c < a.C) a.recv_amp[(size_t)c * a.R + r] = amp[c];
+        }
+      }
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(&gf[bi]);
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      sum_max += __shfl_xor_sync(0xffffffffu, sum_max, o);
+      sum_sq += __shfl_xor_sync(0xffffffffu, sum_sq, o);
+    }
+    // (the cluster barrier below orders the warps' sums)
+    if (lane == 0) sums[warp - NC] = {sum_max, sum_sq};
+  }
+  c2 p1[RPT][CB], p2[RPT][CB];
+#pragma unroll
+  for (int q = 0; q < RPT; q++)
+#pragma unroll
+    for (int c = 0; c < CB; c++) { p1[q][c] = {0.f, 0.f}; p2[q][c] = {0.f, 0.f}; }
+  if (warp < NC) {
+    // ---- compute.  The first tiles are on their way; wait for the U kernel,
+    // then stage the coefficients of the stage's rows (0 for padding): U for
+    // metasurface rows, W for the H_d rows
+    cudaGridDependencySynchronize();
+    for (int i = t; i < sh.rows * CB; i += NT) {
+      const int s = i / CB, c = i % CB;
+      c2 v = {0.f, 0.f};
+      if (c < a.C) {
+        if (s < nr) v = ld2(U, (size_t)c * sh.M + k0 + s);
+        else if (s >= hd && s - hd < nd) v = ld2(a.W, (size_t)c * sh.S + d0 + s - hd);
+      }
+      coef[i] = v;
+    }
+    asm volatile("bar.sync 1, %0;" ::"r"(NT) : "memory");  // the compute warps
+    for (int it = 0; it < n + kLag; it++) {
+      // (A) this CTA's part of Y for the columns: CH lanes take a row's 16-byte
+      // chunks (two columns each), a warp 32 / CH rows at a time
+      if (it < n) {
+        const int stg = it % sh.stages;
+        if (!warp_wait(&full[stg], (uint32_t)(it / sh.stages) & 1u)) {
+          atomicOr(err, 1u);
+          break;
+        }
+        const unsigned char *T = base + (size_t)stg * stage_bytes;
+        c2 y0[CB], y1[CB];
+#pragma unroll
+        for (int c = 0; c < CB; c++) { y0[c] = {0.f, 0.f}; y1[c] = {0.f, 0.f}; }
+        const int sub = lane / CH, ch = lane % CH;
+#pragma unroll 4
+        for (int s = 32 / CH * warp + sub; s < used; s += 32 / CH * NC) {
+          const float4 h = *reinterpret_cast<const float4 *>(T + tile_chunk<TR>(s, ch));
+#pragma unroll
+          for (int c = 0; c < CB; c++) {
+            const c2 u = coef[s * CB + c];
+            mac(y0[c], u, c2{h.x, h.y});
+            mac(y1[c], u, c2{h.z, h.w});
+          }
+        }
+        __syncwarp();
+#pragma unroll
+        for (int c = 0; c < CB; c++) {
+#pragma unroll
+          for (int o = CH; o < 32; o <<= 1) {
+            y0[c].x += __shfl_xor_sync(0xffffffffu, y0[c].x, o);
+            y0[c].y += __shfl_xor_sync(0xffffffffu, y0[c].y, o);
+            y1[c].x += __shfl_xor_sync(0xffffffffu, y1[c].x, o);
+            y1[c].y += __shfl_xor_sync(0xffffffffu, y1[c].y, o);
+          }
+          if (lane < CH)
+            *reinterpret_cast<float4 *>(&red[it % kBufs][warp][c][2 * ch]) =
+                make_float4(y0[c].x, y0[c].y, y1[c].x, y1[c].y);
+        }
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(&redf[it % kBufs]);
+      }
+      if (it < kLag) continue;
+      // (C) P += G conj(H) over the columns of the tile kLag before, a thread
+      // per row
+      const int ct = it - kLag, bi = ct % kBufs;
+      if (!warp_wait(&gf[bi], (uint32_t)(ct / kBufs) & 1u)) {
+        atomicOr(err, 1u);
+        break;
+      }
+      const unsigned char *T = base + (size_t)(ct % sh.stages) * stage_bytes;
+#pragma unroll
+      for (int hcol = 0; hcol < TR; hcol += 8) {
+        c2 g1[CB][8], g2[CB][8];
+#pragma unroll
+        for (int c = 0; c < CB; c++)
+#pragma unroll
+          for (int j = 0; j < 8; j += 2) {
+            const float4 u = *reinterpret_cast<const float4 *>(&gbuf[bi][c][hcol + j]);
+            g1[c][j] = {u.x, u.y};
+            g1[c][j + 1] = {u.z, u.w};
+            if (CB > 1) {
+              const float4 v = *reinterpret_cast<const float4 *>(&gbuf[bi][CB + c][hcol + j]);
+              g2[c][j] = {v.x, v.y};
+              g2[c][j + 1] = {v.z, v.w};
+            }
+          }
+#pragma unroll
+        for (int q = 0; q < RPT; q++) {
+          const int s = t + NT * q;
+          if (s < used) {
+#pragma unroll
+            for (int j = 0; j < 8; j += 2) {
+              const float4 h =
+                  *reinterpret_cast<const float4 *>(T + tile_chunk<TR>(s, (hcol + j) >> 1));
+#pragma unroll
+              for (int c = 0; c < CB; c++) {
+                macc(p1[q][c], g1[c][j], c2{h.x, h.y});
+                macc(p1[q][c], g1[c][j + 1], c2{h.z, h.w});
+                if (CB > 1) {
+                  macc(p2[q][c], g2[c][j], c2{h.x, h.y});
+                  macc(p2[q][c], g2[c][j + 1], c2{h.z, h.w});
+                }
+              }
+            }
+          }
+        }
+      }
+      // the stage is free: this warp's generic reads before the async-proxy
+      // refill
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(&empty[ct % sh.stages]);
+    }
+  }
+  // no CTA leaves while another one may still store into its memory
+  __syncwarp();
+  cluster_arrive();
+  cluster_wait();
+  // the tail kernel may launch now; its grid-dependency wait still waits for
+  // this grid to complete, with every write below visible
+  cudaTriggerProgrammaticLaunchCompletion();
+  if (warp >= NC) {
+    if (rank == 0 && t == NT) {
+      double x = 0.0, z = 0.0;
+      for (int e = 0; e < kLag; e++) { x += sums[e].x; z += sums[e].y; }
+      lpart[2 * cluster] = x;
+      lpart[2 * cluster + 1] = z;
+    }
+    return;
+  }
+  // partials of this cluster: P1 at [b][c][k], P2 at [b][C + c][k]
+#pragma unroll
+  for (int q = 0; q < RPT; q++) {
+    const int s = t + NT * q;
+    if (s >= used || (s >= nr && s < hd)) continue;
+    const int k = s < nr ? k0 + s : sh.M + d0 + s - hd;
+#pragma unroll
+    for (int c = 0; c < CB; c++) {
+      if (c >= a.C) continue;
+      float2 *o = reinterpret_cast<float2 *>(Ppart) + ((size_t)cluster * 2 * a.C + c) * sh.K + k;
+      o[0] = make_float2(p1[q][c].x, p1[q][c].y);
+      if (CB > 1) o[(size_t)a.C * sh.K] = make_float2(p2[q][c].x, p2[q][c].y);
+    }
+  }
 }
 
 // the coefficients of the virtual rows into shared memory, coef[k][c]: U for
@@ -1135,211 +1505,6 @@ __device__ __forceinline__ void stage_coef(const ObjArgs &a, int M, int K, const
   }
 }
 
-template <int CB, int TR, int KPT>
-__global__ void __launch_bounds__(256, 2)
-    k_obj_stream(ObjArgs a, const __grid_constant__ CUtensorMap mapR,
-                 const __grid_constant__ CUtensorMap mapD, int M, int Mbox, int Mp, int boxR,
-                 int stage_bytes, int ntiles, const float *U, float *Ppart, double *lpart,
-                 unsigned *err) {
-  constexpr int NTH = 256, NW = NTH / 32;
-  const int K = M + a.S;
-  // H_r rows [0, Mbox) come from boxes of boxR rows, H_d rows start at Mp
-  // (a multiple of 16, so every TMA destination is 128-byte aligned)
-  const uint32_t tx_bytes = (uint32_t)(Mbox + a.S) * TR * 8;
-  extern __shared__ unsigned char smem_dyn[];
-  unsigned char *base = reinterpret_cast<unsigned char *>(
-      (reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~(uintptr_t)1023);
-  c2 *coef = reinterpret_cast<c2 *>(base + 2 * (size_t)stage_bytes);   // [K][CB]
-  __shared__ c2 red[NW][TR][CB];
-  __shared__ c2 g1s[CB][TR], g2s[CB][TR];
-  __shared__ __align__(8) uint64_t full[2];
-  __shared__ int abort_flag;
-  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-
-  auto issue = [&](int tile, int stage) {
-    float2 *dst = reinterpret_cast<float2 *>(base + (size_t)stage * stage_bytes);
-    uint64_t *bar = &full[stage];
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)),
-                 "r"(tx_bytes)
-                 : "memory");
-    const int x = tile * TR * 2;
-    for (int m0 = 0; m0 < Mbox; m0 += boxR)
-      asm volatile(
-          "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes"
-          " [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_addr(dst + (size_t)m0 * TR)),
-          "l"(reinterpret_cast<uint64_t>(&mapR)), "r"(x), "r"(m0), "r"(smem_addr(bar))
-          : "memory");
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes"
-        " [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_addr(dst + (size_t)Mp * TR)),
-        "l"(reinterpret_cast<uint64_t>(&mapD)), "r"(x), "r"(0), "r"(smem_addr(bar))
-        : "memory");
-  };
-  const int first = blockIdx.x;
-  if (t == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&full[0])), "r"(1));
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(&full[1])), "r"(1));
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    abort_flag = 0;
-    if (first < ntiles) issue(first, 0);
-    if (first + (int)gridDim.x < ntiles) issue(first + gridDim.x, 1);
-  }
-  // the first tiles are in flight; wait for the U kernel, then stage the
-  // coefficients: U for metasurface rows, W for the H_d rows
-  cudaGridDependencySynchronize();
-  stage_coef<NTH, CB>(a, M, K, U, coef);
-  __syncthreads();
-
-  c2 p1[KPT][CB], p2[KPT][CB];
-#pragma unroll
-  for (int q = 0; q < KPT; q++)
-#pragma unroll
-    for (int c = 0; c < CB; c++) { p1[q][c] = {0.f, 0.f}; p2[q][c] = {0.f, 0.f}; }
-  float sum_max = 0.f, sum_sq = 0.f;  // FP32 within a warp, FP64 across warps
-  const int col = t % TR, j = t / TR;
-  constexpr int NJ = NTH / TR;
-
-  int it = 0;
-  for (int tile = first; tile < ntiles; tile += gridDim.x, it++) {
-    const int stg = it & 1;
-    if (!mbar_wait_bounded(&full[stg], (it >> 1) & 1)) {
-      if (t == 0) atomicOr(err, 1u);
-      abort_flag = 1;
-    }
-    __syncthreads();
-    if (abort_flag) {
-      // before the CTA exits, let the copies it issued land (bounded again):
-      // this tile's and, if it was issued, the next tile's in the other stage
-      if (t == 0) {
-        mbar_wait_bounded(&full[stg], (it >> 1) & 1);
-        if (tile + (int)gridDim.x < ntiles) mbar_wait_bounded(&full[stg ^ 1], ((it + 1) >> 1) & 1);
-      }
-      break;
-    }
-    const float2 *T = reinterpret_cast<const float2 *>(base + (size_t)stg * stage_bytes);
-    // (A) Y for the tile's columns; lanes with equal col are TR apart
-    c2 y[CB];
-#pragma unroll
-    for (int c = 0; c < CB; c++) y[c] = {0.f, 0.f};
-#pragma unroll 4
-    for (int k = j; k < K; k += NJ) {
-      const int row = k < M ? k : Mp + (k - M);
-      const float2 h = T[(size_t)row * TR + col];
-#pragma unroll
-      for (int c = 0; c < CB; c++) mac(y[c], coef[(size_t)k * CB + c], c2{h.x, h.y});
-    }
-#pragma unroll
-    for (int c = 0; c < CB; c++)
-      for (int o = TR; o < 32; o <<= 1) {
-        y[c].x += __shfl_xor_sync(0xffffffffu, y[c].x, o);
-        y[c].y += __shfl_xor_sync(0xffffffffu, y[c].y, o);
-      }
-    if (lane < TR)
-#pragma unroll
-      for (int c = 0; c < CB; c++) red[warp][lane][c] = y[c];
-    __syncthreads();
-    // (B) per-Rx capacity, max, mask, gradient parts
-    if (t < TR) {
-      const int r = tile * TR + t;
-      c2 yy[CB];
-      float cap[CB], amp[CB];
-#pragma unroll
-      for (int c = 0; c < CB; c++) {
-        c2 acc = {0.f, 0.f};
-#pragma unroll
-        for (int w = 0; w < NW; w++) { acc.x += red[w][t][c].x; acc.y += red[w][t][c].y; }
-        yy[c] = acc;
-      }
-      int arg = 0;
-      float mx = -1.f;
-#pragma unroll
-      for (int c = 0; c < CB; c++) {
-        if (c >= a.C) { cap[c] = 0.f; amp[c] = 0.f; continue; }
-        amp[c] = sqrtf(yy[c].x * yy[c].x + yy[c].y * yy[c].y);
-        const float aa = amp[c] + kEps;
-        float v = log2f(1.0f + aa * aa / kN0);
-        if (a.drop && a.drop[c]) v = 0.f;
-        cap[c] = v;
-        if (v > mx) { mx = v; arg = c; }
-        if (a.recv_amp && r < a.R) a.recv_amp[(size_t)c * a.R + r] = amp[c];
-      }
-#pragma unroll
-      for (int c = 0; c < CB; c++) {
-        c2 ga = {0.f, 0.f}, gb = {0.f, 0.f};
-        if (c < a.C && r < a.R) {
-          const bool dropped = a.drop && a.drop[c];
-          const float msk = (cap[c] != mx) ? cap[c] : 0.f;
-          sum_sq += msk * msk;
-          const float aa = amp[c] + kEps;
-          const float dcap = (2.0f * aa / kN0) / (1.0f + aa * aa / kN0) * kInvLn2;
-          float g1 = (c == arg) ? -a.w : 0.f, g2 = msk;
-          if (dropped) { g1 = 0.f; g2 = 0.f; }
-          const float sc = amp[c] > 0.f ? dcap / amp[c] : 0.f;
-          ga = {g1 * sc * yy[c].x, g1 * sc * yy[c].y};
-          gb = {g2 * sc * yy[c].x, g2 * sc * yy[c].y};
-        }
-        g1s[c][t] = ga;
-        g2s[c][t] = gb;
-      }
-      if (r < a.R) sum_max += mx;
-    }
-    __syncthreads();
-    // (C) P += G conj(H) over the tile's columns, rows k = t + NTH q; the
-    // column order is rotated by the lane so a warp's reads spread over banks
-#pragma unroll
-    for (int q = 0; q < KPT; q++) {
-      const int k = t + NTH * q;
-      if (k < K) {
-        const int row = k < M ? k : Mp + (k - M);
-        const float2 *hr = T + (size_t)row * TR;
-#pragma unroll
-        for (int cc0 = 0; cc0 < TR; cc0++) {
-          const int cc = (cc0 + lane) & (TR - 1);
-          const float2 h = hr[cc];
-#pragma unroll
-          for (int c = 0; c < CB; c++) {
-            macc(p1[q][c], g1s[c][cc], c2{h.x, h.y});
-            if (CB > 1) macc(p2[q][c], g2s[c][cc], c2{h.x, h.y});
-          }
-        }
-      }
-    }
-    __syncthreads();
-    // the stage is free: order the generic reads before the async-proxy refill
-    if (t == 0) {
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      if (tile + 2 * (int)gridDim.x < ntiles) issue(tile + 2 * gridDim.x, stg);
-    }
-  }
-  // the tail kernel may launch now; its grid-dependency wait still waits for
-  // this grid to complete, with every write below visible
-  cudaTriggerProgrammaticLaunchCompletion();
-  // partials of this CTA: P1 at [b][c][k], P2 at [b][C + c][k]
-#pragma unroll
-  for (int q = 0; q < KPT; q++) {
-    const int k = t + NTH * q;
-    if (k >= K) continue;
-#pragma unroll
-    for (int c = 0; c < CB; c++) {
-      if (c >= a.C) continue;
-      float2 *o = reinterpret_cast<float2 *>(Ppart) + ((size_t)blockIdx.x * 2 * a.C + c) * K + k;
-      o[0] = make_float2(p1[q][c].x, p1[q][c].y);
-      if (CB > 1) o[(size_t)a.C * K] = make_float2(p2[q][c].x, p2[q][c].y);
-    }
-  }
-  if (t < 32) {
-    for (int o = 16; o > 0; o >>= 1) {
-      sum_max += __shfl_xor_sync(0xffffffffu, sum_max, o);
-      sum_sq += __shfl_xor_sync(0xffffffffu, sum_sq, o);
-    }
-    if (t == 0) {
-      lpart[2 * blockIdx.x] = sum_max;
-      lpart[2 * blockIdx.x + 1] = sum_sq;
-    }
-  }
-}
-
-
 using EncodeFn = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *,
                               const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
                               const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
@@ -1358,7 +1523,8 @@ EncodeFn tmap_encoder() {
   return fn;
 }
 
-// complex [rows, R] as a float [rows, 2R] tensor; box (2 TR floats) x box_rows
+// complex [rows, R] as a float [rows, 2R] tensor; box of 2 TR floats (one
+// swizzle row of 128 or 64 bytes) x box_rows
 bool make_cmap(CUtensorMap *m, const float *base, int rows, int R, int TR, int box_rows) {
   EncodeFn enc = tmap_encoder();
   if (!enc) return false;
@@ -1367,84 +1533,112 @@ bool make_cmap(CUtensorMap *m, const float *base, int rows, int R, int TR, int b
   cuuint32_t box[2] = {(cuuint32_t)(2 * TR), (cuuint32_t)box_rows};
   cuuint32_t estr[2] = {1, 1};
   return enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float *>(base), dims, strides, box,
-             estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+             estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+             TR == 16 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 struct StreamPlan {
   bool ok = false;
-  int TR = 0, KPT = 0, Mbox = 0, Mp = 0, boxR = 0, stage_bytes = 0, ntiles = 0, grid = 0;
+  StreamShape sh{};
+  int TR = 0, rpt = 0;  // Rx of a tile, rows of a thread
   size_t smem = 0;
 };
 
 int sm_count() { return ams_device_sms(); }
 
-// the single-pass path needs the whole [H_r; H_d] column tile in shared memory
+// Shared memory of a CTA (227 KB an SM can give one), and its static part.
+constexpr size_t kStreamSmem = 226 * 1024;
+constexpr size_t stream_static_smem(int CB, int TR) {
+  return sizeof(c2) * TR * CB * kBufs * (kNC + 2) + 512;
+}
+
+// The smallest cluster whose CTAs hold their part of a tile in enough stages
+// (kLag tiles between A and C, the one in A, two on their way): tiles of 16 Rx
+// while a cluster of four will do (K up to 1,300), then of 8 Rx (up to 2,550,
+// and to 3,200 with one on its way).
+// Clusters of eight are half as many and no faster each: 250 us against 128 us
+// with clusters of four at K = 1,040, R = 65,536.
 StreamPlan stream_plan(int S, int M, int R, int C, bool grad_y) {
   StreamPlan p;
   const int CB = cbucket(C);
-  if (grad_y || CB > 2 || R % 2 || S > 256 || M < 0) return p;
+  if (grad_y || CB > 2 || R % 2 || M < 0) return p;
   const int K = M + S;
-  const int kpt = (K + 255) / 256;
-  int KPT = kpt <= 4 ? 4 : (kpt <= 8 ? 8 : (kpt <= 16 ? 16 : 0));
-  if (!KPT || (CB == 2 && KPT > 8)) return p;
-  p.boxR = M <= 256 ? std::max(M, 1) : 256;
-  p.Mbox = M <= 0 ? 0 : (M + p.boxR - 1) / p.boxR * p.boxR;
-  p.Mp = (p.Mbox + 15) / 16 * 16;
-  for (int TR : {8, 4, 2}) {
-    const size_t stage = ((size_t)(p.Mp + S) * TR * 8 + 1023) / 1024 * 1024;
-    const size_t smem = 1024 + 2 * stage + (size_t)K * CB * 8;
-    if (smem <= 110 * 1024) {  // two CTAs per SM
+  struct { int TR, ahead; } const tiles[] = {{16, 2}, {8, 2}, {8, 1}};
+  for (const auto &tl : tiles)
+    for (int CL : {1, 2, 4}) {
+      const int TR = tl.TR;
+      StreamShape h{};
+      h.M = M; h.K = K; h.S = S; h.CL = CL;
+      // up to 5% more rows where that splits them into fewer boxes (a box has
+      // 256 rows at most, a multiple of 8)
+      int boxes = 1 << 30;
+      const int least = ((K + CL - 1) / CL + 7) / 8 * 8;
+      for (int Kc = least; Kc <= least + least / 20; Kc += 8) {
+        int nb = 1;
+        while (Kc / 8 % nb || Kc / nb > 256) nb++;
+        if (nb < boxes) { boxes = nb; h.Kc = Kc; h.boxR = Kc / nb; }
+      }
+      h.rows = h.Kc + (M > 0 ? (std::min(S, h.Kc) + kHdBox - 1) / kHdBox * kHdBox : 0);
+      const int rpt = (h.rows + 32 * kNC - 1) / (32 * kNC);
+      if (rpt > 2) continue;
+      const size_t dyn = 1024 + sizeof(c2) * CB * ((size_t)h.rows + (size_t)kSlots * CL * TR);
+      const size_t room = kStreamSmem - stream_static_smem(CB, TR);
+      const size_t stage = (size_t)h.rows * TR * 8;
+      if (dyn + (kLag + 1 + tl.ahead) * stage > room) continue;
+      h.stages = (int)std::min<size_t>(8, (room - dyn) / stage);
+      h.ntiles = (R + TR - 1) / TR;
+      p.sh = h;
       p.TR = TR;
-      p.stage_bytes = (int)stage;
-      p.smem = smem;
-      break;
+      p.rpt = rpt;
+      p.smem = dyn + h.stages * stage;
+      p.ok = true;
+      return p;
     }
-  }
-  if (!p.TR) return p;
-  p.KPT = KPT;
-  p.ntiles = (R + p.TR - 1) / p.TR;
-  p.grid = std::min(2 * sm_count(), p.ntiles);
-  p.ok = true;
   return p;
 }
 
-template <int CB, int TR, int KPT>
+template <int CB, int TR, int RPT>
 cudaError_t launch_stream_t(const ObjArgs &a, const StreamPlan &pl, const CUtensorMap &mr,
-                            const CUtensorMap &md, int M, const float *U, float *Ppart,
-                            double *lpart, unsigned *err, cudaStream_t st) {
-  auto kfn = k_obj_stream<CB, TR, KPT>;
+                            const CUtensorMap &md, const float *U, float *Ppart, double *lpart,
+                            unsigned *err, int *clusters, cudaStream_t st) {
+  auto kfn = k_obj_stream<CB, TR, RPT>;
   static size_t set_bytes[AMS_MAX_DEVICES] = {0};
-  {
-    cudaError_t e = ams_set_smem_atleast(set_bytes, kfn, pl.smem);
-    if (e != cudaSuccess) return e;
-  }
+  // the most dynamic shared memory of any plan (the static part beside it)
+  const size_t room = kStreamSmem - stream_static_smem(CB, TR);
+  cudaError_t e = ams_set_smem_atleast(set_bytes, kfn, room);
+  if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(pl.grid);
-  cfg.blockDim = dim3(256);
-  cfg.dynamicSmemBytes = pl.smem;
+  cfg.blockDim = dim3(32 * (kNC + kLag + 1));
   cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)pl.sh.CL;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kfn, a, mr, md, M, pl.Mbox, pl.Mp, pl.boxR, pl.stage_bytes,
-                            pl.ntiles, U, Ppart, lpart, err);
-}
-
-template <int CB, int TR>
-cudaError_t launch_stream_k(const ObjArgs &a, const StreamPlan &pl, const CUtensorMap &mr,
-                            const CUtensorMap &md, int M, const float *U, float *Ppart,
-                            double *lpart, unsigned *err, cudaStream_t st) {
-  switch (pl.KPT) {
-    case 4: return launch_stream_t<CB, TR, 4>(a, pl, mr, md, M, U, Ppart, lpart, err, st);
-    case 8: return launch_stream_t<CB, TR, 8>(a, pl, mr, md, M, U, Ppart, lpart, err, st);
-    case 16:
-      if (CB == 1) return launch_stream_t<1, TR, 16>(a, pl, mr, md, M, U, Ppart, lpart, err, st);
-      return cudaErrorInvalidValue;
-    default: return cudaErrorInvalidValue;
+  // clusters resident at once with the most shared memory this kernel takes,
+  // looked up once per device and cluster size
+  static std::atomic<int> resident[AMS_MAX_DEVICES][3];
+  const int dev = ams_current_device();
+  if (dev < 0) return cudaErrorInvalidDevice;
+  const int ci = pl.sh.CL == 1 ? 0 : pl.sh.CL == 2 ? 1 : 2;
+  int most = resident[dev][ci].load();
+  if (most == 0) {
+    cfg.numAttrs = 1;
+    cfg.gridDim = dim3((unsigned)pl.sh.CL);
+    cfg.dynamicSmemBytes = room;
+    if ((e = cudaOccupancyMaxActiveClusters(&most, kfn, &cfg)) != cudaSuccess) return e;
+    most = std::max(1, std::min(most, kMaxClusters));
+    resident[dev][ci].store(most);
   }
+  *clusters = std::min(most, pl.sh.ntiles);
+  cfg.numAttrs = 2;
+  cfg.gridDim = dim3((unsigned)(*clusters * pl.sh.CL));
+  cfg.dynamicSmemBytes = pl.smem;
+  return cudaLaunchKernelEx(&cfg, kfn, a, mr, md, pl.sh, U, Ppart, lpart, err);
 }
 
 template <int CB>
@@ -1457,9 +1651,9 @@ cudaError_t run_stream(const ObjArgs &a, const StreamPlan &pl, int M, float *U, 
                        double *lpart, float *GU, float *dwp, unsigned *err, unsigned *counter,
                        cudaStream_t st) {
   CUtensorMap mr, md;
-  const float *Hr = M > 0 ? a.Hr : a.Hd;  // no metasurface: mapR is unused (Mbox = 0)
-  if (!make_cmap(&mr, Hr, std::max(M, 1), a.R, pl.TR, pl.boxR) ||
-      !make_cmap(&md, a.Hd, a.S, a.R, pl.TR, a.S))
+  const float *Hr = M > 0 ? a.Hr : a.Hd;  // no metasurface: mapR is unused
+  if (!make_cmap(&mr, Hr, std::max(M, 1), a.R, pl.TR, pl.sh.boxR) ||
+      !make_cmap(&md, a.Hd, a.S, a.R, pl.TR, kHdBox))
     return cudaErrorInvalidValue;
   if (M > 0) {
     const long long n = (long long)M * a.C * 8;
@@ -1467,13 +1661,17 @@ cudaError_t run_stream(const ObjArgs &a, const StreamPlan &pl, int M, float *U, 
   }
   cudaError_t e = obj_begin_call(err, M > 0, st);
   if (e != cudaSuccess) return e;
-  switch (pl.TR) {
-    case 8: e = launch_stream_k<CB, 8>(a, pl, mr, md, M, U, Ppart, lpart, err, st); break;
-    case 4: e = launch_stream_k<CB, 4>(a, pl, mr, md, M, U, Ppart, lpart, err, st); break;
-    default: e = launch_stream_k<CB, 2>(a, pl, mr, md, M, U, Ppart, lpart, err, st); break;
-  }
+  int clusters = 0;
+  if (pl.TR == 16 && pl.rpt == 1)
+    e = launch_stream_t<CB, 16, 1>(a, pl, mr, md, U, Ppart, lpart, err, &clusters, st);
+  else if (pl.TR == 16)
+    e = launch_stream_t<CB, 16, 2>(a, pl, mr, md, U, Ppart, lpart, err, &clusters, st);
+  else if (pl.rpt == 1)
+    e = launch_stream_t<CB, 8, 1>(a, pl, mr, md, U, Ppart, lpart, err, &clusters, st);
+  else
+    e = launch_stream_t<CB, 8, 2>(a, pl, mr, md, U, Ppart, lpart, err, &clusters, st);
   if (e != cudaSuccess) return e;
-  return stream_tail<CB>(a, M, pl.grid, U, Ppart, lpart, GU, dwp, counter, err, st);
+  return stream_tail<CB>(a, M, clusters, U, Ppart, lpart, GU, dwp, counter, err, st);
 }
 
 // after a streaming kernel: G_U, dphi and the dL/dW parts, then dL/dW
@@ -1497,10 +1695,12 @@ cudaError_t stream_tail(const ObjArgs &a, int M, int nparts, const float *U, con
 
 // ------------------------------------------------------------------
 // Streaming path on a plan's transposed copy HT [Rp][Kp] of [H_r; H_d]
-// (row r = column r over all k): a tile of TR Rx is one contiguous block of
-// TR * Kp * 8 bytes, fetched by a single cp.async.bulk instead of one 32-byte
-// piece per row.  Phases as in k_obj_stream; in (A) warp w takes column
-// w % TR and every (NW / TR)-th run of 32 k, lanes over k.
+// (row r = column r over all k), for an odd number of Rx, unaligned channels
+// and K beyond k_obj_stream's: a tile of TR Rx is one contiguous block of
+// TR * Kp * 8 bytes, fetched by a single cp.async.bulk.  A CTA has all rows of
+// its tile, takes the phases A, B, C one after the other and writes its own
+// partials; in (A) warp w takes column w % TR and every (NW / TR)-th run of 32
+// k, lanes over k.
 
 __global__ void __launch_bounds__(256) k_make_ht(const float *Hr, const float *Hd, int M, int S,
                                                  int R, int Rp, int Kp, float *HT) {
@@ -1978,7 +2178,7 @@ ObjScratchLayout obj_scratch_layout(int S, int M, int R, int C) {
   L.G2 = o; o += al(8 * (size_t)C * R);
   L.part = o; o += al(16 * (size_t)std::max(sp.nb_epi, (R + 31) / 32));  // either epilogue
   L.GU = o; o += al(8 * (size_t)sp.rspl * C * sp.K);      // G_U partials
-  const int nsm = 512;                                    // CTA partials of the streaming path
+  const int nsm = kMaxClusters;                           // partials of the streaming path
   L.Pp = o; o += al(8 * (size_t)nsm * 2 * C * sp.K);
   L.lp = o; o += al(16 * (size_t)nsm);
   L.GUs = o; o += al(8 * (size_t)C * sp.K);
@@ -2003,7 +2203,7 @@ cudaError_t obj_run(const ObjArgs &a0, char *scratch, cudaStream_t st) {
   float *Um = reinterpret_cast<float *>(scratch + L.Um);
   float *gw = reinterpret_cast<float *>(scratch + L.gw);
   const StreamPlan pl = stream_plan(a.S, M, a.R, a.C, a.grad_Y != nullptr);
-  if (pl.ok && pl.grid <= 512 &&
+  if (pl.ok &&
       !((reinterpret_cast<uintptr_t>(a.Hd) | reinterpret_cast<uintptr_t>(ms ? a.Hr : a.Hd)) & 15)) {
     float *Pp = reinterpret_cast<float *>(scratch + L.Pp);
     double *lp = reinterpret_cast<double *>(scratch + L.lp);
@@ -2023,8 +2223,9 @@ cudaError_t obj_run(const ObjArgs &a0, char *scratch, cudaStream_t st) {
 // ------------------------------------------------------------------ plans
 struct ObjTcPlan {
   const float *Hd, *Ha, *Hr;
-  // stream mode (C_max <= 2): transposed FP32 copy and the streaming kernels
-  bool stream = false;
+  // stream mode (C_max <= 2): the streaming kernels, over the channels
+  // themselves (direct) or a transposed FP32 copy
+  bool stream = false, direct = false;
   float *HT = nullptr;
   int tKp = 0, tTR = 0, tKPT = 0, tStage = 0, tTiles = 0, tGrid = 0;
   size_t tSmem = 0, oPp = 0, oLp = 0, oGwS = 0;
@@ -2038,6 +2239,37 @@ struct ObjTcPlan {
 };
 
 namespace {
+// Stream mode over the channels themselves, where k_obj_stream takes them: an
+// even number of Rx, 16-byte aligned arrays, K up to about 3,200.  The
+// transposed copy is no faster there (S = 16, C = 1: R = 65,536, M = 1,024 133
+// against 127 us, M = 2,304 266 against 253 us; R = 4,096, M = 1,024 23.8
+// against 21.6 us), and a plan without it costs nothing to make.
+bool plan_direct(int S, int M, int R, int Cmax, const float *Hd, const float *Hr) {
+  if ((reinterpret_cast<uintptr_t>(Hd) | reinterpret_cast<uintptr_t>(Hr)) & 15) return false;
+  for (int C = 1; C <= Cmax; C++)
+    if (!stream_plan(S, M, R, C, false).ok) return false;
+  return true;
+}
+cudaError_t plan_direct_create(ObjTcPlan *p, cudaStream_t st, ObjTcPlan **out) {
+  auto al = [](size_t v) { return (v + 255) & ~(size_t)255; };
+  const int nparts = std::min(kMaxClusters, (p->R + 7) / 8);
+  size_t o = 0;
+  p->oCtl = o; o += kObjControlBytes;
+  p->oU = o; o += al(8 * (size_t)p->Cmax * p->M);
+  p->oPp = o; o += al(8 * (size_t)nparts * 2 * p->Cmax * p->K);
+  p->oLp = o; o += al(16 * (size_t)nparts);
+  p->oGwS = o; o += al(8 * (size_t)p->Cmax * p->K);
+  p->oDw = o; o += al(8 * (size_t)((p->K + 31) / 32) * p->Cmax * p->S);
+  p->bytes = o;
+  cudaError_t e = cudaMalloc(&p->mem, o);
+  if (e != cudaSuccess) { delete p; return e; }
+  p->stream = p->direct = true;
+  e = cudaMemsetAsync(p->mem + p->oCtl, 0, kObjControlBytes, st);
+  if (e != cudaSuccess) { cudaFree(p->mem); delete p; return e; }
+  *out = p;
+  return cudaSuccess;
+}
+
 // Stream mode: HT [Rp][Kp] holds [H_r; H_d] transposed (FP32 complex, rows
 // padded to an even length so a tile is a whole number of 16-byte units).
 cudaError_t plan_stream_create(ObjTcPlan *p, cudaStream_t st, ObjTcPlan **out) {
@@ -2133,6 +2365,9 @@ cudaError_t run_plan_stream(ObjTcPlan *p, const ObjArgs &a, cudaStream_t st) {
   char *ctl = p->mem + p->oCtl;
   unsigned *counter = reinterpret_cast<unsigned *>(ctl + 40);
   unsigned *err = reinterpret_cast<unsigned *>(ctl + 48);
+  if (p->direct)
+    return run_stream<CB>(a, stream_plan(p->S, M, p->R, a.C, false), M, U, Pp, lp, gw,
+                          reinterpret_cast<float *>(p->mem + p->oDw), err, counter, st);
   const long long n = (long long)M * a.C * 8;
   k_prep_wide<<<(int)((n + 255) / 256), 256, 0, st>>>(a, M, U, err);
   cudaError_t e = obj_begin_call(err, true, st);
@@ -2166,6 +2401,8 @@ cudaError_t obj_tc_plan_create(const float *Hd, const float *Ha, const float *Hr
   // stream mode when the streaming kernel's per-thread rows cover K (16 rows
   // a thread for one code, 8 for two); otherwise the tensor-core mode
   const int kpt = (p->K + 255) / 256;
+  if (!force_tc && Cmax <= 2 && plan_direct(S, M, R, Cmax, Hd, Hr))
+    return plan_direct_create(p, st, out);
   if (!force_tc && Cmax <= 2 && kpt <= (Cmax == 1 ? 16 : 8)) return plan_stream_create(p, st, out);
   pick_split((p->Rp / tcg::BN) * (p->Mp / tcg::BM), p->Kp / tcg::BK, sms, p->ksy, p->kpy);
   pick_split((p->Np / tcg::BN) * (p->Mp / tcg::BM), p->K2p / tcg::BK, sms, p->ksg, p->kpg);

@@ -30,6 +30,9 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes) {
                "r"(bytes)
                : "memory");
 }
+__device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
 // try_wait with a suspend-time hint (ns): the thread sleeps until the phase
 // completes or the hint runs out, instead of spinning on the barrier
 constexpr uint32_t kSuspendNs = 1000000u;

@@ -282,7 +282,7 @@ class Model(nn.Module):
                  global_random=False, drop_rate=0.1, device="cuda", plans=True):
         super().__init__()
         # one metasurface hop: an ObjectivePlan per channel set (made on first
-        # use; C <= 2 streams a transposed copy, larger codebooks run on the
+        # use; C <= 2 streams the channels in FP32, larger codebooks run on the
         # tensor cores)
         self.use_plans = bool(plans) and code_num <= 64
         self._plans = {}

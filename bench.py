@@ -328,7 +328,7 @@ def objective_bench(torch, steps, flush, cpu_baseline=False):
             "ms_per_eval": t, "evals": reps * NSET,
             "config": {"S": S, "M": M, "R": R, "C": 1,
                        "l2": "8 channel sets (274 MB) evaluated in turn, CUDA-graph replay",
-                       "path": "evaluation plan per channel set (transposed FP32 copy)",
+                       "path": "evaluation plan per channel set (FP32 streaming kernels)",
                        "plan_create_ms": t_plan * 1e3},
             "direct_call": {"value": 1e3 / t_direct, "ms_per_eval": t_direct,
                             "max_rel_loss_diff": rel},
