@@ -1014,6 +1014,70 @@ ams_status ams_objective_plan_coef_fwd_bwd(ams_objective_plan *plan, const float
   return AMS_OK;
 }
 
+unsigned long long ams_objective_multihop_scratch(const ams_objective_plan *plan, int C,
+                                                  int hops) {
+  if (!plan || C <= 0 || hops <= 0) return 0;
+  return mh_scratch_bytes(plan->M, C, plan->S, hops);
+}
+
+ams_status ams_objective_multihop_fwd_bwd(ams_objective_plan *plan, int n_ms, const int *sizes,
+                                          int hops, const float *const *H_a,
+                                          const float *const *H_mm, const float *phi,
+                                          const float *max_phase, const float *W, int C, float w,
+                                          const uint8_t *drop, float *loss, float *grad_W,
+                                          float *grad_phi, float *recv_amp, void *scratch,
+                                          void *stream, char *errbuf, size_t errlen) {
+  clear_stale_error();
+  if (!plan || !plan->p) { set_err(errbuf, errlen, "plan is NULL"); return AMS_ERR_ARG; }
+  if (!plan->stacked) {
+    set_err(errbuf, errlen, "paths over metasurfaces need a plan from ams_objective_plan_create_stacked");
+    return AMS_ERR_ARG;
+  }
+  if (n_ms < 1 || n_ms > kMhMax || hops < 1) {
+    set_err(errbuf, errlen, "need 1 <= n_ms <= %d and hops >= 1 (n_ms=%d hops=%d)", kMhMax, n_ms, hops);
+    return AMS_ERR_ARG;
+  }
+  if (!sizes || !H_a || !phi || !max_phase || !W || !loss || !scratch ||
+      (hops > 1 && n_ms > 1 && !H_mm)) {
+    set_err(errbuf, errlen, "null argument");
+    return AMS_ERR_ARG;
+  }
+  if (C <= 0 || C > plan->Cmax) {
+    set_err(errbuf, errlen, "C=%d outside [1, %d] of this plan", C, plan->Cmax);
+    return AMS_ERR_ARG;
+  }
+  MhArgs m{};
+  m.n = n_ms;
+  m.hops = hops;
+  m.phi = phi;
+  m.grad_phi = grad_phi;
+  long long total = 0;
+  for (int i = 0; i < n_ms; i++) {
+    m.size[i] = sizes[i];
+    m.Ha[i] = H_a[i];
+    m.max_phase[i] = max_phase[i];
+    total += sizes[i];
+    if (sizes[i] <= 0 || !H_a[i] || !(max_phase[i] > 0.f)) {
+      set_err(errbuf, errlen, "metasurface %d: size %d, max_phase %g or H_a missing", i, sizes[i],
+              (double)max_phase[i]);
+      return AMS_ERR_ARG;
+    }
+    for (int j = i + 1; j < n_ms && hops > 1; j++)
+      if (!(m.Hmm[i * n_ms + j] = H_mm[i * n_ms + j])) {
+        set_err(errbuf, errlen, "the channel between metasurfaces %d and %d is missing", i, j);
+        return AMS_ERR_ARG;
+      }
+  }
+  if (total != plan->M) {
+    set_err(errbuf, errlen, "the metasurfaces have %lld elements, the plan %d", total, plan->M);
+    return AMS_ERR_ARG;
+  }
+  ObjArgs a{nullptr, nullptr, nullptr, nullptr, W, 1.0f, plan->S, plan->M, plan->R, C, w, drop,
+            loss, grad_W, nullptr, recv_amp, nullptr};
+  CK(mh_run(plan->p, m, a, static_cast<char *>(scratch), (cudaStream_t)stream));
+  return AMS_OK;
+}
+
 ams_status ams_cgemm(int m, int n, int k, const float *A, int lda, int opA, const float *B,
                      int ldb, int opB, float *Cm, int ldc, int accumulate, void *stream,
                      char *errbuf, size_t errlen) {

@@ -2639,6 +2639,306 @@ __global__ void __launch_bounds__(256) k_cgemm_small(int m, int n, int k, const 
 }
 }  // namespace
 
+// ------------------------------------------------------------------
+// Paths over several metasurfaces (go.py:107-157).  With V^l_m the sum, over the
+// paths of l hops that end on metasurface m, of the path products,
+//   V^1_m = (W H_a^m) o e_m,  V^(l+1)_m = (sum_{m' != m} V^l_m' H^(m'm)) o e_m,
+//   U_m = sum_l V^l_m,  e = exp(j phi'),
+// and of the adjoint, with G_U from the stacked evaluation,
+//   D^hops_m = G_U,m,  D^l_m = G_U,m + sum_{m' != m} (D^(l+1)_m' o conj e_m') H^(mm')^H,
+//   dphi_m = -sum_l Im(conj(D^l_m) o V^l_m) over the codes,
+//   dW = G_W + sum_m (D^1_m o conj e_m) (H_a^m)^H.
+// (H^(m'm) = H^(mm')^T: only m < m' is stored.)  A level is one launch: a CTA
+// forms 32 codes x 16 elements of one metasurface from all its sources.  Path
+// by path, the step took a product per path and hop and eight elementwise
+// launches beside each, all issued from Python, and that bound it: a step with
+// its backward pass, two hops, C = 30, S = 36: M = 576 + 256, R = 2,116 2,390 ->
+// 790 us; M = 2,304 + 1,024 2,375 -> 1,087 us; three hops over 3 x 1,024, C = 64,
+// R = 1,000 11.5 -> 1.6 ms.  The products are FP32 FMAs (what is stored is read
+// once per 32 codes); the kernel is bound by its shared-memory reads.
+namespace {
+struct MhSrc {
+  const float2 *A;  // [C, k], lda
+  const float2 *e;  // A's columns are multiplied by conj(e[k]) (NULL: not)
+  const float2 *B;  // op(B) [k, n]
+  int lda, ldb, op, k;
+};
+struct MhDst {
+  float2 *out;        // [C, n], ldo
+  const float2 *add;  // added (ld ldo), or NULL
+  const float2 *e;    // out's columns multiplied by e[n], or NULL
+  float2 *sum;        // out also goes here (ld ldo): stored, or added with sum_add
+  int ldo, n, nsrc, tile0, sum_add;
+  MhSrc src[kMhMax];
+};
+struct MhLevel {
+  int C, ndst;
+  MhDst dst[kMhMax];
+};
+constexpr int kMhK = 64;  // inner dimension staged at a time
+
+__global__ void __launch_bounds__(256) k_mh_gemm(const __grid_constant__ MhLevel lv) {
+  __shared__ float2 As[kMhK][33];
+  __shared__ __align__(16) float2 Bs[kMhK][16];
+  int di = 0;
+  while (di + 1 < lv.ndst && (int)blockIdx.x >= lv.dst[di + 1].tile0) di++;
+  const MhDst &d = lv.dst[di];
+  const int n0 = ((int)blockIdx.x - d.tile0) * 16, c0 = blockIdx.y * 32;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  c2 acc0 = {0.f, 0.f}, acc1 = {0.f, 0.f};  // columns 2 warp, 2 warp + 1 of row lane
+  for (int si = 0; si < d.nsrc; si++) {
+    const MhSrc &s = d.src[si];
+    const bool trans = s.op == 1 || s.op == 2;
+    const float conj_b = s.op >= 2 ? -1.f : 1.f;
+    float2 ra[8], rb[4];
+    auto fetch = [&](int k0) {
+#pragma unroll
+      for (int i = 0; i < 8; i++) {  // thread t: column t % 64 of rows t / 64 + 4 i
+        const int k = k0 + (t & 63), r = c0 + (t >> 6) + 4 * i;
+        ra[i] = make_float2(0.f, 0.f);
+        if (k < s.k && r < lv.C) {
+          ra[i] = __ldg(s.A + (size_t)r * s.lda + k);
+          if (s.e) {
+            const float2 e = __ldg(s.e + k), x = ra[i];
+            ra[i] = make_float2(x.x * e.x + x.y * e.y, x.y * e.x - x.x * e.y);
+          }
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        const int q = t + 256 * i;
+        const int kk = trans ? q % kMhK : q / 16, col = trans ? q / kMhK : q % 16;
+        const int k = k0 + kk, n = n0 + col;
+        rb[i] = make_float2(0.f, 0.f);
+        if (k < s.k && n < d.n) {
+          rb[i] = __ldg(s.B + (trans ? (size_t)n * s.ldb + k : (size_t)k * s.ldb + n));
+          rb[i].y *= conj_b;
+        }
+      }
+    };
+    fetch(0);
+    for (int k0 = 0; k0 < s.k; k0 += kMhK) {
+      __syncthreads();
+#pragma unroll
+      for (int i = 0; i < 8; i++) As[t & 63][(t >> 6) + 4 * i] = ra[i];
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        const int q = t + 256 * i;
+        const int kk = trans ? q % kMhK : q / 16, col = trans ? q / kMhK : q % 16;
+        Bs[kk][col] = rb[i];
+      }
+      __syncthreads();
+      if (k0 + kMhK < s.k) fetch(k0 + kMhK);  // in flight during the products
+#pragma unroll 8
+      for (int k = 0; k < kMhK; k++) {
+        const float2 x = As[k][lane];
+        const float4 b = *reinterpret_cast<const float4 *>(&Bs[k][2 * warp]);
+        mac(acc0, c2{x.x, x.y}, c2{b.x, b.y});
+        mac(acc1, c2{x.x, x.y}, c2{b.z, b.w});
+      }
+    }
+  }
+  const int c = c0 + lane;
+  if (c >= lv.C) return;
+#pragma unroll
+  for (int j = 0; j < 2; j++) {
+    const int n = n0 + 2 * warp + j;
+    if (n >= d.n) continue;
+    c2 v = j ? acc1 : acc0;
+    const size_t o = (size_t)c * d.ldo + n;
+    if (d.add) { const float2 x = __ldg(d.add + o); v.x += x.x; v.y += x.y; }
+    if (d.e) {
+      const float2 e = __ldg(d.e + n);
+      v = {v.x * e.x - v.y * e.y, v.x * e.y + v.y * e.x};
+    }
+    d.out[o] = make_float2(v.x, v.y);
+    if (d.sum) {
+      const float2 x = d.sum_add ? d.sum[o] : make_float2(0.f, 0.f);
+      d.sum[o] = make_float2(x.x + v.x, x.y + v.y);
+    }
+  }
+}
+
+// e[m] = exp(j (phi[m] mod max_phase of its metasurface))
+struct MhSizes { int n; int first[kMhMax + 1]; float max_phase[kMhMax]; };
+__global__ void __launch_bounds__(256) k_mh_phase(const float *phi, MhSizes z, float2 *e) {
+  const int m = blockIdx.x * blockDim.x + threadIdx.x;
+  if (m >= z.first[z.n]) return;
+  int i = 0;
+  while (m >= z.first[i + 1]) i++;
+  float sn, cs;
+  sincosf(py_mod(__ldg(phi + m), z.max_phase[i]), &sn, &cs);
+  e[m] = make_float2(cs, sn);
+}
+
+// dphi[m] = -sum over levels and codes of Im(conj(D) V); a CTA takes 32
+// elements (lanes), its 8 warps split the levels' codes.  D of the last level is
+// G_U (gu); the others lie behind each other in D, all V in V ([hops][C][M]).
+__global__ void __launch_bounds__(256) k_mh_dphi(const float2 *V, const float2 *D, const float2 *gu,
+                                                 int hops, int C, int M, float *dphi) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int m = blockIdx.x * 32 + lane;
+  float acc = 0.f;
+  if (m < M)
+    for (int q = wid; q < hops * C; q += 8) {
+      const int l = q / C, c = q - l * C;
+      const float2 v = __ldg(V + (size_t)q * M + m);
+      const float2 g = __ldg((l == hops - 1 ? gu + (size_t)c * M : D + (size_t)q * M) + m);
+      acc += g.x * v.y - g.y * v.x;  // Im(conj(g) v)
+    }
+  __shared__ float red[8][32];
+  red[wid][lane] = acc;
+  __syncthreads();
+  if (wid == 0 && m < M) {
+    float t = 0.f;
+#pragma unroll
+    for (int w = 0; w < 8; w++) t += red[w][lane];
+    dphi[m] = -t;
+  }
+}
+
+cudaError_t mh_launch(MhLevel &lv, cudaStream_t st) {
+  int tiles = 0;
+  for (int i = 0; i < lv.ndst; i++) {
+    lv.dst[i].tile0 = tiles;
+    tiles += (lv.dst[i].n + 15) / 16;
+  }
+  k_mh_gemm<<<dim3(tiles, (lv.C + 31) / 32), 256, 0, st>>>(lv);
+  return cudaGetLastError();
+}
+}  // namespace
+
+size_t mh_scratch_bytes(int M, int C, int S, int hops) {
+  auto al = [](size_t v) { return (v + 255) & ~(size_t)255; };
+  const size_t cm = 8 * (size_t)C * M;
+  return al(8 * (size_t)M) + al(cm * hops) + al(cm * std::max(hops - 1, 0)) + 2 * al(cm) +
+         al(8 * (size_t)C * S);
+}
+
+cudaError_t mh_run(ObjTcPlan *p, const MhArgs &m, const ObjArgs &a0, char *scratch,
+                   cudaStream_t st) {
+  if (m.n < 1 || m.n > kMhMax || m.hops < 1) return cudaErrorInvalidValue;
+  const int M = p->M, C = a0.C, S = p->S, n = m.n;
+  auto al = [](size_t v) { return (v + 255) & ~(size_t)255; };
+  const size_t cm = (size_t)C * M;
+  char *at = scratch;
+  auto take = [&](size_t bytes) { float2 *r = reinterpret_cast<float2 *>(at); at += al(bytes); return r; };
+  float2 *e = take(8 * (size_t)M), *V = take(8 * cm * m.hops),
+         *D = take(8 * cm * std::max(m.hops - 1, 0)), *U = take(8 * cm), *gU = take(8 * cm),
+         *gW = take(8 * (size_t)C * S);
+  MhSizes z{};
+  z.n = n;
+  for (int i = 0; i < n; i++) {
+    z.first[i + 1] = z.first[i] + m.size[i];
+    z.max_phase[i] = m.max_phase[i];
+  }
+  if (z.first[n] != M) return cudaErrorInvalidValue;
+  k_mh_phase<<<(M + 255) / 256, 256, 0, st>>>(m.phi, z, e);
+  cudaError_t err = cudaGetLastError();
+  if (err != cudaSuccess) return err;
+  // H between metasurfaces a -> b as op(B) of what is stored
+  auto between = [&](int a, int b, bool adjoint, MhSrc &s) {
+    const int lo = std::min(a, b), hi = std::max(a, b);
+    s.B = reinterpret_cast<const float2 *>(m.Hmm[lo * n + hi]);
+    s.ldb = m.size[hi];
+    const bool trans = (a > b) != adjoint;  // stored as [lo, hi]
+    s.op = (trans ? 1 : 0);
+    if (adjoint) s.op = trans ? 2 : 3;
+  };
+  // paths forward
+  for (int l = 0; l < m.hops; l++) {
+    MhLevel lv{};
+    lv.C = C;
+    lv.ndst = n;
+    for (int i = 0; i < n; i++) {
+      MhDst &d = lv.dst[i];
+      d.out = V + cm * l + z.first[i];
+      d.ldo = M;
+      d.n = m.size[i];
+      d.e = e + z.first[i];
+      d.sum = U + z.first[i];
+      d.sum_add = l > 0;
+      if (l == 0) {
+        d.nsrc = 1;
+        MhSrc &s = d.src[0];
+        s.A = reinterpret_cast<const float2 *>(a0.W);
+        s.lda = S;
+        s.k = S;
+        s.B = reinterpret_cast<const float2 *>(m.Ha[i]);
+        s.ldb = m.size[i];
+      } else {
+        for (int j = 0; j < n; j++) {
+          if (j == i) continue;
+          MhSrc &s = d.src[d.nsrc++];
+          s.A = V + cm * (l - 1) + z.first[j];
+          s.lda = M;
+          s.k = m.size[j];
+          between(j, i, false, s);
+        }
+      }
+    }
+    if ((err = mh_launch(lv, st)) != cudaSuccess) return err;
+  }
+  ObjArgs a = a0;
+  a.U_in = reinterpret_cast<const float *>(U);
+  a.grad_U = reinterpret_cast<float *>(gU);
+  a.grad_W = reinterpret_cast<float *>(gW);
+  a.grad_phi = nullptr;
+  if ((err = obj_tc_run(p, a, st)) != cudaSuccess) return err;
+  // adjoint: D^(l + 1) is G_U for the last level, else at D + cm l
+  for (int l = m.hops - 2; l >= 0; l--) {
+    const float2 *next = l + 1 == m.hops - 1 ? gU : D + cm * (l + 1);
+    MhLevel lv{};
+    lv.C = C;
+    lv.ndst = n;
+    for (int i = 0; i < n; i++) {
+      MhDst &d = lv.dst[i];
+      d.out = D + cm * l + z.first[i];
+      d.add = gU + z.first[i];
+      d.ldo = M;
+      d.n = m.size[i];
+      for (int j = 0; j < n; j++) {
+        if (j == i) continue;
+        MhSrc &s = d.src[d.nsrc++];
+        s.A = next + z.first[j];
+        s.lda = M;
+        s.k = m.size[j];
+        s.e = e + z.first[j];
+        between(i, j, true, s);  // (H^(ij))^H [M_j, M_i]
+      }
+    }
+    if ((err = mh_launch(lv, st)) != cudaSuccess) return err;
+  }
+  const float2 *D1 = m.hops == 1 ? gU : D;
+  if (a0.grad_W) {
+    MhLevel lv{};
+    lv.C = C;
+    lv.ndst = 1;
+    MhDst &d = lv.dst[0];
+    d.out = reinterpret_cast<float2 *>(a0.grad_W);
+    d.add = gW;
+    d.ldo = S;
+    d.n = S;
+    d.nsrc = n;
+    for (int i = 0; i < n; i++) {
+      MhSrc &s = d.src[i];
+      s.A = D1 + z.first[i];
+      s.lda = M;
+      s.k = m.size[i];
+      s.e = e + z.first[i];
+      s.B = reinterpret_cast<const float2 *>(m.Ha[i]);
+      s.ldb = m.size[i];
+      s.op = 2;
+    }
+    if ((err = mh_launch(lv, st)) != cudaSuccess) return err;
+  }
+  if (m.grad_phi) {
+    k_mh_dphi<<<(M + 31) / 32, 256, 0, st>>>(V, D, gU, m.hops, C, M, m.grad_phi);
+    err = cudaGetLastError();
+  }
+  return err;
+}
+
 cudaError_t cgemm_run(int m, int n, int k, const float *A, int lda, int opA, const float *B,
                       int ldb, int opB, float *C, int ldc, bool accumulate, cudaStream_t st) {
   if (m <= 0 || n <= 0 || k <= 0 || opA < 0 || opA > 3 || opB < 0 || opB > 3)

@@ -64,6 +64,22 @@ const unsigned *obj_tc_plan_status_word(const ObjTcPlan *p);
 bool obj_tc_plan_streams(const ObjTcPlan *p);
 void obj_tc_plan_destroy(ObjTcPlan *p);
 
+// Several metasurfaces (kMhMax at most), metasurface paths of up to `hops` hops:
+// the whole evaluation on a stacked plan.  Ha[i] [S, M_i]; Hmm[i * n + j] for
+// i < j [M_i, M_j] (hops > 1); phi, grad_phi over all elements; scratch of
+// mh_scratch_bytes.
+constexpr int kMhMax = 8;
+struct MhArgs {
+  int n, hops;
+  int size[kMhMax];
+  const float *Ha[kMhMax], *Hmm[kMhMax * kMhMax];
+  const float *phi;
+  float max_phase[kMhMax];
+  float *grad_phi;  // may be NULL
+};
+size_t mh_scratch_bytes(int M, int C, int S, int hops);
+cudaError_t mh_run(ObjTcPlan *p, const MhArgs &m, const ObjArgs &a, char *scratch, cudaStream_t st);
+
 // C = op(A) op(B) (+ C when accumulate) for row-major complex64 matrices on
 // the CUDA cores; op 0 = as is, 1 = transposed, 2 = conjugate transposed,
 // 3 = conjugated.

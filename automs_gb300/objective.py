@@ -255,6 +255,60 @@ class MultiHopObjective(torch.autograd.Function):
         return (dW.to(ctx.w_dtype), dphi, None, None, None, None, None, None, None)
 
 
+class FusedMultiHop(torch.autograd.Function):
+    """MultiHopObjective for up to FUSED_MS metasurfaces and every path of up
+    to `hops` hops: one library call (ams_objective_multihop_fwd_bwd) forms the
+    path products level by level, the stacked evaluation and both gradients;
+    backward only scales them."""
+
+    @staticmethod
+    def forward(ctx, W, phi_cat, plan, chans, max_phases, hops, w, drop, want_recv):
+        Wc = _c64(W.detach())
+        Cc, n, dev = Wc.shape[0], len(plan.sizes), W.device
+        Ha = [_c64(chans["src_to_ms{%d}" % i].detach()) for i in range(n)]
+        Hmm = [None] * (n * n)
+        if hops > 1:
+            for i in range(n):
+                for j in range(i + 1, n):
+                    Hmm[i * n + j] = _c64(chans["ms{%d}_to_ms{%d}" % (i, j)].detach())
+        for i, m in enumerate(plan.sizes):
+            if tuple(Ha[i].shape) != (plan.S, m) or any(
+                    h is not None and tuple(h.shape) != (m, plan.sizes[j])
+                    for j, h in enumerate(Hmm[i * n:(i + 1) * n])):
+                raise ValueError("channel shapes do not match the plan")
+        if tuple(Wc.shape[1:]) != (plan.S,) or phi_cat.shape != (plan.M,):
+            raise ValueError("W or the phases do not match the plan")
+        ph = phi_cat.detach().to(torch.float32).contiguous()
+        loss = torch.empty((), dtype=torch.float32, device=dev)
+        grads = torch.empty(2 * Cc * plan.S + plan.M, dtype=torch.float32, device=dev)
+        recv = torch.empty(Cc, plan.R, dtype=torch.float32, device=dev) if want_recv else None
+        dr = drop.to(device=dev, dtype=torch.uint8).contiguous() if drop is not None else None
+        scratch = torch.empty(int(lib().ams_objective_multihop_scratch(plan._h, Cc, hops)),
+                              dtype=torch.uint8, device=dev)
+        call("ams_objective_multihop_fwd_bwd", plan._h, n, (C.c_int * n)(*plan.sizes), hops,
+             (C.c_void_p * n)(*[h.data_ptr() for h in Ha]),
+             (C.c_void_p * (n * n))(*[h.data_ptr() if h is not None else None for h in Hmm]),
+             _ptr(ph), (C.c_float * n)(*max_phases), _ptr(Wc), Cc, float(w), _ptr(dr), _ptr(loss),
+             _ptr(grads), C.c_void_p(grads.data_ptr() + 8 * Cc * plan.S), _ptr(recv),
+             _ptr(scratch), _stream())
+        ctx.save_for_backward(grads)
+        ctx.w_shape, ctx.w_dtype = tuple(Wc.shape), W.dtype
+        if recv is not None:
+            ctx.mark_non_differentiable(recv)
+            return loss, recv
+        return loss, torch.empty(0, device=dev)
+
+    @staticmethod
+    def backward(ctx, gl, _grecv):
+        g = ctx.saved_tensors[0] * gl
+        k = 2 * ctx.w_shape[0] * ctx.w_shape[1]
+        dW = torch.view_as_complex(g[:k].view(*ctx.w_shape, 2)).to(ctx.w_dtype)
+        return (dW, g[k:], None, None, None, None, None, None, None)
+
+
+FUSED_MS = 8  # metasurfaces that the one-call evaluation takes
+
+
 def check_status(plan=None):
     """Raise AmsError if a bounded wait of the last objective call ran out
     (its outputs are then NaN): the last call on `plan`, or with plan=None the
@@ -383,8 +437,8 @@ class Model(nn.Module):
                 loss, recv = capacity_objective(W, ch["src_to_dst"], w=self.w, drop=drop,
                                                 return_recv=True)
         else:
-            # several metasurfaces / hops: path products on the library's
-            # complex GEMM, one stacked tensor-core evaluation
+            # several metasurfaces / hops: path products, one stacked
+            # tensor-core evaluation
             ch = self.pick_channel(True)
             n = len(self.ms_list)
             plan = self._plans.get(("stacked", id(ch)))
@@ -392,9 +446,11 @@ class Model(nn.Module):
                 plan = StackedPlan(ch["src_to_dst"], [ch["ms{%d}_to_dst" % i] for i in range(n)],
                                    c_max=C_)
                 self._plans[("stacked", id(ch))] = plan
-            loss, recv = MultiHopObjective.apply(
+            fused = n <= FUSED_MS and all(m.max_phase > 0 for m in self.ms_list)
+            loss, recv = (FusedMultiHop if fused else MultiHopObjective).apply(
                 W, torch.cat(list(self.ms_theta)), plan, ch,
-                [m.max_phase for m in self.ms_list], ms_paths(n, self.max_ms_reflex), self.w,
+                [m.max_phase for m in self.ms_list],
+                self.max_ms_reflex if fused else ms_paths(n, self.max_ms_reflex), self.w,
                 drop, True)
         self.result = recv.detach().clone()
         self.max_code_ids = recv.max(0)[1].detach().clone()

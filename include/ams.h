@@ -270,6 +270,23 @@ ams_status ams_objective_plan_coef_fwd_bwd(ams_objective_plan *plan,
                                            void *stream, char *errbuf,
                                            size_t errlen);
 
+/* The whole evaluation over several metasurfaces in one call (go.py:107-245):
+ * the products of every metasurface path of up to `hops` hops (no metasurface
+ * twice in a row), the stacked evaluation and the adjoint chained back through
+ * the products.  n_ms <= 8 metasurfaces of sizes[i] elements (their sum is the
+ * plan's M); H_a[i] [S, sizes[i]]; H_mm[i * n_ms + j], i < j, [sizes[i],
+ * sizes[j]], needed with hops > 1; max_phase[i]; sizes, the pointer arrays and
+ * max_phase are host memory.  phi and grad_phi run over all elements.  scratch:
+ * device memory of ams_objective_multihop_scratch(...) bytes, 256-byte
+ * aligned, in use until the call's work has run.  Outputs but loss may be
+ * NULL.  Asynchronous. */
+unsigned long long ams_objective_multihop_scratch(const ams_objective_plan *plan, int C, int hops);
+ams_status ams_objective_multihop_fwd_bwd(
+    ams_objective_plan *plan, int n_ms, const int *sizes, int hops, const float *const *H_a,
+    const float *const *H_mm, const float *phi, const float *max_phase, const float *W, int C,
+    float w, const uint8_t *drop, float *loss, float *grad_W, float *grad_phi, float *recv_amp,
+    void *scratch, void *stream, char *errbuf, size_t errlen);
+
 /* C = op(A) op(B) (+ C when accumulate != 0) for row-major complex64
  * device matrices (interleaved float pairs) on the CUDA cores, FP32: op 0
  * as is, 1 transposed, 2 conjugate transposed, 3 conjugated; C is m x n, k the inner
