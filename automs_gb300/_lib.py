@@ -124,10 +124,18 @@ def lib():
         return L
 
 
+_tls = threading.local()
+
+
 def call(name, *args):
-    """Call an entry point that ends with (errbuf, errlen); raise on failure."""
-    buf = C.create_string_buffer(1024)
-    rc = getattr(lib(), name)(*args, buf, C.sizeof(buf))
+    """Call an entry point that ends with (errbuf, errlen); raise on failure.
+    Each thread keeps one message buffer."""
+    try:
+        buf = _tls.buf
+    except AttributeError:
+        buf = _tls.buf = C.create_string_buffer(1024)
+    buf[0] = 0
+    rc = getattr(_lib or lib(), name)(*args, buf, 1024)
     if rc != AMS_OK:
         raise AmsError(rc, buf.value.decode(errors="replace"))
     return rc

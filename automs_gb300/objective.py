@@ -30,6 +30,20 @@ def _c64(t):
     return t if t.is_contiguous() else t.contiguous()
 
 
+def _at(t):
+    return t.data_ptr() if t is not None else None
+
+
+def _drop(drop, device):
+    """The dropped codes as bytes on the device (a boolean mask that is there
+    already is read in place)."""
+    if drop is None:
+        return None
+    if drop.dtype == torch.bool and drop.device == device and drop.is_contiguous():
+        return drop.view(torch.uint8)
+    return drop.to(device=device, dtype=torch.uint8).contiguous()
+
+
 class ObjectivePlan:
     """Tensor-core objective for a fixed channel set (ams_objective_plan_*).
 
@@ -74,47 +88,52 @@ class CapacityObjective(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, W, phi, H_d, H_a, H_r, max_phase, w, drop, want_recv, plan=None):
+        # (tensors are not recorded in here: no detach needed)
         Cc, S = W.shape
         R = H_d.shape[1]
         ms = H_a is not None
         M = H_a.shape[1] if ms else 0
-        Wc = _c64(W.detach())
-        Hd = _c64(H_d.detach())
-        Ha = _c64(H_a.detach()) if ms else None
-        Hr = _c64(H_r.detach()) if ms else None
-        ph = phi.detach().to(torch.float32).contiguous() if ms else None
-        loss = torch.empty((), dtype=torch.float32, device=W.device)
-        gW = torch.empty_like(Wc)
-        gphi = torch.empty(M, dtype=torch.float32, device=W.device) if ms else None
+        dev = W.device
+        Wc, Hd = _c64(W), _c64(H_d)
+        Ha = _c64(H_a) if ms else None
+        Hr = _c64(H_r) if ms else None
+        ph = phi.to(torch.float32).contiguous() if ms else None
+        loss = torch.empty((), dtype=torch.float32, device=dev)
+        gW = torch.empty(Cc, S, dtype=torch.complex64, device=dev)
+        gphi = torch.empty(M, dtype=torch.float32, device=dev) if ms else None
         need_gy = H_d.requires_grad
-        gY = torch.empty(Cc, R, dtype=torch.complex64, device=W.device) if need_gy else None
-        recv = torch.empty(Cc, R, dtype=torch.float32, device=W.device) if want_recv else None
-        dr = drop.to(device=W.device, dtype=torch.uint8).contiguous() if drop is not None else None
+        gY = torch.empty(Cc, R, dtype=torch.complex64, device=dev) if need_gy else None
+        recv = torch.empty(Cc, R, dtype=torch.float32, device=dev) if want_recv else None
+        dr = _drop(drop, dev)
+        out = (_at(dr), loss.data_ptr(), gW.data_ptr(), _at(gphi), _at(gY), _at(recv),
+               torch.cuda.current_stream().cuda_stream)
         if plan is not None:
             if not ms or (plan.S, plan.M, plan.R) != (S, M, R):
                 raise ValueError("the plan was made for other channel shapes")
-            call("ams_objective_plan_fwd_bwd", plan._h, _ptr(ph), float(max_phase), _ptr(Wc), Cc,
-                 float(w), _ptr(dr), _ptr(loss), _ptr(gW), _ptr(gphi), _ptr(gY), _ptr(recv),
-                 _stream())
+            call("ams_objective_plan_fwd_bwd", plan._h, ph.data_ptr(), float(max_phase),
+                 Wc.data_ptr(), Cc, float(w), *out)
         else:
-            call("ams_objective_fwd_bwd", _ptr(Hd), _ptr(Ha), _ptr(Hr), _ptr(ph),
-                 float(max_phase), _ptr(Wc), S, M, R, Cc, float(w), _ptr(dr), _ptr(loss),
-                 _ptr(gW), _ptr(gphi), _ptr(gY), _ptr(recv), _stream())
-        ctx.save_for_backward(gW, gphi if gphi is not None else torch.empty(0, device=W.device),
-                              gY if gY is not None else torch.empty(0, device=W.device), Wc)
-        ctx.ms = ms
+            call("ams_objective_fwd_bwd", Hd.data_ptr(), _at(Ha), _at(Hr), _at(ph),
+                 float(max_phase), Wc.data_ptr(), S, M, R, Cc, float(w), *out)
+        ctx.save_for_backward(gW, gphi, gY, Wc.detach() if need_gy else None)
         ctx.need_gy = need_gy
         ctx.w_dtype = W.dtype
+        # no zeros of [C, R] for the amplitudes, which have no gradient
+        ctx.set_materialize_grads(False)
         if recv is not None:
             ctx.mark_non_differentiable(recv)
             return loss, recv
-        return loss, torch.empty(0, device=W.device)
+        return loss, torch.empty(0, device=dev)
 
     @staticmethod
     def backward(ctx, gl, _grecv):
         gW, gphi, gY, Wc = ctx.saved_tensors
-        dW = (gW * gl).to(ctx.w_dtype) if ctx.needs_input_grad[0] else None
-        dphi = gphi * gl if (ctx.ms and ctx.needs_input_grad[1]) else None
+        if gl is None:
+            gl = torch.zeros((), dtype=torch.float32, device=gW.device)
+        dW = gW * gl if ctx.needs_input_grad[0] else None
+        if dW is not None and ctx.w_dtype != torch.complex64:
+            dW = dW.to(ctx.w_dtype)
+        dphi = gphi * gl if gphi is not None and ctx.needs_input_grad[1] else None
         dHd = None
         if ctx.need_gy and ctx.needs_input_grad[2]:
             # Y = W H_d  =>  dL/dH_d = W^H dL/dY (torch's complex convention)
@@ -263,14 +282,14 @@ class FusedMultiHop(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, W, phi_cat, plan, chans, max_phases, hops, w, drop, want_recv):
-        Wc = _c64(W.detach())
+        Wc = _c64(W)
         Cc, n, dev = Wc.shape[0], len(plan.sizes), W.device
-        Ha = [_c64(chans["src_to_ms{%d}" % i].detach()) for i in range(n)]
+        Ha = [_c64(chans["src_to_ms{%d}" % i]) for i in range(n)]
         Hmm = [None] * (n * n)
         if hops > 1:
             for i in range(n):
                 for j in range(i + 1, n):
-                    Hmm[i * n + j] = _c64(chans["ms{%d}_to_ms{%d}" % (i, j)].detach())
+                    Hmm[i * n + j] = _c64(chans["ms{%d}_to_ms{%d}" % (i, j)])
         for i, m in enumerate(plan.sizes):
             if tuple(Ha[i].shape) != (plan.S, m) or any(
                     h is not None and tuple(h.shape) != (m, plan.sizes[j])
@@ -278,21 +297,23 @@ class FusedMultiHop(torch.autograd.Function):
                 raise ValueError("channel shapes do not match the plan")
         if tuple(Wc.shape[1:]) != (plan.S,) or phi_cat.shape != (plan.M,):
             raise ValueError("W or the phases do not match the plan")
-        ph = phi_cat.detach().to(torch.float32).contiguous()
+        ph = phi_cat.to(torch.float32).contiguous()
         loss = torch.empty((), dtype=torch.float32, device=dev)
-        grads = torch.empty(2 * Cc * plan.S + plan.M, dtype=torch.float32, device=dev)
+        gW = torch.empty(Cc, plan.S, dtype=torch.complex64, device=dev)
+        gphi = torch.empty(plan.M, dtype=torch.float32, device=dev)
         recv = torch.empty(Cc, plan.R, dtype=torch.float32, device=dev) if want_recv else None
-        dr = drop.to(device=dev, dtype=torch.uint8).contiguous() if drop is not None else None
+        dr = _drop(drop, dev)
         scratch = torch.empty(int(lib().ams_objective_multihop_scratch(plan._h, Cc, hops)),
                               dtype=torch.uint8, device=dev)
         call("ams_objective_multihop_fwd_bwd", plan._h, n, (C.c_int * n)(*plan.sizes), hops,
              (C.c_void_p * n)(*[h.data_ptr() for h in Ha]),
-             (C.c_void_p * (n * n))(*[h.data_ptr() if h is not None else None for h in Hmm]),
-             _ptr(ph), (C.c_float * n)(*max_phases), _ptr(Wc), Cc, float(w), _ptr(dr), _ptr(loss),
-             _ptr(grads), C.c_void_p(grads.data_ptr() + 8 * Cc * plan.S), _ptr(recv),
-             _ptr(scratch), _stream())
-        ctx.save_for_backward(grads)
-        ctx.w_shape, ctx.w_dtype = tuple(Wc.shape), W.dtype
+             (C.c_void_p * (n * n))(*[_at(h) for h in Hmm]), ph.data_ptr(),
+             (C.c_float * n)(*max_phases), Wc.data_ptr(), Cc, float(w), _at(dr), loss.data_ptr(),
+             gW.data_ptr(), gphi.data_ptr(), _at(recv), scratch.data_ptr(),
+             torch.cuda.current_stream().cuda_stream)
+        ctx.save_for_backward(gW, gphi)
+        ctx.w_dtype = W.dtype
+        ctx.set_materialize_grads(False)
         if recv is not None:
             ctx.mark_non_differentiable(recv)
             return loss, recv
@@ -300,10 +321,13 @@ class FusedMultiHop(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, gl, _grecv):
-        g = ctx.saved_tensors[0] * gl
-        k = 2 * ctx.w_shape[0] * ctx.w_shape[1]
-        dW = torch.view_as_complex(g[:k].view(*ctx.w_shape, 2)).to(ctx.w_dtype)
-        return (dW, g[k:], None, None, None, None, None, None, None)
+        gW, gphi = ctx.saved_tensors
+        if gl is None:
+            gl = torch.zeros((), dtype=torch.float32, device=gW.device)
+        dW = gW * gl
+        if ctx.w_dtype != torch.complex64:
+            dW = dW.to(ctx.w_dtype)
+        return dW, gphi * gl, None, None, None, None, None, None, None
 
 
 FUSED_MS = 8  # metasurfaces that the one-call evaluation takes
