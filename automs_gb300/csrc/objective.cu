@@ -441,6 +441,26 @@ __global__ void __launch_bounds__(256) k_epilogue_wide(ObjArgs a, int kspl, cons
   }
 }
 
+// Operands lie k-block by k-block: 64 values (128 bytes) of row after row, so a
+// stage's tile is one contiguous piece of memory (its pieces of 128 bytes lay
+// 4 KB or more apart with K contiguous in a row: 211 us against 219 for the two
+// products of 60 codes, K = 1,040, R = 65,536).  In pairs of values: pair `col2` of row `row` of `rows`.
+__device__ __forceinline__ size_t kb_pair(int row, int col2, int rows) {
+  return ((size_t)(col2 >> 5) * rows + row) * 32 + (col2 & 31);
+}
+
+namespace tcg {
+constexpr int BM = 128, BK = 64, BN_MIN = 64, BN_MAX = 160, STAGES_MAX = 6;
+constexpr uint32_t A_BYTES = BM * BK * 2;  // one of the two A tiles of a stage
+constexpr uint32_t stage_bytes(int bn) { return 2 * A_BYTES + 2u * bn * BK * 2; }
+constexpr size_t SMEM = 225 * 1024;  // 1 KB of it for alignment
+constexpr int stages(int bn) {
+  const int n = (int)((SMEM - 1024) / stage_bytes(bn));
+  return n < STAGES_MAX ? n : STAGES_MAX;
+}
+static_assert(stages(BN_MAX) >= 3 && BN_MAX % 16 == 0, "stages");
+}  // namespace tcg
+
 // Two-phase epilogue of the tensor-core path (CB >= 8), same thread layout
 // as k_epilogue_wide.  Phase A: loss partials, and per Rx the max over codes
 // and its first index.  Phase B: re-reads Y, forms G = G1 + G2 / ||masked||
@@ -585,27 +605,35 @@ __global__ void __launch_bounds__(256) k_tc_epi_b(ObjArgs a, int kspl, const flo
       if (a.grad_Y) reinterpret_cast<float2 *>(a.grad_Y)[(size_t)c * a.R + r] = make_float2(g.x, g.y);
     }
     if (r < K2p / 2) {
-      put_pair(hi, lo, ((size_t)(2 * c) * K2p + 2 * r) / 2, g.x, g.y);
-      put_pair(hi, lo, ((size_t)(2 * c + 1) * K2p + 2 * r) / 2, g.y, -g.x);
+      put_pair(hi, lo, kb_pair(2 * c, r, tcg::BM), g.x, g.y);
+      put_pair(hi, lo, kb_pair(2 * c + 1, r, tcg::BM), g.y, -g.x);
     }
   }
 }
 
-// G_U[c, k] = sum over the splits of the partials, one thread per entry
-__global__ void k_gu_reduce(const float *GUp, int splits, long long n, float *GU) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+// G_U[c, k] = sum over the splits of the partials: 32 entries a CTA, its 8 warps
+// share the splits (one thread an entry and 70 splits took 6 us, latency)
+__global__ void __launch_bounds__(256) k_gu_reduce(const float *GUp, int splits, long long n,
+                                                   float *GU) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const long long i = (long long)blockIdx.x * 32 + lane;
   float x = 0.f, y = 0.f;
-  for (int s = 0; s < splits; s++) {
-    const float2 v = __ldg(reinterpret_cast<const float2 *>(GUp) + (size_t)s * n + i);
-    x += v.x;
-    y += v.y;
+  if (i < n)
+    for (int s = wid; s < splits; s += 8) {
+      const float2 v = __ldg(reinterpret_cast<const float2 *>(GUp) + (size_t)s * n + i);
+      x += v.x;
+      y += v.y;
+    }
+  __shared__ float2 red[8][32];
+  red[wid][lane] = make_float2(x, y);
+  __syncthreads();
+  if (wid == 0 && i < n) {
+#pragma unroll
+    for (int w = 1; w < 8; w++) { x += red[w][lane].x; y += red[w][lane].y; }
+    reinterpret_cast<float2 *>(GU)[i] = make_float2(x, y);
   }
-  reinterpret_cast<float2 *>(GU)[i] = make_float2(x, y);
 }
 
-// pass 2: partial G_U[c, k] = sum_r G[c, r] conj(row_k[r]) over an r-range;
-// one warp per row, lanes stride over columns, G staged in shared memory.
 template <int CB>
 __global__ void __launch_bounds__(256) k_pass2(ObjArgs a, int M, int K, int rper, const float *G1,
                                                const float *G2, const float *scal, float *GUp) {
@@ -765,51 +793,68 @@ __global__ void __launch_bounds__(256) k_tc_dphi(const float *GU, const float *U
 }
 
 // grad_W[c, s] = G_U[c, M + s] + sum_m G_U[c, m] e^{-j phi'_m} conj(H_a[s, m]).
-// k_tc_dw_part: CTA (c, part) takes a slice of the m range, one element per
-// thread, keeps 16 AP elements' sums at a time in registers (H_a loads
-// coalesced over m) and writes the CTA's sums to dwp[c][part][s];
-// k_tc_dw_sum adds the slices and the H_d term.
-constexpr int kDwParts = 8;
-__global__ void __launch_bounds__(128) k_tc_dw_part(const float *GU, const float *Ha,
-                                                    const float *phi, float max_phase, int S,
-                                                    int M, int K, float *dwp) {
-  constexpr int SB = 16;
-  __shared__ float2 red[4][SB];
-  const int c = blockIdx.x, part = blockIdx.y;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int per = (M + kDwParts - 1) / kDwParts;
+// k_tc_dw_part: a CTA forms 16 AP elements' sums of every code (64 at most) over
+// a slice of the m range, 32 of it in shared memory at a time, and writes them
+// to dwp[c][part][s]; k_tc_dw_sum adds the slices and the H_d term.  (A CTA per
+// code read all of H_a and formed every e^{-j phi'_m} for each code and was
+// bound by its shuffles: 18 us for M = 2,304, S = 36, 60 codes, 5 us now.)
+// Slices are whole 32s, one where that makes no more than 128 of them.
+int dw_parts(int M) {
+  const int n = (M + 31) / 32, per = (n + 127) / 128;
+  return (n + per - 1) / per;
+}
+__global__ void __launch_bounds__(256) k_tc_dw_part(const float *GU, const float *Ha,
+                                                    const float *phi, float max_phase, int C,
+                                                    int S, int M, int K, float *dwp) {
+  __shared__ c2 ge[32][65], ha[32][16];
+  const int part = blockIdx.x, parts = gridDim.x, s0 = blockIdx.y * 16;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int per = ((M + 31) / 32 + parts - 1) / parts * 32;
   const int m_lo = part * per, m_hi = min(M, m_lo + per);
-  for (int s0 = 0; s0 < S; s0 += SB) {
-    c2 acc[SB];
+  const int s = t & 15, cg = t >> 4;  // this thread's sums: codes cg + 16 j
+  c2 acc[4];
 #pragma unroll
-    for (int q = 0; q < SB; q++) acc[q] = {0.f, 0.f};
-    for (int m = m_lo + threadIdx.x; m < m_hi; m += blockDim.x) {
-      const float2 g = __ldg(reinterpret_cast<const float2 *>(GU) + (size_t)c * K + m);
-      float sn, cs;
-      sincosf(py_mod(__ldg(phi + m), max_phase), &sn, &cs);
-      const c2 ge = {g.x * cs + g.y * sn, g.y * cs - g.x * sn};  // g e^{-j p}
+  for (int j = 0; j < 4; j++) acc[j] = {0.f, 0.f};
+  for (int m0 = m_lo; m0 < m_hi; m0 += 32) {
+    const int m = m0 + lane;
+    const bool in = m < m_hi;
+    float sn = 0.f, cs = 0.f;
+    c2 g[8], h[2];
 #pragma unroll
-      for (int q = 0; q < SB; q++)
-        if (s0 + q < S) macc(acc[q], ge, ld2(Ha, (size_t)(s0 + q) * M + m));
+    for (int i = 0; i < 8; i++) {
+      const int c = warp + 8 * i;
+      g[i] = {0.f, 0.f};
+      if (in && c < C) g[i] = ld2(GU, (size_t)c * K + m);
     }
 #pragma unroll
-    for (int q = 0; q < SB; q++) {
-      float x = acc[q].x, y = acc[q].y;
-      for (int o = 16; o > 0; o >>= 1) {
-        x += __shfl_xor_sync(0xffffffffu, x, o);
-        y += __shfl_xor_sync(0xffffffffu, y, o);
-      }
-      if (lane == 0) red[wid][q] = make_float2(x, y);
+    for (int i = 0; i < 2; i++) {
+      const int q = s0 + warp + 8 * i;
+      h[i] = {0.f, 0.f};
+      if (in && q < S) h[i] = ld2(Ha, (size_t)q * M + m);
     }
+    if (in) sincosf(py_mod(__ldg(phi + m), max_phase), &sn, &cs);
     __syncthreads();
-    if (threadIdx.x < SB && s0 + threadIdx.x < S) {
-      float2 t = red[0][threadIdx.x];
 #pragma unroll
-      for (int w2 = 1; w2 < 4; w2++) { t.x += red[w2][threadIdx.x].x; t.y += red[w2][threadIdx.x].y; }
-      reinterpret_cast<float2 *>(dwp)[((size_t)c * kDwParts + part) * S + s0 + threadIdx.x] = t;
-    }
+    for (int i = 0; i < 8; i++)  // g e^{-j p}
+      ge[lane][warp + 8 * i] = {g[i].x * cs + g[i].y * sn, g[i].y * cs - g[i].x * sn};
+#pragma unroll
+    for (int i = 0; i < 2; i++) ha[lane][warp + 8 * i] = h[i];
     __syncthreads();
+#pragma unroll 8
+    for (int k = 0; k < 32; k++) {
+      const c2 x = ha[k][s];
+#pragma unroll
+      for (int j = 0; j < 4; j++) macc(acc[j], ge[k][cg + 16 * j], x);
+    }
   }
+  if (s0 + s < S)
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const int c = cg + 16 * j;
+      if (c < C)
+        reinterpret_cast<float2 *>(dwp)[((size_t)c * parts + part) * S + s0 + s] =
+            make_float2(acc[j].x, acc[j].y);
+    }
 }
 
 // out[c][j] = GU[c][k0 + j], j < n (complex), NaN after a run-out wait
@@ -823,19 +868,32 @@ __global__ void k_tc_copy_rows(const float *GU, int K, int k0, int n, int C, flo
   reinterpret_cast<float2 *>(out)[i] = v;
 }
 
-__global__ void k_tc_dw_sum(const float *GU, const float *dwp, int C, int S, int M, int K,
-                            float *grad_W, const unsigned *err) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= C * S) return;
-  const int c = i / S, s2 = i % S;
-  float2 t = __ldg(reinterpret_cast<const float2 *>(GU) + (size_t)c * K + M + s2);
-  for (int q = 0; q < kDwParts; q++) {
-    const float2 v = reinterpret_cast<const float2 *>(dwp)[((size_t)c * kDwParts + q) * S + s2];
-    t.x += v.x;
-    t.y += v.y;
+// 32 entries a CTA, its 8 warps share the slices
+__global__ void __launch_bounds__(256) k_tc_dw_sum(const float *GU, const float *dwp, int C, int S,
+                                                   int M, int K, int parts, float *grad_W,
+                                                   const unsigned *err) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int i = blockIdx.x * 32 + lane;
+  const bool in = i < C * S;
+  const int c = in ? i / S : 0, s2 = in ? i % S : 0;
+  c2 t = {0.f, 0.f};
+  if (in) {
+    if (wid == 0) t = ld2(GU, (size_t)c * K + M + s2);
+    for (int q = wid; q < parts; q += 8) {
+      const c2 v = ld2(dwp, ((size_t)c * parts + q) * S + s2);
+      t.x += v.x;
+      t.y += v.y;
+    }
   }
-  if (obj_failed(err)) t = make_float2(obj_nan(), obj_nan());
-  reinterpret_cast<float2 *>(grad_W)[i] = t;
+  __shared__ c2 red[8][32];
+  red[wid][lane] = t;
+  __syncthreads();
+  if (wid == 0 && in) {
+#pragma unroll
+    for (int w = 1; w < 8; w++) { t.x += red[w][lane].x; t.y += red[w][lane].y; }
+    if (obj_failed(err)) t = {obj_nan(), obj_nan()};
+    reinterpret_cast<float2 *>(grad_W)[i] = make_float2(t.x, t.y);
+  }
 }
 
 // Streaming paths, after the streaming kernel: one CTA per 32 rows k of
@@ -1946,12 +2004,6 @@ __global__ void __launch_bounds__(256)
 // below 2^-16 of it).  B_y and B_g are built once per channel set (a plan);
 // an evaluation rebuilds only the small A operands.
 
-namespace tcg {
-constexpr int BM = 128, BN = 128, BK = 64, STAGES = 3;
-constexpr uint32_t A_BYTES = BM * BK * 2, B_BYTES = BN * BK * 2;
-constexpr uint32_t STAGE_BYTES = 2 * A_BYTES + 2 * B_BYTES;
-constexpr size_t SMEM = STAGES * STAGE_BYTES + 1024;
-}  // namespace tcg
 
 
 // B_y [Rp, Kp] from [H_r; H_d] [K, R] complex: 32 x 32 complex tiles turned
@@ -1975,7 +2027,7 @@ __global__ void __launch_bounds__(256) k_tc_make_by(const float *Hr, const float
     const int r = r0 + i, k = k0 + threadIdx.x;
     if (r >= Rp || 2 * k >= Kp) continue;
     const float2 v = t[threadIdx.x][i];
-    put_pair(hi, lo, ((size_t)r * Kp + 2 * k) / 2, v.x, v.y);
+    put_pair(hi, lo, kb_pair(r, k, Rp), v.x, v.y);
   }
 }
 
@@ -1990,7 +2042,7 @@ __global__ void k_tc_make_bg(const float *Hr, const float *Hd, int M, int S, int
   if (k < M + S && r < R)
     v = __ldg(reinterpret_cast<const float2 *>(k < M ? Hr + (size_t)k * R * 2
                                                       : Hd + (size_t)(k - M) * R * 2) + r);
-  put_pair(hi, lo, (size_t)i, v.x, v.y);
+  put_pair(hi, lo, kb_pair(k, r, Np), v.x, v.y);
 }
 
 // A_y rows 2c, 2c+1 [., Kp] from coef[c, k] = U[c, k] (k < M), W[c, k - M]
@@ -2004,8 +2056,8 @@ __global__ void k_tc_make_ay(const float *U, const float *W, int C, int M, int S
   float2 v = make_float2(0.f, 0.f);
   if (k < M) v = reinterpret_cast<const float2 *>(U)[(size_t)c * M + k];
   else if (k < M + S) v = __ldg(reinterpret_cast<const float2 *>(W) + (size_t)c * S + (k - M));
-  put_pair(hi, lo, ((size_t)(2 * c) * Kp + 2 * k) / 2, v.x, -v.y);
-  put_pair(hi, lo, ((size_t)(2 * c + 1) * Kp + 2 * k) / 2, v.y, v.x);
+  put_pair(hi, lo, kb_pair(2 * c, k, tcg::BM), v.x, -v.y);
+  put_pair(hi, lo, kb_pair(2 * c + 1, k, tcg::BM), v.y, v.x);
 }
 
 // A_g rows 2c, 2c+1 [., K2p] from G = G1 + G2 / ||masked||; one thread per
@@ -2026,139 +2078,209 @@ __global__ void k_tc_make_ag(const float *G1, const float *G2, const float *scal
       g.y = fmaf(h.y, inv, g.y);
     }
   }
-  put_pair(hi, lo, ((size_t)(2 * c) * K2p + 2 * r) / 2, g.x, g.y);
-  put_pair(hi, lo, ((size_t)(2 * c + 1) * K2p + 2 * r) / 2, g.y, -g.x);
+  put_pair(hi, lo, kb_pair(2 * c, r, tcg::BM), g.x, g.y);
+  put_pair(hi, lo, kb_pair(2 * c + 1, r, tcg::BM), g.y, -g.x);
 }
 
-// D = sum over this CTA's k-blocks of A_hi B_hi^T + A_hi B_lo^T + A_lo B_hi^T
-// for a 128 x 128 tile, A [Mp, Kd] and B [Np, Kd] bf16 with K contiguous.
-// Warp 0 / lane 0 feeds a 3-stage TMA ring (four 16 KB tiles per stage),
-// warp 1 / lane 0 issues 12 tcgen05.mma per stage, all 4 warps drain TMEM.
-// Rows 2c / 2c+1 of D are stored as out[(z * C + c) * ldo + n] (complex) for
-// c < C and n < n_valid, z = blockIdx.z (the split of the k range).
-__global__ void __launch_bounds__(128, 1)
+// D = A_hi B_hi^T + A_hi B_lo^T + A_lo B_hi^T, A [128, Kd] and B [N, Kd] bf16 k-block by
+// k-block, in items of 128 x bn outputs over kper k-blocks.  Rows 2c /
+// 2c+1 of D are stored as out[(z * C + c) * ldo + n] (complex) for c < C and n <
+// n_valid, z the split of the k range.
+//
+// B is read once from HBM, and A comes along with every B tile from L2; the two
+// together bound the kernel.  So the two CTAs of a cluster work on neighbouring
+// B tiles and share A: rank 0 loads A_hi and rank 1 A_lo, each into both (1.44
+// bytes from L2 a byte of B at bn = 144 instead of 2).  A CTA stays for all its
+// items, with two accumulators: warps 2-5 drain one while warp 0 loads and warp
+// 1 multiplies the next, and bn is chosen so that the items fill whole rounds of
+// the chip (pick_split).
+//   60 codes, K = 1,040, R = 65,536: Y and the adjoint 123 us each with 128 x 128
+//   tiles, one a CTA; 103 and 100 us now, 5.5 TB/s of HBM (71 and 78%)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
     k_cgemm3(const __grid_constant__ CUtensorMap tah, const __grid_constant__ CUtensorMap tal,
              const __grid_constant__ CUtensorMap tbh, const __grid_constant__ CUtensorMap tbl,
-             int kb_per, int nkb, int C, int n_valid, long long ldo, float *out, unsigned *err) {
+             int bn, int pairs, int nitems, int kper, int nkb, int C, int n_valid, long long ldo,
+             float *out, unsigned *err) {
   using namespace tcg;
   extern __shared__ unsigned char smem_raw[];
   unsigned char *smem = reinterpret_cast<unsigned char *>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  __shared__ __align__(8) uint64_t full[STAGES], empty[STAGES], done;
+  __shared__ __align__(8) uint64_t full[STAGES_MAX], empty[STAGES_MAX], accf[2], acce[2];
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag, n_issued, n_used;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int n0 = blockIdx.x * BN, m0 = blockIdx.y * BM;
-  const int kb0 = blockIdx.z * kb_per;
-  const int nk = min(kb_per, nkb - kb0);  // >= 1: the host sizes the grid so
+  const int rank = blockIdx.x & 1, cluster = blockIdx.x >> 1, nclusters = gridDim.x >> 1;
+  const int nst = stages(bn);
+  const uint32_t sbytes = stage_bytes(bn), b_bytes = (uint32_t)bn * BK * 2;
+  // two accumulators of up to 256 columns, or one where each CTA has one item
+  const uint32_t tcols = nitems > nclusters ? 512u : 256u;
   if (tid == 0) {
-    for (int s = 0; s < STAGES; s++) { tc::mbar_init(&full[s], 1); tc::mbar_init(&empty[s], 1); }
-    tc::mbar_init(&done, 1);
+    // a stage is free when both CTAs' products have read it (A is in both)
+    for (int s = 0; s < nst; s++) { tc::mbar_init(&full[s], 1); tc::mbar_init(&empty[s], 2); }
+    for (int i = 0; i < 2; i++) { tc::mbar_init(&accf[i], 1); tc::mbar_init(&acce[i], 4); }
     abort_flag = 0;
     n_issued = 0;
     n_used = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 0) tc::tmem_alloc(&tmem_slot, (uint32_t)BN);
+  if (warp == 1) tc::tmem_alloc(&tmem_slot, tcols);
   tc::fence_before();
   __syncthreads();
   tc::fence_after();
   const uint32_t tmem = tmem_slot;
+  // both CTAs' barriers are set before either one's loads arrive
+  cluster_arrive();
+  cluster_wait();
 
   if (warp == 0 && lane == 0) {
-    int kb = 0;
-    for (; kb < nk; kb++) {
-      const int s = kb % STAGES;
-      if (kb >= STAGES && !tc::mbar_wait(&empty[s], ((kb / STAGES) - 1) & 1)) {
-        abort_flag = 1;
-        atomicOr(err, 1u);
-        break;
+    int it = 0;  // k-blocks issued
+    bool ok = true;
+    for (int i = cluster; ok && i < nitems; i += nclusters) {
+      const int z = i / pairs, n0 = (2 * (i - z * pairs) + rank) * bn;
+      const int k0 = z * kper, nk = min(kper, nkb - k0);
+      for (int kb = 0; kb < nk; kb++, it++) {
+        const int s = it % nst;
+        if (it >= nst && !tc::mbar_wait(&empty[s], (uint32_t)(it / nst - 1) & 1u)) {
+          atomicOr(err, 1u);
+          ok = false;
+        }
+        if (!ok || *(volatile int *)&abort_flag) { ok = false; break; }
+        unsigned char *sp = smem + (size_t)s * sbytes;
+        const int ya = (k0 + kb) * BM;
+        tc::mbar_expect_tx(&full[s], sbytes);
+        if (rank == 0) tc::tma_load_2d_multicast(sp, &tah, 0, ya, &full[s], 3);
+        else tc::tma_load_2d_multicast(sp + A_BYTES, &tal, 0, ya, &full[s], 3);
+        tc::tma_load_3d(sp + 2 * A_BYTES, &tbh, 0, n0, k0 + kb, &full[s]);
+        tc::tma_load_3d(sp + 2 * A_BYTES + b_bytes, &tbl, 0, n0, k0 + kb, &full[s]);
       }
-      if (*(volatile int *)&abort_flag) break;
-      unsigned char *sp = smem + s * STAGE_BYTES;
-      const int x = (kb0 + kb) * BK;
-      tc::mbar_expect_tx(&full[s], STAGE_BYTES);
-      tc::tma_load_2d(sp, &tah, x, m0, &full[s]);
-      tc::tma_load_2d(sp + A_BYTES, &tal, x, m0, &full[s]);
-      tc::tma_load_2d(sp + 2 * A_BYTES, &tbh, x, n0, &full[s]);
-      tc::tma_load_2d(sp + 2 * A_BYTES + B_BYTES, &tbl, x, n0, &full[s]);
     }
-    n_issued = kb;
+    n_issued = it;
+    if (!ok) *(volatile int *)&abort_flag = 1;
+    // the other CTA's last releases arrive here before this one may leave
+    for (int j = max(0, it - nst); ok && j < it; j++)
+      if (!tc::mbar_wait(&empty[j % nst], (uint32_t)(j / nst) & 1u)) { atomicOr(err, 1u); ok = false; }
   } else if (warp == 1 && lane == 0) {
-    constexpr uint32_t idesc = tc::idesc_bf16(BM, BN);
-    int kb = 0;
-    for (; kb < nk; kb++) {
-      const int s = kb % STAGES;
-      if (!tc::mbar_wait(&full[s], (kb / STAGES) & 1)) {
-        abort_flag = 1;
+    const uint32_t idesc = tc::idesc_bf16(BM, bn);
+    int it = 0, q = 0;
+    bool ok = true;
+    for (int i = cluster; ok && i < nitems; i += nclusters, q++) {
+      const int k0 = i / pairs * kper, nk = min(kper, nkb - k0);
+      const uint32_t acc = tmem + (uint32_t)(q & 1) * 256u;
+      // the accumulator's last item but one has been drained
+      if (q >= 2 && !tc::mbar_wait(&acce[q & 1], (uint32_t)(q / 2 - 1) & 1u)) {
         atomicOr(err, 2u);
+        ok = false;
         break;
       }
       tc::fence_after();
-      const uint32_t ah = tc::smem_u32(smem + s * STAGE_BYTES), al = ah + A_BYTES;
-      const uint32_t bh = ah + 2 * A_BYTES, bl = bh + B_BYTES;
+      for (int kb = 0; kb < nk; kb++, it++) {
+        const int s = it % nst;
+        if (!tc::mbar_wait(&full[s], (uint32_t)(it / nst) & 1u)) {
+          atomicOr(err, 2u);
+          ok = false;
+          break;
+        }
+        tc::fence_after();
+        const uint32_t ah = tc::smem_u32(smem + (size_t)s * sbytes), al = ah + A_BYTES;
+        const uint32_t bh = ah + 2 * A_BYTES, bl = bh + b_bytes;
 #pragma unroll
-      for (int kk = 0; kk < BK / 16; kk++) {
-        const uint32_t o = kk * 32;  // 16 bf16 = 32 bytes along K
-        tc::umma_bf16(tmem, tc::sdesc_sw128(ah + o), tc::sdesc_sw128(bh + o), idesc,
-                      (kb > 0 || kk > 0) ? 1u : 0u);
-        tc::umma_bf16(tmem, tc::sdesc_sw128(ah + o), tc::sdesc_sw128(bl + o), idesc, 1u);
-        tc::umma_bf16(tmem, tc::sdesc_sw128(al + o), tc::sdesc_sw128(bh + o), idesc, 1u);
+        for (int kk = 0; kk < BK / 16; kk++) {
+          const uint32_t o = kk * 32;  // 16 bf16 = 32 bytes along K
+          tc::umma_bf16(acc, tc::sdesc_sw128(ah + o), tc::sdesc_sw128(bh + o), idesc,
+                        (kb > 0 || kk > 0) ? 1u : 0u);
+          tc::umma_bf16(acc, tc::sdesc_sw128(ah + o), tc::sdesc_sw128(bl + o), idesc, 1u);
+          tc::umma_bf16(acc, tc::sdesc_sw128(al + o), tc::sdesc_sw128(bh + o), idesc, 1u);
+        }
+        tc::umma_commit_multicast(&empty[s], 3);
       }
-      tc::umma_commit(&empty[s]);
+      tc::umma_commit(&accf[q & 1]);
     }
-    n_used = kb;
-    tc::umma_commit(&done);
+    n_used = it;
+    if (!ok) *(volatile int *)&abort_flag = 1;
+  } else if (warp >= 2) {
+    const int quarter = warp & 3;  // the TMEM lanes a warp can read
+    const int c = quarter * 16 + (lane >> 1);
+    const bool odd = (lane & 1) != 0, rows = quarter * 32 < 2 * C;
+    int q = 0;
+    for (int i = cluster; i < nitems; i += nclusters, q++) {
+      const bool have = warp_wait(&accf[q & 1], (uint32_t)(q / 2) & 1u);
+      if (!have && lane == 0) { atomicOr(err, 4u); *(volatile int *)&abort_flag = 1; }
+      // warp-uniform: tcgen05.ld and the shuffles below are warp-collective
+      if (__any_sync(0xffffffffu, !have || *(volatile int *)&abort_flag)) break;
+      tc::fence_after();
+      const int z = i / pairs, n0 = (2 * (i - z * pairs) + rank) * bn;
+      const int n1 = min(n0 + bn, n_valid);
+      const uint32_t acc = tmem + (uint32_t)(q & 1) * 256u + ((uint32_t)(quarter * 32) << 16);
+      float2 *o2 = reinterpret_cast<float2 *>(out) + ((size_t)z * C + c) * (size_t)ldo;
+      if (rows)
+#pragma unroll 1
+        for (int c0 = 0; c0 < bn; c0 += 32) {
+          uint32_t r[32];
+          tc::tmem_ld32(acc + (uint32_t)c0, r);
+          // the even lane of a pair writes columns 0-15 of the chunk, the odd 16-31
+#pragma unroll
+          for (int j = 0; j < 16; j++) {
+            const float a0 = __uint_as_float(r[j]), a1 = __uint_as_float(r[16 + j]);
+            const float b0 = __shfl_xor_sync(0xffffffffu, a0, 1);
+            const float b1 = __shfl_xor_sync(0xffffffffu, a1, 1);
+            const int n = n0 + c0 + (odd ? 16 : 0) + j;
+            if (c < C && n < n1) o2[n] = odd ? make_float2(b1, a1) : make_float2(a0, b0);
+          }
+        }
+      tc::fence_before();
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(&acce[q & 1]);
+    }
   }
   __syncwarp();
-  const bool have = tc::mbar_wait(&done, 0);
-  if (!have && lane == 0) atomicOr(err, 4u);
-  // block-uniform: tcgen05.ld and the shuffles below are warp-collective
-  const bool drain = __syncthreads_and(have ? 1 : 0) && !abort_flag;
+  __syncthreads();
   // after an abort, the tiles issued but never consumed land before the CTA
   // exits (each stage holds at most one of them; bounded waits again)
   if (abort_flag && tid == 0)
-    for (int kb = n_used; kb < n_issued; kb++) tc::mbar_wait(&full[kb % STAGES], (kb / STAGES) & 1);
-  tc::fence_after();
-  if (drain) {
-    const int row = warp * 32 + lane;
-    const int c = (m0 + row) >> 1;
-    const bool odd = (lane & 1) != 0;
-    const uint32_t lane_base = (uint32_t)(warp * 32) << 16;
-    float2 *o2 = reinterpret_cast<float2 *>(out) + ((size_t)blockIdx.z * C + c) * (size_t)ldo;
-#pragma unroll 1
-    for (int c0 = 0; c0 < BN; c0 += 32) {
-      uint32_t r[32];
-      tc::tmem_ld32(tmem + lane_base + (uint32_t)c0, r);
-      // the even lane of a pair writes columns 0-15 of the chunk, the odd 16-31
-#pragma unroll
-      for (int j = 0; j < 16; j++) {
-        const float a0 = __uint_as_float(r[j]), a1 = __uint_as_float(r[16 + j]);
-        const float b0 = __shfl_xor_sync(0xffffffffu, a0, 1);
-        const float b1 = __shfl_xor_sync(0xffffffffu, a1, 1);
-        const int n = n0 + c0 + (odd ? 16 : 0) + j;
-        if (c < C && n < n_valid)
-          o2[n] = odd ? make_float2(b1, a1) : make_float2(a0, b0);
-      }
-    }
-  }
+    for (int j = n_used; j < n_issued; j++) tc::mbar_wait(&full[j % nst], (uint32_t)(j / nst) & 1u);
+  __syncwarp();
   tc::fence_before();
   __syncthreads();
-  if (warp == 0) {
+  if (warp == 1) {
     tc::fence_after();
-    tc::tmem_dealloc(tmem, (uint32_t)BN);
+    tc::tmem_dealloc(tmem, tcols);
   }
+  __syncwarp();
+  // no CTA leaves while the other's loads may still arrive in its memory
+  cluster_arrive();
+  cluster_wait();
 }
 
 int round_up(long long v, int m) { return (int)((v + m - 1) / m * m); }
 
-// split of a k range of nkb blocks so that the CTAs fill about one wave
-void pick_split(int ntiles, int nkb, int sms, int &ks, int &kper) {
-  // one CTA fits an SM (shared memory), so keep tiles x splits within a wave
-  int want = std::max(1, sms / ntiles);
-  want = std::min(want, nkb);
-  kper = (nkb + want - 1) / want;
-  ks = (nkb + kper - 1) / kper;
+// Items of a product of N columns and nkb k-blocks: the tile width bn and the
+// split of the k range whose rounds of CTA pairs over the chip take the least
+// time.  In units of a row of B (256 bytes a k-block) an item's k-block costs
+// its bn rows and about 48 for the shared A, 144 at least (its latency); every
+// split writes its partial sums, and the epilogues read them twice (48 bytes a
+// sum: with 16 or 24 the splits of small products cost up to 5% more).
+struct GemmSplit {
+  int bn = 0, pairs = 0, ks = 1, kper = 0;
+  int items() const { return pairs * ks; }
+};
+GemmSplit pick_split(int N, int nkb, int C, int sms) {
+  GemmSplit best;
+  double least = 0;
+  const int slots = std::max(1, sms / 2);
+  for (int bn = tcg::BN_MIN; bn <= tcg::BN_MAX; bn += 16)
+    for (int want = 1; want <= std::min(nkb, slots); want++) {
+      GemmSplit g;
+      g.bn = bn;
+      g.pairs = ((N + bn - 1) / bn + 1) / 2;
+      g.kper = (nkb + want - 1) / want;
+      g.ks = (nkb + g.kper - 1) / g.kper;
+      if (g.ks != want) continue;
+      const int rounds = (g.items() + slots - 1) / slots;
+      const double t = (double)rounds * g.kper * std::max(bn + 48, 144) + 2.0 * bn +
+                       (g.ks > 1 ? (double)g.ks * N * C * 48 / (256.0 * sms) : 0.0);
+      if (!best.bn || t < least) { best = g; least = t; }
+    }
+  return best;
 }
 
 }  // namespace
@@ -2249,7 +2371,7 @@ struct ObjTcPlan {
   int tKp = 0, tTR = 0, tKPT = 0, tStage = 0, tTiles = 0, tGrid = 0;
   size_t tSmem = 0, oPp = 0, oLp = 0, oGwS = 0;
   int S, M, R, Cmax, K, Kp, Rp, Np, K2p, Mp;
-  int ksy, kpy, ksg, kpg;
+  GemmSplit gy, gg;
   __nv_bfloat16 *by_hi, *by_lo, *bg_hi, *bg_lo, *ay_hi, *ay_lo, *ag_hi, *ag_lo;
   CUtensorMap m_byh, m_byl, m_bgh, m_bgl, m_ayh, m_ayl, m_agh, m_agl;
   char *mem;      // one allocation: operands then scratch
@@ -2412,8 +2534,8 @@ cudaError_t obj_tc_plan_create(const float *Hd, const float *Ha, const float *Hr
   p->S = S; p->M = M; p->R = R; p->Cmax = Cmax;
   p->K = M + S;
   p->Kp = round_up(2LL * p->K, 64);
-  p->Rp = round_up(R, tcg::BN);
-  p->Np = round_up(p->K, tcg::BN);
+  p->Rp = round_up(R, 32);
+  p->Np = p->K;
   p->K2p = round_up(2LL * R, 64);
   p->Mp = round_up(2LL * Cmax, tcg::BM);
   const int sms = sm_count();
@@ -2423,8 +2545,8 @@ cudaError_t obj_tc_plan_create(const float *Hd, const float *Ha, const float *Hr
   if (!force_tc && Cmax <= 2 && plan_direct(S, M, R, Cmax, Hd, Hr))
     return plan_direct_create(p, st, out);
   if (!force_tc && Cmax <= 2 && kpt <= (Cmax == 1 ? 16 : 8)) return plan_stream_create(p, st, out);
-  pick_split((p->Rp / tcg::BN) * (p->Mp / tcg::BM), p->Kp / tcg::BK, sms, p->ksy, p->kpy);
-  pick_split((p->Np / tcg::BN) * (p->Mp / tcg::BM), p->K2p / tcg::BK, sms, p->ksg, p->kpg);
+  p->gy = pick_split(R, p->Kp / tcg::BK, Cmax, sms);
+  p->gg = pick_split(p->K, p->K2p / tcg::BK, Cmax, sms);
   auto al = [](size_t v) { return (v + 255) & ~(size_t)255; };
   size_t o = 0;
   const size_t nby = (size_t)p->Rp * p->Kp, nbg = (size_t)p->Np * p->K2p;
@@ -2436,13 +2558,13 @@ cudaError_t obj_tc_plan_create(const float *Hd, const float *Ha, const float *Hr
   p->oCtl = o;
   o += kObjControlBytes;
   p->oU = o; o += al(8 * (size_t)Cmax * M);
-  p->oY = o; o += al(8 * (size_t)p->ksy * Cmax * R);
+  p->oY = o; o += al(8 * (size_t)p->gy.ks * Cmax * R);
   p->oG1 = o; o += al(8 * (size_t)Cmax * R);
   p->oG2 = o; o += al(8 * (size_t)Cmax * R);
   p->oPart = o; o += al(16 * (size_t)((R + 31) / 32));
-  p->oGU = o; o += al(8 * (size_t)p->ksg * Cmax * p->K);
+  p->oGU = o; o += al(8 * (size_t)p->gg.ks * Cmax * p->K);
   p->oGUs = o; o += al(8 * (size_t)Cmax * p->K);
-  p->oDw = o; o += al(8 * (size_t)Cmax * kDwParts * S);
+  p->oDw = o; o += al(8 * (size_t)Cmax * dw_parts(M) * S);
   p->bytes = o;
   cudaError_t e = cudaMalloc(&p->mem, o);
   if (e != cudaSuccess) { delete p; return e; }
@@ -2455,14 +2577,14 @@ cudaError_t obj_tc_plan_create(const float *Hd, const float *Ha, const float *Hr
   p->ag_hi = reinterpret_cast<__nv_bfloat16 *>(p->mem + oag);
   p->ag_lo = reinterpret_cast<__nv_bfloat16 *>(p->mem + oag + al(2 * nag));
   const bool ok =
-      tc::make_map_bf16(&p->m_byh, p->by_hi, p->Rp, p->Kp, tcg::BN) &&
-      tc::make_map_bf16(&p->m_byl, p->by_lo, p->Rp, p->Kp, tcg::BN) &&
-      tc::make_map_bf16(&p->m_bgh, p->bg_hi, p->Np, p->K2p, tcg::BN) &&
-      tc::make_map_bf16(&p->m_bgl, p->bg_lo, p->Np, p->K2p, tcg::BN) &&
-      tc::make_map_bf16(&p->m_ayh, p->ay_hi, p->Mp, p->Kp, tcg::BM) &&
-      tc::make_map_bf16(&p->m_ayl, p->ay_lo, p->Mp, p->Kp, tcg::BM) &&
-      tc::make_map_bf16(&p->m_agh, p->ag_hi, p->Mp, p->K2p, tcg::BM) &&
-      tc::make_map_bf16(&p->m_agl, p->ag_lo, p->Mp, p->K2p, tcg::BM);
+      tc::make_map_bf16_planes(&p->m_byh, p->by_hi, p->Kp / 64, p->Rp, p->gy.bn) &&
+      tc::make_map_bf16_planes(&p->m_byl, p->by_lo, p->Kp / 64, p->Rp, p->gy.bn) &&
+      tc::make_map_bf16_planes(&p->m_bgh, p->bg_hi, p->K2p / 64, p->Np, p->gg.bn) &&
+      tc::make_map_bf16_planes(&p->m_bgl, p->bg_lo, p->K2p / 64, p->Np, p->gg.bn) &&
+      tc::make_map_bf16(&p->m_ayh, p->ay_hi, (long long)p->Mp * (p->Kp / 64), 64, tcg::BM) &&
+      tc::make_map_bf16(&p->m_ayl, p->ay_lo, (long long)p->Mp * (p->Kp / 64), 64, tcg::BM) &&
+      tc::make_map_bf16(&p->m_agh, p->ag_hi, (long long)p->Mp * (p->K2p / 64), 64, tcg::BM) &&
+      tc::make_map_bf16(&p->m_agl, p->ag_lo, (long long)p->Mp * (p->K2p / 64), 64, tcg::BM);
   if (!ok) { cudaFree(p->mem); delete p; return cudaErrorInvalidValue; }
   static size_t attr[AMS_MAX_DEVICES] = {0};
   e = ams_set_smem_atleast(attr, k_cgemm3, tcg::SMEM);
@@ -2518,24 +2640,25 @@ cudaError_t run_tc(ObjTcPlan *p, const ObjArgs &a, char *ctl, cudaStream_t st) {
   const long long nay = (long long)C * (p->Kp / 2);
   k_tc_make_ay<<<(unsigned)((nay + 255) / 256), 256, 0, st>>>(U, a.W, C, M, p->S, p->Kp,
                                                               p->ay_hi, p->ay_lo);
-  dim3 gy(p->Rp / tcg::BN, p->Mp / tcg::BM, p->ksy);
-  k_cgemm3<<<gy, 128, tcg::SMEM, st>>>(p->m_ayh, p->m_ayl, p->m_byh, p->m_byl, p->kpy,
-                                        p->Kp / tcg::BK, C, R, R, Ypart, err);
+  const int slots = std::max(1, sm_count() / 2);
+  k_cgemm3<<<2 * std::min(p->gy.items(), slots), 192, tcg::SMEM, st>>>(
+      p->m_ayh, p->m_ayl, p->m_byh, p->m_byl, p->gy.bn, p->gy.pairs, p->gy.items(), p->gy.kper,
+      p->Kp / tcg::BK, C, R, R, Ypart, err);
   const bool need_g = a.grad_W || a.grad_phi || a.grad_U;
   if (CB >= 8) {
     constexpr int CW = CB >= 8 ? CB : 8;
     float *maxr = G1;  // G1 / G2 are not needed on this branch: per-Rx max and argmax
     int *argr = reinterpret_cast<int *>(G2 ? G2 : G1 + R);
     const int nb = (R + 31) / 32;
-    k_tc_epi_a<CW><<<nb, 256, 0, st>>>(a, p->ksy, Ypart, maxr, argr, part, counter, scal, err);
+    k_tc_epi_a<CW><<<nb, 256, 0, st>>>(a, p->gy.ks, Ypart, maxr, argr, part, counter, scal, err);
     if (need_g || a.grad_Y) {
       // with no gradient wanted the A operand is still written (harmless)
       const int nbb = std::max(nb, (p->K2p / 2 + 31) / 32);
-      k_tc_epi_b<CW><<<nbb, 256, 0, st>>>(a, p->ksy, Ypart, maxr, argr, scal, p->K2p, p->ag_hi,
+      k_tc_epi_b<CW><<<nbb, 256, 0, st>>>(a, p->gy.ks, Ypart, maxr, argr, scal, p->K2p, p->ag_hi,
                                           p->ag_lo);
     }
   } else {
-    k_epilogue<CB><<<(R + 127) / 128, 128, 0, st>>>(a, p->ksy, Ypart, G1, G2, part, counter,
+    k_epilogue<CB><<<(R + 127) / 128, 128, 0, st>>>(a, p->gy.ks, Ypart, G1, G2, part, counter,
                                                     scal, err);
     if (a.grad_Y) {
       const long long n = (long long)C * R;
@@ -2550,12 +2673,12 @@ cudaError_t run_tc(ObjTcPlan *p, const ObjArgs &a, char *ctl, cudaStream_t st) {
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   if (!need_g) return cudaGetLastError();
-  dim3 gg(p->Np / tcg::BN, p->Mp / tcg::BM, p->ksg);
-  k_cgemm3<<<gg, 128, tcg::SMEM, st>>>(p->m_agh, p->m_agl, p->m_bgh, p->m_bgl, p->kpg,
-                                        p->K2p / tcg::BK, C, p->K, p->K, GUp, err);
+  k_cgemm3<<<2 * std::min(p->gg.items(), slots), 192, tcg::SMEM, st>>>(
+      p->m_agh, p->m_agl, p->m_bgh, p->m_bgl, p->gg.bn, p->gg.pairs, p->gg.items(), p->gg.kper,
+      p->K2p / tcg::BK, C, p->K, p->K, GUp, err);
   float *GU = reinterpret_cast<float *>(p->mem + p->oGUs);
   const long long ngu = (long long)C * p->K;
-  k_gu_reduce<<<(unsigned)((ngu + 255) / 256), 256, 0, st>>>(GUp, p->ksg, ngu, GU);
+  k_gu_reduce<<<(unsigned)((ngu + 31) / 32), 256, 0, st>>>(GUp, p->gg.ks, ngu, GU);
   if (given) {
     // dL/dU is G_U's metasurface rows, dL/dW its H_d rows (poisoned like
     // the other outputs when a wait ran out)
@@ -2568,9 +2691,10 @@ cudaError_t run_tc(ObjTcPlan *p, const ObjArgs &a, char *ctl, cudaStream_t st) {
   if (a.grad_phi) k_tc_dphi<<<(M + 31) / 32, 256, 0, st>>>(GU, U, C, M, p->K, a.grad_phi, err);
   if (a.grad_W) {
     float *dwp = reinterpret_cast<float *>(p->mem + p->oDw);
-    k_tc_dw_part<<<dim3(C, kDwParts), 128, 0, st>>>(GU, p->Ha, a.phi, a.max_phase, p->S, M,
-                                                    p->K, dwp);
-    k_tc_dw_sum<<<(C * p->S + 127) / 128, 128, 0, st>>>(GU, dwp, C, p->S, M, p->K, a.grad_W,
+    const int parts = dw_parts(M);
+    k_tc_dw_part<<<dim3(parts, (p->S + 15) / 16), 256, 0, st>>>(GU, p->Ha, a.phi, a.max_phase, C,
+                                                                p->S, M, p->K, dwp);
+    k_tc_dw_sum<<<(C * p->S + 31) / 32, 256, 0, st>>>(GU, dwp, C, p->S, M, p->K, parts, a.grad_W,
                                                         err);
   }
   return cudaGetLastError();
