@@ -470,28 +470,36 @@ static_assert(stages(BN_MAX) >= 3 && BN_MAX % 16 == 0, "stages");
 template <int CPT>
 __device__ __forceinline__ void epi_load_y(const ObjArgs &a, int kspl, const float *Ypart, int wid,
                                            int rr, c2 (&y)[CPT]) {
-  for (int sp = 0; sp < kspl; sp++) {
-    c2 v[CPT];
+  const float2 *q = reinterpret_cast<const float2 *>(Ypart) + (size_t)wid * a.R + rr;
+  const size_t step = (size_t)8 * a.R;
+  for (int sp = 0; sp < kspl; sp++, q += (size_t)a.C * a.R) {
+    float2 v[CPT];
 #pragma unroll
     for (int j = 0; j < CPT; j++) {
-      const int c = min(wid + 8 * j, a.C - 1);
-      v[j] = ld2(Ypart, ((size_t)sp * a.C + c) * a.R + rr);
+      v[j] = make_float2(0.f, 0.f);
+      if (wid + 8 * j < a.C) v[j] = __ldg(q + j * step);
     }
 #pragma unroll
     for (int j = 0; j < CPT; j++) {
-      if (sp == 0) y[j] = v[j];
+      if (sp == 0) y[j] = {v[j].x, v[j].y};
       else { y[j].x += v[j].x; y[j].y += v[j].y; }
     }
   }
 }
+// 1 / N0 = 1e9 is a float32 value, which float32(1e-9) is not exactly: the
+// product is the nearer one, and a division is ten instructions
+constexpr float kInvN0 = 1e9f;
 __device__ __forceinline__ void epi_cap(const ObjArgs &a, int c, c2 y, float &amp, float &cap) {
   amp = sqrtf(y.x * y.x + y.y * y.y);
   const float aa = amp + kEps;
-  float v = log2f(1.0f + aa * aa / kN0);
+  float v = log2f(1.0f + aa * aa * kInvN0);
   if (a.drop && a.drop[c]) v = 0.f;
   cap = v;
 }
 
+// (Phase A takes groups of 32 Rx in turn and forms its loss partial once: with
+// a CTA and an arrival per group it waited at its barriers, 28.5 us for 60 codes
+// and R = 65,536 against 22.4.)
 template <int CB>
 __global__ void __launch_bounds__(256) k_tc_epi_a(ObjArgs a, int kspl, const float *Ypart,
                                                   float *maxr, int *argr, double *partials,
@@ -499,45 +507,55 @@ __global__ void __launch_bounds__(256) k_tc_epi_a(ObjArgs a, int kspl, const flo
                                                   const unsigned *err) {
   constexpr int CPT = CB / 8;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int r = blockIdx.x * 32 + lane;
-  const bool live = r < a.R;
-  c2 y[CPT];
-  float cap[CPT];
-  epi_load_y<CPT>(a, kspl, Ypart, wid, live ? r : 0, y);
-  float mx = -1.f;
-  int arg = 0x7fffffff;
+  __shared__ float smx[2][8][32];
+  __shared__ int sarg[2][8][32];
+  float sum_max = 0.f, sum_sq = 0.f;  // FP32 within a warp (FP64 is slow here), FP64 across
+  const int ngroups = (a.R + 31) / 32;
+  for (int grp = blockIdx.x, buf = 0; grp < ngroups; grp += gridDim.x, buf ^= 1) {
+    const int r = grp * 32 + lane;
+    const bool live = r < a.R;
+    c2 y[CPT];
+    float cap[CPT];
+    epi_load_y<CPT>(a, kspl, Ypart, wid, live ? r : 0, y);
+    float mx = -1.f;
+    int arg = 0x7fffffff;
 #pragma unroll
-  for (int j = 0; j < CPT; j++) {
-    const int c = wid + 8 * j;
-    cap[j] = 0.f;
-    if (!live || c >= a.C) continue;
-    float amp;
-    epi_cap(a, c, y[j], amp, cap[j]);
-    if (cap[j] > mx) { mx = cap[j]; arg = c; }
-    if (a.recv_amp) a.recv_amp[(size_t)c * a.R + r] = amp;
-  }
-  __shared__ float smx[8][32];
-  __shared__ int sarg[8][32];
-  smx[wid][lane] = mx;
-  sarg[wid][lane] = arg;
-  __syncthreads();
-  float M_ = smx[0][lane];
-  int A_ = sarg[0][lane];
+    for (int j = 0; j < CPT; j++) {
+      const int c = wid + 8 * j;
+      cap[j] = 0.f;
+      if (!live || c >= a.C) continue;
+      float amp;
+      epi_cap(a, c, y[j], amp, cap[j]);
+      if (cap[j] > mx) { mx = cap[j]; arg = c; }
+      if (a.recv_amp) a.recv_amp[(size_t)c * a.R + r] = amp;
+    }
+    // (the buffers alternate: a warp may write the next group's while others
+    // still read this one's)
+    smx[buf][wid][lane] = mx;
+    sarg[buf][wid][lane] = arg;
+    __syncthreads();
+    float M_ = smx[buf][0][lane];
+    int A_ = sarg[buf][0][lane];
 #pragma unroll
-  for (int w2 = 1; w2 < 8; w2++) {
-    const float v = smx[w2][lane];
-    const int g = sarg[w2][lane];
-    if (v > M_ || (v == M_ && g < A_)) { M_ = v; A_ = g; }
-  }
-  if (wid == 0 && live) { maxr[r] = M_; argr[r] = A_; }
-  // FP32 within a warp (FP64 arithmetic is slow here), FP64 across warps
-  float sum_max = (live && wid == 0) ? M_ : 0.f, sum_sq = 0.f;
+    for (int w2 = 1; w2 < 8; w2++) {
+      const float v = smx[buf][w2][lane];
+      const int g = sarg[buf][w2][lane];
+      if (v > M_ || (v == M_ && g < A_)) { M_ = v; A_ = g; }
+    }
+    if (wid == 0 && live) {
+      maxr[r] = M_;
+      argr[r] = A_;
+      sum_max += M_;
+    }
+    float sq = 0.f;
 #pragma unroll
-  for (int j = 0; j < CPT; j++) {
-    const int c = wid + 8 * j;
-    if (!live || c >= a.C) continue;
-    const float msk = (cap[j] != M_) ? cap[j] : 0.f;
-    sum_sq += msk * msk;
+    for (int j = 0; j < CPT; j++) {
+      const int c = wid + 8 * j;
+      if (!live || c >= a.C) continue;
+      const float msk = (cap[j] != M_) ? cap[j] : 0.f;
+      sq += msk * msk;
+    }
+    sum_sq += sq;
   }
   for (int o = 16; o > 0; o >>= 1) {
     sum_max += __shfl_xor_sync(0xffffffffu, sum_max, o);
@@ -593,7 +611,7 @@ __global__ void __launch_bounds__(256) k_tc_epi_b(ObjArgs a, int kspl, const flo
       const bool dropped = a.drop && a.drop[c];
       const float msk = (cap != M_) ? cap : 0.f;
       const float aa = amp + kEps;
-      const float dcap = (2.0f * aa / kN0) / (1.0f + aa * aa / kN0) * kInvLn2;
+      const float dcap = (2.0f * aa * kInvN0) / (1.0f + aa * aa * kInvN0) * kInvLn2;
       float g1 = (c == A_) ? -a.w : 0.f, g2 = msk;
       if (dropped) { g1 = 0.f; g2 = 0.f; }
       const float sc = amp > 0.f ? dcap / amp : 0.f;
@@ -605,8 +623,17 @@ __global__ void __launch_bounds__(256) k_tc_epi_b(ObjArgs a, int kspl, const flo
       if (a.grad_Y) reinterpret_cast<float2 *>(a.grad_Y)[(size_t)c * a.R + r] = make_float2(g.x, g.y);
     }
     if (r < K2p / 2) {
-      put_pair(hi, lo, kb_pair(2 * c, r, tcg::BM), g.x, g.y);
-      put_pair(hi, lo, kb_pair(2 * c + 1, r, tcg::BM), g.y, -g.x);
+      // rows (g.x, g.y) and (g.y, -g.x); the split of -x is that of x negated
+      __nv_bfloat16 hx, lx, hy, ly;
+      split_bf16(g.x, hx, lx);
+      split_bf16(g.y, hy, ly);
+      const size_t at = kb_pair(2 * c, r, tcg::BM);
+      __nv_bfloat162 *h2 = reinterpret_cast<__nv_bfloat162 *>(hi) + at;
+      __nv_bfloat162 *l2 = reinterpret_cast<__nv_bfloat162 *>(lo) + at;
+      h2[0] = __halves2bfloat162(hx, hy);
+      l2[0] = __halves2bfloat162(lx, ly);
+      h2[32] = __halves2bfloat162(hy, __hneg(hx));
+      l2[32] = __halves2bfloat162(ly, __hneg(lx));
     }
   }
 }
@@ -2650,7 +2677,7 @@ cudaError_t run_tc(ObjTcPlan *p, const ObjArgs &a, char *ctl, cudaStream_t st) {
     float *maxr = G1;  // G1 / G2 are not needed on this branch: per-Rx max and argmax
     int *argr = reinterpret_cast<int *>(G2 ? G2 : G1 + R);
     const int nb = (R + 31) / 32;
-    k_tc_epi_a<CW><<<nb, 256, 0, st>>>(a, p->gy.ks, Ypart, maxr, argr, part, counter, scal, err);
+    k_tc_epi_a<CW><<<std::min(nb, 4 * sm_count()), 256, 0, st>>>(a, p->gy.ks, Ypart, maxr, argr, part, counter, scal, err);
     if (need_g || a.grad_Y) {
       // with no gradient wanted the A operand is still written (harmless)
       const int nbb = std::max(nb, (p->K2p / 2 + 31) / 32);
