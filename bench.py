@@ -334,7 +334,7 @@ def objective_bench(torch, steps, flush, cpu_baseline=False):
                             "max_rel_loss_diff": rel},
             "rel_err_vs_fp64": err,
             "cpu_baseline": cpu,
-            "roofline": {"bound": "hbm", "kernel": "k_obj_stream_t", "achieved": achieved,
+            "roofline": {"bound": "hbm", "kernel": "k_obj_stream", "achieved": achieved,
                          "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
                          "traffic": profile_value("k_obj_stream_c1_traffic.md",
                                                   "traffic_bytes_per_launch"),
@@ -417,11 +417,9 @@ def objective_codes_bench(torch, R=4096, C=60, nset=4, reps=20):
     rel = float(((loss_tc - loss).abs() / loss.abs()).max())
     K = M + S
     Kp = -(-2 * K // 64) * 64
-    Rp = -(-R // 128) * 128
-    Np = -(-K // 128) * 128
     K2p = -(-2 * R // 64) * 64
-    op_bytes = 4 * (Rp * Kp + Np * K2p)                 # B_y and B_g, hi + lo
-    mma_flop = 3 * 2 * 128 * (Kp * Rp + K2p * Np)        # executed on the tensor pipe
+    op_bytes = 4 * (R * Kp + K * K2p)                   # B_y and B_g, hi + lo
+    mma_flop = 3 * 2 * 128 * (Kp * R + K2p * K)          # on the tensor pipe, no padding
     alg_flop = 16 * C * K * R                            # complex fwd + adjoint
     hbm, kind = peaks()
     bf16 = 1913.2
