@@ -2115,18 +2115,17 @@ __global__ void k_tc_make_ag(const float *G1, const float *G2, const float *scal
 // n_valid, z the split of the k range.
 //
 // B is read once from HBM, and A comes along with every B tile from L2; the two
-// together bound the kernel.  So the two CTAs of a cluster work on neighbouring
-// B tiles and share A: rank 0 loads A_hi and rank 1 A_lo, each into both (1.44
-// bytes from L2 a byte of B at bn = 144 instead of 2).  A CTA stays for all its
-// items, with two accumulators: warps 2-5 drain one while warp 0 loads and warp
-// 1 multiplies the next, and bn is chosen so that the items fill whole rounds of
-// the chip (pick_split).
-//   60 codes, K = 1,040, R = 65,536: Y and the adjoint 123 us each with 128 x 128
-//   tiles, one a CTA; 103 and 100 us now, 5.5 TB/s of HBM (71 and 78%)
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
+// together bound the kernel.  A CTA stays for all its items, with two
+// accumulators: warps 2-5 drain one while warp 0 loads and warp 1 multiplies the
+// next, and bn is chosen so that the items fill whole rounds of the chip
+// (pick_split).
+// 60 codes, K = 1,040, R = 65,536: Y and the adjoint 124 us each with 128 x 128
+// tiles, one a CTA; 101 and 107 us now.  (Two CTAs of a cluster that shared A by
+// multicast loads took 102 and 108 us.)
+__global__ void __launch_bounds__(192, 1)
     k_cgemm3(const __grid_constant__ CUtensorMap tah, const __grid_constant__ CUtensorMap tal,
              const __grid_constant__ CUtensorMap tbh, const __grid_constant__ CUtensorMap tbl,
-             int bn, int pairs, int nitems, int kper, int nkb, int C, int n_valid, long long ldo,
+             int bn, int tiles, int nitems, int kper, int nkb, int C, int n_valid, long long ldo,
              float *out, unsigned *err) {
   using namespace tcg;
   extern __shared__ unsigned char smem_raw[];
@@ -2136,14 +2135,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag, n_issued, n_used;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int rank = blockIdx.x & 1, cluster = blockIdx.x >> 1, nclusters = gridDim.x >> 1;
+  const int first = blockIdx.x, step = gridDim.x;
   const int nst = stages(bn);
   const uint32_t sbytes = stage_bytes(bn), b_bytes = (uint32_t)bn * BK * 2;
   // two accumulators of up to 256 columns, or one where each CTA has one item
-  const uint32_t tcols = nitems > nclusters ? 512u : 256u;
+  const uint32_t tcols = nitems > step ? 512u : 256u;
   if (tid == 0) {
-    // a stage is free when both CTAs' products have read it (A is in both)
-    for (int s = 0; s < nst; s++) { tc::mbar_init(&full[s], 1); tc::mbar_init(&empty[s], 2); }
+    for (int s = 0; s < nst; s++) { tc::mbar_init(&full[s], 1); tc::mbar_init(&empty[s], 1); }
     for (int i = 0; i < 2; i++) { tc::mbar_init(&accf[i], 1); tc::mbar_init(&acce[i], 4); }
     abort_flag = 0;
     n_issued = 0;
@@ -2155,15 +2153,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
   __syncthreads();
   tc::fence_after();
   const uint32_t tmem = tmem_slot;
-  // both CTAs' barriers are set before either one's loads arrive
-  cluster_arrive();
-  cluster_wait();
 
   if (warp == 0 && lane == 0) {
     int it = 0;  // k-blocks issued
     bool ok = true;
-    for (int i = cluster; ok && i < nitems; i += nclusters) {
-      const int z = i / pairs, n0 = (2 * (i - z * pairs) + rank) * bn;
+    for (int i = first; ok && i < nitems; i += step) {
+      const int z = i / tiles, n0 = (i - z * tiles) * bn;
       const int k0 = z * kper, nk = min(kper, nkb - k0);
       for (int kb = 0; kb < nk; kb++, it++) {
         const int s = it % nst;
@@ -2175,23 +2170,23 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
         unsigned char *sp = smem + (size_t)s * sbytes;
         const int ya = (k0 + kb) * BM;
         tc::mbar_expect_tx(&full[s], sbytes);
-        if (rank == 0) tc::tma_load_2d_multicast(sp, &tah, 0, ya, &full[s], 3);
-        else tc::tma_load_2d_multicast(sp + A_BYTES, &tal, 0, ya, &full[s], 3);
+        tc::tma_load_2d(sp, &tah, 0, ya, &full[s]);
+        tc::tma_load_2d(sp + A_BYTES, &tal, 0, ya, &full[s]);
         tc::tma_load_3d(sp + 2 * A_BYTES, &tbh, 0, n0, k0 + kb, &full[s]);
         tc::tma_load_3d(sp + 2 * A_BYTES + b_bytes, &tbl, 0, n0, k0 + kb, &full[s]);
       }
     }
     n_issued = it;
     if (!ok) *(volatile int *)&abort_flag = 1;
-    // the other CTA's last releases arrive here before this one may leave
+    // the last releases arrive before the CTA may leave
     for (int j = max(0, it - nst); ok && j < it; j++)
       if (!tc::mbar_wait(&empty[j % nst], (uint32_t)(j / nst) & 1u)) { atomicOr(err, 1u); ok = false; }
   } else if (warp == 1 && lane == 0) {
     const uint32_t idesc = tc::idesc_bf16(BM, bn);
     int it = 0, q = 0;
     bool ok = true;
-    for (int i = cluster; ok && i < nitems; i += nclusters, q++) {
-      const int k0 = i / pairs * kper, nk = min(kper, nkb - k0);
+    for (int i = first; ok && i < nitems; i += step, q++) {
+      const int k0 = i / tiles * kper, nk = min(kper, nkb - k0);
       const uint32_t acc = tmem + (uint32_t)(q & 1) * 256u;
       // the accumulator's last item but one has been drained
       if (q >= 2 && !tc::mbar_wait(&acce[q & 1], (uint32_t)(q / 2 - 1) & 1u)) {
@@ -2218,7 +2213,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
           tc::umma_bf16(acc, tc::sdesc_sw128(ah + o), tc::sdesc_sw128(bl + o), idesc, 1u);
           tc::umma_bf16(acc, tc::sdesc_sw128(al + o), tc::sdesc_sw128(bh + o), idesc, 1u);
         }
-        tc::umma_commit_multicast(&empty[s], 3);
+        tc::umma_commit(&empty[s]);
       }
       tc::umma_commit(&accf[q & 1]);
     }
@@ -2229,13 +2224,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
     const int c = quarter * 16 + (lane >> 1);
     const bool odd = (lane & 1) != 0, rows = quarter * 32 < 2 * C;
     int q = 0;
-    for (int i = cluster; i < nitems; i += nclusters, q++) {
+    for (int i = first; i < nitems; i += step, q++) {
       const bool have = warp_wait(&accf[q & 1], (uint32_t)(q / 2) & 1u);
       if (!have && lane == 0) { atomicOr(err, 4u); *(volatile int *)&abort_flag = 1; }
       // warp-uniform: tcgen05.ld and the shuffles below are warp-collective
       if (__any_sync(0xffffffffu, !have || *(volatile int *)&abort_flag)) break;
       tc::fence_after();
-      const int z = i / pairs, n0 = (2 * (i - z * pairs) + rank) * bn;
+      const int z = i / tiles, n0 = (i - z * tiles) * bn;
       const int n1 = min(n0 + bn, n_valid);
       const uint32_t acc = tmem + (uint32_t)(q & 1) * 256u + ((uint32_t)(quarter * 32) << 16);
       float2 *o2 = reinterpret_cast<float2 *>(out) + ((size_t)z * C + c) * (size_t)ldo;
@@ -2272,33 +2267,30 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
     tc::fence_after();
     tc::tmem_dealloc(tmem, tcols);
   }
-  __syncwarp();
-  // no CTA leaves while the other's loads may still arrive in its memory
-  cluster_arrive();
-  cluster_wait();
 }
 
 int round_up(long long v, int m) { return (int)((v + m - 1) / m * m); }
 
 // Items of a product of N columns and nkb k-blocks: the tile width bn and the
-// split of the k range whose rounds of CTA pairs over the chip take the least
-// time.  In units of a row of B (256 bytes a k-block) an item's k-block costs
-// its bn rows and about 48 for the shared A, 144 at least (its latency); every
+// split of the k range whose rounds over the chip take the least time.  In units
+// of a row of B (256 bytes a k-block) an item's k-block costs its bn rows and
+// about 48 for A (32, 64, 96 and 128 within 2% or slower), 144 at least (its
+// latency); every
 // split writes its partial sums, and the epilogues read them twice (48 bytes a
 // sum: with 16 or 24 the splits of small products cost up to 5% more).
 struct GemmSplit {
-  int bn = 0, pairs = 0, ks = 1, kper = 0;
-  int items() const { return pairs * ks; }
+  int bn = 0, tiles = 0, ks = 1, kper = 0;
+  int items() const { return tiles * ks; }
 };
 GemmSplit pick_split(int N, int nkb, int C, int sms) {
   GemmSplit best;
   double least = 0;
-  const int slots = std::max(1, sms / 2);
+  const int slots = std::max(1, sms);
   for (int bn = tcg::BN_MIN; bn <= tcg::BN_MAX; bn += 16)
     for (int want = 1; want <= std::min(nkb, slots); want++) {
       GemmSplit g;
       g.bn = bn;
-      g.pairs = ((N + bn - 1) / bn + 1) / 2;
+      g.tiles = (N + bn - 1) / bn;
       g.kper = (nkb + want - 1) / want;
       g.ks = (nkb + g.kper - 1) / g.kper;
       if (g.ks != want) continue;
@@ -2667,9 +2659,9 @@ cudaError_t run_tc(ObjTcPlan *p, const ObjArgs &a, char *ctl, cudaStream_t st) {
   const long long nay = (long long)C * (p->Kp / 2);
   k_tc_make_ay<<<(unsigned)((nay + 255) / 256), 256, 0, st>>>(U, a.W, C, M, p->S, p->Kp,
                                                               p->ay_hi, p->ay_lo);
-  const int slots = std::max(1, sm_count() / 2);
-  k_cgemm3<<<2 * std::min(p->gy.items(), slots), 192, tcg::SMEM, st>>>(
-      p->m_ayh, p->m_ayl, p->m_byh, p->m_byl, p->gy.bn, p->gy.pairs, p->gy.items(), p->gy.kper,
+  const int slots = std::max(1, sm_count());
+  k_cgemm3<<<std::min(p->gy.items(), slots), 192, tcg::SMEM, st>>>(
+      p->m_ayh, p->m_ayl, p->m_byh, p->m_byl, p->gy.bn, p->gy.tiles, p->gy.items(), p->gy.kper,
       p->Kp / tcg::BK, C, R, R, Ypart, err);
   const bool need_g = a.grad_W || a.grad_phi || a.grad_U;
   if (CB >= 8) {
@@ -2700,8 +2692,8 @@ cudaError_t run_tc(ObjTcPlan *p, const ObjArgs &a, char *ctl, cudaStream_t st) {
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   if (!need_g) return cudaGetLastError();
-  k_cgemm3<<<2 * std::min(p->gg.items(), slots), 192, tcg::SMEM, st>>>(
-      p->m_agh, p->m_agl, p->m_bgh, p->m_bgl, p->gg.bn, p->gg.pairs, p->gg.items(), p->gg.kper,
+  k_cgemm3<<<std::min(p->gg.items(), slots), 192, tcg::SMEM, st>>>(
+      p->m_agh, p->m_agl, p->m_bgh, p->m_bgl, p->gg.bn, p->gg.tiles, p->gg.items(), p->gg.kper,
       p->K2p / tcg::BK, C, p->K, p->K, GUp, err);
   float *GU = reinterpret_cast<float *>(p->mem + p->oGUs);
   const long long ngu = (long long)C * p->K;
