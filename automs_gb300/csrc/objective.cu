@@ -1799,8 +1799,8 @@ cudaError_t stream_tail(const ObjArgs &a, int M, int nparts, const float *U, con
 
 // ------------------------------------------------------------------
 // Streaming path on a plan's transposed copy HT [Rp][Kp] of [H_r; H_d]
-// (row r = column r over all k), for an odd number of Rx, unaligned channels
-// and K beyond k_obj_stream's: a tile of TR Rx is one contiguous block of
+// (row r = column r over all k), for an odd number of Rx and K beyond
+// k_obj_stream's: a tile of TR Rx is one contiguous block of
 // TR * Kp * 8 bytes, fetched by a single cp.async.bulk.  A CTA has all rows of
 // its tile, takes the phases A, B, C one after the other and writes its own
 // partials; in (A) warp w takes column w % TR and every (NW / TR)-th run of 32
@@ -2383,8 +2383,8 @@ cudaError_t obj_run(const ObjArgs &a0, char *scratch, cudaStream_t st) {
 // ------------------------------------------------------------------ plans
 struct ObjTcPlan {
   const float *Hd, *Ha, *Hr;
-  // stream mode (C_max <= 2): the streaming kernels, over the channels
-  // themselves (direct) or a transposed FP32 copy
+  // stream mode (C_max <= 2): the streaming kernels, over an FP32 copy of the
+  // channels, as they are (direct) or transposed
   bool stream = false, direct = false;
   float *HT = nullptr;
   int tKp = 0, tTR = 0, tKPT = 0, tStage = 0, tTiles = 0, tGrid = 0;
@@ -2399,13 +2399,13 @@ struct ObjTcPlan {
 };
 
 namespace {
-// Stream mode over the channels themselves, where k_obj_stream takes them: an
-// even number of Rx, 16-byte aligned arrays, K up to about 3,200.  The
-// transposed copy is no faster there (S = 16, C = 1: R = 65,536, M = 1,024 133
-// against 127 us, M = 2,304 266 against 253 us; R = 4,096, M = 1,024 23.8
-// against 21.6 us), and a plan without it costs nothing to make.
-bool plan_direct(int S, int M, int R, int Cmax, const float *Hd, const float *Hr) {
-  if ((reinterpret_cast<uintptr_t>(Hd) | reinterpret_cast<uintptr_t>(Hr)) & 15) return false;
+// Stream mode over the channels as they are, where k_obj_stream takes them: an
+// even number of Rx, K up to about 3,200.  A transposed copy is no faster there
+// (S = 16, C = 1: R = 65,536, M = 1,024 133 against 127 us, M = 2,304 266
+// against 253 us; R = 4,096, M = 1,024 23.8 against 21.6 us).  Like every other
+// plan this one evaluates the H_d and H_r that it was made of, whatever is
+// written into the caller's arrays later, so it keeps a copy of them.
+bool plan_direct(int S, int M, int R, int Cmax) {
   for (int C = 1; C <= Cmax; C++)
     if (!stream_plan(S, M, R, C, false).ok) return false;
   return true;
@@ -2413,7 +2413,10 @@ bool plan_direct(int S, int M, int R, int Cmax, const float *Hd, const float *Hr
 cudaError_t plan_direct_create(ObjTcPlan *p, cudaStream_t st, ObjTcPlan **out) {
   auto al = [](size_t v) { return (v + 255) & ~(size_t)255; };
   const int nparts = std::min(kMaxClusters, (p->R + 7) / 8);
+  const size_t n_hr = 8 * (size_t)p->M * p->R, n_hd = 8 * (size_t)p->S * p->R;
   size_t o = 0;
+  const size_t ohr = o; o += al(n_hr);
+  const size_t ohd = o; o += al(n_hd);
   p->oCtl = o; o += kObjControlBytes;
   p->oU = o; o += al(8 * (size_t)p->Cmax * p->M);
   p->oPp = o; o += al(8 * (size_t)nparts * 2 * p->Cmax * p->K);
@@ -2425,7 +2428,13 @@ cudaError_t plan_direct_create(ObjTcPlan *p, cudaStream_t st, ObjTcPlan **out) {
   if (e != cudaSuccess) { delete p; return e; }
   p->stream = p->direct = true;
   e = cudaMemsetAsync(p->mem + p->oCtl, 0, kObjControlBytes, st);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(p->mem + ohr, p->Hr, n_hr, cudaMemcpyDeviceToDevice, st);
+  if (e == cudaSuccess)
+    e = cudaMemcpyAsync(p->mem + ohd, p->Hd, n_hd, cudaMemcpyDeviceToDevice, st);
   if (e != cudaSuccess) { cudaFree(p->mem); delete p; return e; }
+  p->Hr = reinterpret_cast<const float *>(p->mem + ohr);
+  p->Hd = reinterpret_cast<const float *>(p->mem + ohd);
   *out = p;
   return cudaSuccess;
 }
@@ -2561,7 +2570,7 @@ cudaError_t obj_tc_plan_create(const float *Hd, const float *Ha, const float *Hr
   // stream mode when the streaming kernel's per-thread rows cover K (16 rows
   // a thread for one code, 8 for two); otherwise the tensor-core mode
   const int kpt = (p->K + 255) / 256;
-  if (!force_tc && Cmax <= 2 && plan_direct(S, M, R, Cmax, Hd, Hr))
+  if (!force_tc && Cmax <= 2 && plan_direct(S, M, R, Cmax))
     return plan_direct_create(p, st, out);
   if (!force_tc && Cmax <= 2 && kpt <= (Cmax == 1 ? 16 : 8)) return plan_stream_create(p, st, out);
   p->gy = pick_split(R, p->Kp / tcg::BK, Cmax, sms);

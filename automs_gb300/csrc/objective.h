@@ -50,8 +50,9 @@ cudaError_t obj_noalloc_scratch(char **out);
 // Evaluation plan for a fixed channel set with a metasurface hop.  Cmax > 2:
 // tensor cores (tcgen05, 3xBF16 split precision); the plan holds BF16 hi/lo
 // copies of [H_r; H_d] in the two layouts the forward and adjoint GEMMs read.
-// Cmax <= 2: streaming kernels over the channels or a transposed FP32 copy
-// [R][M+S] (grad_Y is not produced).  The plan owns its scratch.  H_d, H_a and H_r must stay valid while the plan is used;
+// Cmax <= 2: streaming kernels over an FP32 copy of the channels, as they are or
+// transposed to [R][M+S] (grad_Y is not produced).  The plan owns its scratch and
+// its copies of H_d and H_r; H_a must stay valid while the plan is used;
 // evaluations on one plan must not overlap.  1 <= C <= Cmax <= 64.
 struct ObjTcPlan;
 cudaError_t obj_tc_plan_create(const float *Hd, const float *Ha, const float *Hr, int S, int M,

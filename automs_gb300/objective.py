@@ -45,12 +45,17 @@ def _drop(drop, device):
 
 
 class ObjectivePlan:
-    """Tensor-core objective for a fixed channel set (ams_objective_plan_*).
+    """Objective for a fixed channel set (ams_objective_plan_*), evaluated many
+    times as in optimize_model; C up to c_max <= 64.
 
-    [H_r; H_d] are converted once into BF16 hi/lo pairs; each evaluation then
-    runs the forward and adjoint contractions as tcgen05 GEMMs (3xBF16
-    products, FP32 accumulation, relative error about 1e-5).  For codebooks
-    (C up to c_max <= 64) evaluated many times, as in optimize_model."""
+    c_max > 2: [H_r; H_d] are converted once into BF16 hi/lo pairs; each
+    evaluation then runs the forward and adjoint contractions as tcgen05 GEMMs
+    (3xBF16 products, FP32 accumulation, relative error about 1e-5).
+    c_max <= 2: the FP32 streaming kernels over a copy of them (long columns,
+    M + S beyond 4096 for one code or 2048 for two, may take the first form).
+
+    The plan holds its own copy of H_d and H_r: what is written into them later
+    does not show.  H_a is read by every evaluation."""
 
     def __init__(self, H_d, H_a, H_r, c_max=64):
         lib()

@@ -219,16 +219,16 @@ ams_status ams_objective_fwd_bwd_noalloc(
  * channels are fixed.  With C_max > 2 it is the tensor-core path.  The plan converts [H_r; H_d] once into BF16 hi/lo
  * pairs (x = hi + lo, 3xBF16 products with FP32 accumulation, relative
  * error about 1e-5) in the two layouts of the forward and adjoint GEMMs
- * (tcgen05 tensor cores).  H_d, H_a, H_r must stay valid and unchanged while
- * the plan lives.  ams_objective_plan_fwd_bwd has the arguments and results
+ * (tcgen05 tensor cores).  Every plan holds a copy of H_d and H_r, which may be
+ * written or freed once the creation's work on `stream` is done; H_a is read by
+ * each evaluation and must stay valid while the plan lives.  ams_objective_plan_fwd_bwd has the arguments and results
  * of ams_objective_fwd_bwd (the channels come from the plan); calls on one
  * plan must not overlap.  The plan owns about 8 (R (M+S) + (M+S) R) bytes of
  * device memory (ams_objective_plan_bytes).  A plan made with C_max <= 2
  * (and M+S <= 4096 for one code, 2048 for two) instead runs the single-pass
- * streaming kernels in FP32, over the channels themselves or, for an odd R,
- * channels that are not 16-byte aligned or large M+S, over a copy of
- * [H_r; H_d] transposed to [R][M+S]; it does not produce grad_Y
- * (AMS_ERR_ARG). */
+ * streaming kernels in FP32 over one copy of [H_r; H_d] (8 R (M+S) bytes), as
+ * they are or, for an odd R or large M+S, transposed to [R][M+S]; it does not
+ * produce grad_Y (AMS_ERR_ARG). */
 typedef struct ams_objective_plan ams_objective_plan;
 ams_status ams_objective_plan_create(const float *H_d, const float *H_a,
                                      const float *H_r, int S, int M, int R,
