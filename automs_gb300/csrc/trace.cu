@@ -961,10 +961,11 @@ __global__ void __launch_bounds__(256) k_rx_grid(const float *dst, const float *
     return;
   __threadfence();
   for (int k = 0; k < 6; k++) m[k] = __ldcg(out + k);
-  // (NaN compares false)
-  const bool ok = g.ok && (n0 == 1 || m[0] <= 0.25f * fabsf(du)) &&
-                  (n1 == 1 || m[1] <= 0.25f * fabsf(dv)) && m[2] <= m[5] && m[3] < 1e6f &&
-                  m[4] < 1e6f && m[5] < 1e6f;
+  // (NaN compares false; without a step the rows lie on one another, and a ray
+  // may meet any of them first)
+  const bool ok = g.ok && (n0 == 1 || (du != 0.0f && m[0] <= 0.25f * fabsf(du))) &&
+                  (n1 == 1 || (dv != 0.0f && m[1] <= 0.25f * fabsf(dv))) && m[2] <= m[5] &&
+                  m[3] < 1e6f && m[4] < 1e6f && m[5] < 1e6f;
   reinterpret_cast<int *>(out)[7] = ok ? 1 : 0;
 }
 __device__ __forceinline__ RxGrid rx_grid(const TraceDev &P) {
