@@ -87,6 +87,7 @@ SIGNATURES = {
                                             _P, _P, _P, _P, _P, _E, _S]),
     "ams_cgemm": (_I, [_I, _I, _I, _P, _I, _I, _P, _I, _I, _P, _I, _I, _P, _E, _S]),
     "ams_debug_inject_wait_timeout": (None, [_I]),
+    "ams_debug_refuse_allocations": (None, [C.c_ulonglong]),
     "ams_coverage_db": (_I, [_P, _I, _I, _F, _F, _P, _P, _E, _S]),
     "ams_scratch_bytes": (C.c_ulonglong, []),
     "ams_gemm_bf16": (_I, [_P, _P, _I, _I, _I, _P, _I, _P, _P, _P, _E, _S]),

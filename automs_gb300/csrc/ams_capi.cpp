@@ -66,7 +66,13 @@ size_t size_class(size_t bytes) {
   }
   return c;
 }
+// ams_debug_refuse_allocations of this thread
+thread_local unsigned long long t_refuse_from = 0;
 cudaError_t pool_malloc(void **out, size_t bytes) {
+  if (t_refuse_from && bytes >= t_refuse_from) {
+    *out = nullptr;
+    return cudaErrorMemoryAllocation;
+  }
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
@@ -601,11 +607,20 @@ ams_status trace_impl(ams_scene *S, const ams_trace_params *p, const float *src,
       };
       // No round can list more than every path in every cell.  With memory
       // for that, rounds whose stage 2 leaves the chip mostly idle run in
-      // batches without the host looking at their counts.
+      // batches without the host looking at their counts.  Where the device has
+      // not got it, every round waits for its count.
       const unsigned long long most = (unsigned long long)ng * n_paths;
-      const bool batches = !records && most * per_task <= ((size_t)256 << 20);
+      bool batches = !records && most * per_task <= ((size_t)256 << 20);
       constexpr int kBatch = 4;
-      if (batches) CK(ensure_tasks(most, most));
+      if (batches) {
+        const cudaError_t e = ensure_tasks(most, most);
+        if (e == cudaErrorMemoryAllocation) {
+          clear_stale_error();
+          batches = false;
+        } else {
+          CK(e);
+        }
+      }
       bool listed = false;
       while (n_new > 0) {
         if (listed && trace_round_is_small(P, n_new)) {
@@ -1168,6 +1183,8 @@ ams_status ams_objective_status(const ams_objective_plan *plan, void *stream, ch
 }
 
 void ams_debug_inject_wait_timeout(int calls) { obj_inject_timeouts(calls); }
+
+void ams_debug_refuse_allocations(unsigned long long min_bytes) { t_refuse_from = min_bytes; }
 
 unsigned long long ams_scratch_bytes(void) {
   unsigned long long t = 0;

@@ -318,6 +318,11 @@ ams_status ams_objective_status(const ams_objective_plan *plan, void *stream,
  * state.  0 cancels.  Not for production use. */
 void ams_debug_inject_wait_timeout(int calls);
 
+/* Fault injection for tests: device blocks of min_bytes and more that scenes ask
+ * for on the calling thread are refused, as by a full device, on the host and
+ * without touching it.  0 ends it.  Not for production use. */
+void ams_debug_refuse_allocations(unsigned long long min_bytes);
+
 /* Received amplitude |Y| [C,R] of the same model (forward only). */
 ams_status ams_objective_recv(const float *H_d, const float *H_a,
                               const float *H_r, const float *phi,
