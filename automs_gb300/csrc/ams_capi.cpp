@@ -247,12 +247,19 @@ void clear_stale_error() { (void)cudaGetLastError(); }
 
 // The 32-wide form of the scene hierarchy for stage 2's beams.  The passes
 // that a balanced tree needs are enqueued at once, then the level counts are
-// read and any deeper level is added.  A hierarchy that does not fit the wide
-// nodes' memory goes without (stage 2 then traverses the binary nodes).
+// read and any deeper level is added.  They take 896 bytes a node, about 300 a
+// triangle (the rest of a scene 190).  A hierarchy that does not fit them, or a
+// device without that memory, goes without (stage 2 then traverses the binary
+// nodes).
 cudaError_t build_wide(ams_scene *s, cudaStream_t st) {
   const int n = s->n_tri;
   s->wide_bytes = wide_bvh_bytes(n);
   cudaError_t e = pool_malloc(reinterpret_cast<void **>(&s->wide), s->wide_bytes);
+  if (e == cudaErrorMemoryAllocation) {
+    clear_stale_error();
+    s->wide_bytes = 0;
+    return cudaSuccess;
+  }
   if (e != cudaSuccess) return e;
   int levels = 2;
   for (long long k = 32; k < n; k *= 16) levels++;
@@ -389,7 +396,7 @@ ams_status ams_scene_create(const float *tris, int n_tri, const int *mat, const 
   }
   if (n_tri > 1 && (e = build_wide(s, st)) != cudaSuccess) {
     set_err(errbuf, errlen, "wide triangle BVH build: %s", cudaGetErrorString(e));
-    return fail(e == cudaErrorMemoryAllocation ? AMS_ERR_OOM : AMS_ERR_CUDA);
+    return fail(AMS_ERR_CUDA);
   }
   s->ms_bvh_scene =
       std::chrono::duration<float, std::milli>(std::chrono::steady_clock::now() - t0).count();

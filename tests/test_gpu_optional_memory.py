@@ -63,3 +63,22 @@ def test_task_list_of_every_path_in_every_cell():
     _same(got, want)
     _same(sc.trace(src, dst, _params(3)), want)
     sc.close()
+
+
+def test_wide_nodes():
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from automs_gb300 import tracer
+    room = _room()
+    src, dst = _ends()
+    plain = tracer.Scene(*room)
+    want = plain.trace(src, dst, _params(3))
+    plain.close()
+    n = len(room[0])
+    try:
+        _refuse(896 * (n // 3 + 64))  # nothing else of this scene is as large
+        sc = tracer.Scene(*room)
+    finally:
+        _refuse(0)
+    _same(sc.trace(src, dst, _params(3)), want)
+    sc.close()
