@@ -497,6 +497,23 @@ __device__ __forceinline__ void epi_cap(const ObjArgs &a, int c, c2 y, float &am
   cap = v;
 }
 
+// s + x with the rounding error added to e (Knuth's two-sum): a loss partial of
+// many Rx is summed in FP32, where FP64 is slow, and keeps what FP64 would
+__device__ __forceinline__ void add_kept(float &s, float &e, float x) {
+  const float t = s + x, b = t - s;
+  e += (s - (t - b)) + (x - b);
+  s = t;
+}
+__device__ __forceinline__ double warp_sum_kept(float s, float e) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const float x = __shfl_xor_sync(0xffffffffu, s, o), y = __shfl_xor_sync(0xffffffffu, e, o);
+    add_kept(s, e, x);
+    e += y;
+  }
+  return (double)s + (double)e;
+}
+
 // (Phase A takes groups of 32 Rx in turn and forms its loss partial once: with
 // a CTA and an arrival per group it waited at its barriers, 28.5 us for 60 codes
 // and R = 65,536 against 22.4.)
@@ -509,7 +526,7 @@ __global__ void __launch_bounds__(256) k_tc_epi_a(ObjArgs a, int kspl, const flo
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   __shared__ float smx[2][8][32];
   __shared__ int sarg[2][8][32];
-  float sum_max = 0.f, sum_sq = 0.f;  // FP32 within a warp (FP64 is slow here), FP64 across
+  float sum_max = 0.f, sum_sq = 0.f, low_max = 0.f, low_sq = 0.f;
   const int ngroups = (a.R + 31) / 32;
   for (int grp = blockIdx.x, buf = 0; grp < ngroups; grp += gridDim.x, buf ^= 1) {
     const int r = grp * 32 + lane;
@@ -545,7 +562,7 @@ __global__ void __launch_bounds__(256) k_tc_epi_a(ObjArgs a, int kspl, const flo
     if (wid == 0 && live) {
       maxr[r] = M_;
       argr[r] = A_;
-      sum_max += M_;
+      add_kept(sum_max, low_max, M_);
     }
     float sq = 0.f;
 #pragma unroll
@@ -555,15 +572,12 @@ __global__ void __launch_bounds__(256) k_tc_epi_a(ObjArgs a, int kspl, const flo
       const float msk = (cap[j] != M_) ? cap[j] : 0.f;
       sq += msk * msk;
     }
-    sum_sq += sq;
+    add_kept(sum_sq, low_sq, sq);
   }
-  for (int o = 16; o > 0; o >>= 1) {
-    sum_max += __shfl_xor_sync(0xffffffffu, sum_max, o);
-    sum_sq += __shfl_xor_sync(0xffffffffu, sum_sq, o);
-  }
+  const double warp_max = warp_sum_kept(sum_max, low_max), warp_sq = warp_sum_kept(sum_sq, low_sq);
   __shared__ double spart[2][8];
   __shared__ bool last;
-  if (lane == 0) { spart[0][wid] = sum_max; spart[1][wid] = sum_sq; }
+  if (lane == 0) { spart[0][wid] = warp_max; spart[1][wid] = warp_sq; }
   __syncthreads();
   if (threadIdx.x == 0) {
     double x = 0, z = 0;
@@ -1308,7 +1322,7 @@ __global__ void __launch_bounds__(32 * (kNC + kLag + 1), 1)
   __shared__ __align__(16) c2 red[kBufs][NC][CB][TR];
   __shared__ __align__(16) c2 gbuf[kBufs][2 * CB][TR];
   __shared__ __align__(8) uint64_t full[8], empty[8], redf[kBufs], gf[kBufs], got[kSlots];
-  __shared__ c2 sums[kLag];
+  __shared__ double sums[kLag][2];
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const int rank = (int)blockIdx.x % sh.CL, cluster = (int)blockIdx.x / sh.CL,
             nclusters = (int)gridDim.x / sh.CL;
@@ -1363,7 +1377,7 @@ __global__ void __launch_bounds__(32 * (kNC + kLag + 1), 1)
     }
   } else if (warp >= NC) {
     // ---- G of tiles warp - NC, warp - NC + kLag, ...
-    float sum_max = 0.f, sum_sq = 0.f;  // FP32 within a warp, FP64 across warps
+    float sum_max = 0.f, sum_sq = 0.f, low_max = 0.f, low_sq = 0.f;
     const int col = lane & (TR - 1), cs = lane / TR;
     for (int it = warp - NC; it < n; it += kLag) {
       const int bi = it % kBufs, si = it % kSlots;
@@ -1407,8 +1421,8 @@ __global__ void __launch_bounds__(32 * (kNC + kLag + 1), 1)
           if (CB > 1) gbuf[bi][CB + c][col] = live ? gb[c] : c2{0.f, 0.f};
         }
         if (rank == 0 && live) {
-          sum_max += mx;
-          sum_sq += sq;
+          add_kept(sum_max, low_max, mx);
+          add_kept(sum_sq, low_sq, sq);
           if (a.recv_amp)
 #pragma unroll
             for (int c = 0; c < CB; c++)
@@ -1418,12 +1432,9 @@ __global__ void __launch_bounds__(32 * (kNC + kLag + 1), 1)
       __syncwarp();
       if (lane == 0) tc::mbar_arrive(&gf[bi]);
     }
-    for (int o = 16; o > 0; o >>= 1) {
-      sum_max += __shfl_xor_sync(0xffffffffu, sum_max, o);
-      sum_sq += __shfl_xor_sync(0xffffffffu, sum_sq, o);
-    }
+    const double x = warp_sum_kept(sum_max, low_max), z = warp_sum_kept(sum_sq, low_sq);
     // (the cluster barrier below orders the warps' sums)
-    if (lane == 0) sums[warp - NC] = {sum_max, sum_sq};
+    if (lane == 0) { sums[warp - NC][0] = x; sums[warp - NC][1] = z; }
   }
   c2 p1[RPT][CB], p2[RPT][CB];
 #pragma unroll
@@ -1564,7 +1575,7 @@ __global__ void __launch_bounds__(32 * (kNC + kLag + 1), 1)
   if (warp >= NC) {
     if (rank == 0 && t == NT) {
       double x = 0.0, z = 0.0;
-      for (int e = 0; e < kLag; e++) { x += sums[e].x; z += sums[e].y; }
+      for (int e = 0; e < kLag; e++) { x += sums[e][0]; z += sums[e][1]; }
       lpart[2 * cluster] = x;
       lpart[2 * cluster + 1] = z;
     }
