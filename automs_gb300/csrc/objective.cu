@@ -2915,13 +2915,18 @@ __global__ void __launch_bounds__(256) k_mh_gemm(const __grid_constant__ MhLevel
       }
       __syncthreads();
       if (k0 + kMhK < s.k) fetch(k0 + kMhK);  // in flight during the products
+      // what is staged is summed by itself first: one chain over all sources is
+      // longer than a path's product was
+      c2 t0 = {0.f, 0.f}, t1 = {0.f, 0.f};
 #pragma unroll 8
       for (int k = 0; k < kMhK; k++) {
         const float2 x = As[k][lane];
         const float4 b = *reinterpret_cast<const float4 *>(&Bs[k][2 * warp]);
-        mac(acc0, c2{x.x, x.y}, c2{b.x, b.y});
-        mac(acc1, c2{x.x, x.y}, c2{b.z, b.w});
+        mac(t0, c2{x.x, x.y}, c2{b.x, b.y});
+        mac(t1, c2{x.x, x.y}, c2{b.z, b.w});
       }
+      acc0.x += t0.x; acc0.y += t0.y;
+      acc1.x += t1.x; acc1.y += t1.y;
     }
   }
   const int c = c0 + lane;
