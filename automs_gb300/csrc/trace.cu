@@ -357,8 +357,8 @@ __device__ void traverse(const BvhNode *nodes, const float4 *prims, int n, const
 // finds; only the culling is shared.  Ray by ray, a query made 14 (2,172
 // triangles) to 25 dependent visits of binary nodes; a beam makes 2.6 to 6.5
 // visits of wide nodes and 4 to 5 triangle tests for 27 to 32 rays.  Stage-2
-// kernels: 3.05 -> 2.6 ms on coverage-128, 42 -> 33 ms on a 62k-triangle room
-// with 256 x 256 Rx, 90 -> 44 ms with 1,024 metasurface elements as Tx.
+// kernels: 3.1 -> 2.2 ms on coverage-128, 42 -> 25 ms on a 62k-triangle room with
+// 256 x 256 Rx, 90 -> 43 ms with 1,024 metasurface elements as Tx.
 // Bound by instruction issue (66% of the slots) and instruction fetch.
 constexpr unsigned kFullWarp = 0xffffffffu;
 
@@ -386,6 +386,7 @@ struct Beam {
   // bit 8 + k, directions of both signs (both planes bound t from below)
   unsigned flags;
   float spread;  // largest extent of the directions along an axis
+  float reach;   // largest extent of the origins along an axis
 };
 
 // rcp.approx keeps the error (1 ulp) far inside the slack of the box test;
@@ -406,6 +407,7 @@ __device__ __forceinline__ BeamAxis beam_axis(float o, float d, bool on, int axi
   if (neg) b.flags |= 1u << axis;
   if (dmin < 0.0f && dmax > 0.0f) b.flags |= 256u << axis;
   b.spread = fmaxf(b.spread, dmax - dmin);
+  b.reach = fmaxf(b.reach, omax - omin);
   a.o1 = neg ? omin : omax; a.i1 = neg ? ihi : ilo;
   a.o2 = neg ? omax : omin; a.i2 = neg ? ilo : ihi;
   return a;
@@ -415,6 +417,7 @@ __device__ __forceinline__ Beam beam_of(af3 o, af3 d, bool on) {
   Beam b;
   b.flags = 0u;
   b.spread = 0.0f;
+  b.reach = 0.0f;
   b.x = beam_axis(o.x, d.x, on, 0, b);
   b.y = beam_axis(o.y, d.y, on, 1, b);
   b.z = beam_axis(o.z, d.z, on, 2, b);
@@ -473,9 +476,18 @@ __device__ __forceinline__ float tri_hit_b(const RayB &r, const float *p) {
 // node visits + triangle tests after which a beam is given up; its lanes then
 // traverse the binary nodes one ray each
 #define AMS_BEAM_WORK 64
-// Directions further apart than this along an axis (rays that met different
-// surfaces) are taken as several beams of closer ones.
+// Directions (rays that met different surfaces) or origins (in m: neighbouring
+// Rx of a coarse grid) further apart than this along an axis are taken as several
+// beams of closer rays.  Where the rays around the one in the middle are less
+// than half of them, no few beams will do, and they traverse the binary nodes
+// one each.  38k triangles, Rx 0.5 m apart, all as beams / all one each / this
+// rule: 1 Tx 6.2 / 1.5 / 1.4 ms, 4 Tx 4.1 / 1.7 / 1.8, 16 Tx 3.8 / 2.8 / 2.0, 36
+// Tx 6.4 / 5.3 / 3.5 ms; Rx 0.1 m apart, 36 Tx 21.8 / 25.1 / 14.  A third, a
+// quarter or a sixth instead of half: few Tx up to 1.5 times as long, many Tx the
+// same; origins 0.2 or 0.5 m: within 4%, 36 Tx at 0.5 m 3.4 and 4.3 ms.
 #define AMS_BEAM_SPREAD 0.1f
+#define AMS_BEAM_REACH 0.3f
+#define AMS_BEAM_SHARE 2
 
 // Closest scene hit of every alive lane's ray, or with `any` whether there is
 // one at all before `best` (such a lane's `alive` becomes false).  Warp
@@ -561,17 +573,8 @@ __device__ __forceinline__ bool beam_scene(const TraceDev &P, const Beam &bm, co
   }
 }
 
-// whether a ray (r.inv set) meets the box of the whole Tx array, or with a
-// beam whether any of its rays may (tx_info words 8-10 and 12-14)
-__device__ __forceinline__ bool beam_near_tx(const TraceDev &P, const Beam &bm) {
-  const float4 lo = __ldg(P.tx_info + 2), hi = __ldg(P.tx_info + 3);
-  const bool nx = bm.flags & 1u, ny = bm.flags & 2u, nz = bm.flags & 4u;
-  float tn = -3.0e38f, tf = 3.0e38f;
-  beam_slab(bm.x, bm.flags & 256u, nx ? hi.x : lo.x, nx ? lo.x : hi.x, tn, tf);
-  beam_slab(bm.y, bm.flags & 512u, ny ? hi.y : lo.y, ny ? lo.y : hi.y, tn, tf);
-  beam_slab(bm.z, bm.flags & 1024u, nz ? hi.z : lo.z, nz ? lo.z : hi.z, tn, tf);
-  return beam_in(tn, tf, 3.0e38f);
-}
+// whether a ray (r.inv set) may meet the box of the whole Tx array (tx_info words
+// 8-10 and 12-14)
 __device__ __forceinline__ bool ray_near_tx(const TraceDev &P, const RayT &r) {
   const float4 lo = __ldg(P.tx_info + 2), hi = __ldg(P.tx_info + 3);
   float tn;
@@ -646,30 +649,48 @@ __device__ __forceinline__ Hit closest_s2(const TraceDev &P, af3 o, af3 d, int s
     if (others) h = traverse_tx(P, o, d, h);
     __syncwarp();
   }
-  // the rays that the scene is asked for, as beams of similar ones
-  bool ask = on && (!last || h.inst == 1), near_tx = false;
+  // the rays that the scene is asked for, as beams of close ones
+  const int lane = threadIdx.x & 31;
+  const bool ask = on && (!last || h.inst == 1);
+  bool alone = ask && P.n_tri_wide == 0;  // traverses the binary nodes by itself
   const RayB r = ray_b(o, d);
-  for (unsigned left = __ballot_sync(kFullWarp, ask); left;) {
-    bool in = (left >> (threadIdx.x & 31)) & 1u;
+  for (unsigned left = P.n_tri_wide == 0 ? 0u : __ballot_sync(kFullWarp, ask); left;) {
+    bool in = (left >> lane) & 1u;
     Beam bm = beam_of(o, d, in);
-    if (bm.spread > AMS_BEAM_SPREAD) {
-      const int lead = __ffs(left) - 1;
+    unsigned now = left;
+    if (bm.spread > AMS_BEAM_SPREAD || bm.reach > AMS_BEAM_REACH) {
+      // around the ray in the middle of them
+      const int lead = __ffs(__ballot_sync(kFullWarp, in && __popc(left & ((1u << lane) - 1u)) ==
+                                                                __popc(left) / 2)) - 1;
       const float dx = __shfl_sync(kFullWarp, d.x, lead), dy = __shfl_sync(kFullWarp, d.y, lead),
-                  dz = __shfl_sync(kFullWarp, d.z, lead);
-      in = in && (lead == (int)(threadIdx.x & 31) ||
-                  fmaxf(fmaxf(fabsf(d.x - dx), fabsf(d.y - dy)), fabsf(d.z - dz)) <
-                      0.5f * AMS_BEAM_SPREAD);
+                  dz = __shfl_sync(kFullWarp, d.z, lead), ox = __shfl_sync(kFullWarp, o.x, lead),
+                  oy = __shfl_sync(kFullWarp, o.y, lead), oz = __shfl_sync(kFullWarp, o.z, lead);
+      const bool near =
+          fmaxf(fmaxf(fabsf(d.x - dx), fabsf(d.y - dy)), fabsf(d.z - dz)) < 0.5f * AMS_BEAM_SPREAD &&
+          fmaxf(fmaxf(fabsf(o.x - ox), fabsf(o.y - oy)), fabsf(o.z - oz)) < 0.5f * AMS_BEAM_REACH;
+      now = __ballot_sync(kFullWarp, in && (near || lead == lane));
+      if (__popc(now) * AMS_BEAM_SHARE < __popc(left)) {
+        alone = alone || in;
+        break;
+      }
+      in = (now >> lane) & 1u;
       bm = beam_of(o, d, in);
     }
-    left &= ~__ballot_sync(kFullWarp, in);
-    if (!last && !near_tx) near_tx = beam_near_tx(P, bm);
+    left &= ~now;
     bool alive = in;
-    bool given_up = P.n_tri_wide == 0;
-    if (!given_up) given_up = !beam_scene(P, bm, r, h, alive, last, stk);
-    if (given_up && alive) h = traverse_scene(P, o, d, h);
+    if (!beam_scene(P, bm, r, h, alive, last, stk)) alone = alone || alive;
     __syncwarp();
   }
-  if (near_tx && on) h = traverse_tx(P, o, d, h);
+  if (alone) h = traverse_scene(P, o, d, h);
+  // (ray by ray: by the beams' bounds most rays of a loose beam seemed to pass
+  // the Tx array, and every one of them asked its hierarchy: 34 -> 25 ms)
+  if (!last && on) {
+    RayT q;
+    q.o = o;
+    q.d = d;
+    ray_setup_box(q);
+    if (ray_near_tx(P, q)) h = traverse_tx(P, o, d, h);
+  }
   __syncwarp();
   return h;
 }
@@ -1330,7 +1351,7 @@ __global__ void __launch_bounds__(128, 8) k_stage1(const __grid_constant__ Trace
 }
 
 // ------------------------------------------------------------- Tx array
-// tx_info of the Tx positions, 4 float4 (beam_near_tx, tx_alone): two
+// tx_info of the Tx positions, 4 float4 (ray_near_tx, tx_alone): two
 // directions that the array is thin along (the normal of a planar array
 // twice, two normals of a linear one), each with the sine above which a ray
 // meets one Tx only; then the box of all Tx boxes, widened as a node's.  Word
