@@ -606,13 +606,6 @@ __device__ __noinline__ Hit traverse_scene(const TraceDev &P, af3 o, af3 d, Hit 
   return h;
 }
 
-__device__ __noinline__ Hit traverse_rx(const TraceDev &P, af3 o, af3 d, Hit h) {
-  RayT r;
-  ray_setup(r, o, d);
-  traverse<2>(P.rx_nodes, P.rx_prims, P.n_dst, r, h, P.dst_r, P.err);
-  return h;
-}
-
 // Backward-ray query of stage 2 for a warp: optixTrace with the visibility
 // mask of the scene and the Tx spheres (optixPathTracer.cpp:417-424), from
 // (o, d) of the lanes with `on` towards Tx s.  On a path's last segment a
@@ -874,7 +867,7 @@ struct CurMatrix {
 // Stage 1 runs as a persistent loop per warp with dynamic fetching (after
 // Aila & Laine, "Understanding the efficiency of ray traversal on GPUs",
 // HPG 2009).  A round answers one closest-hit query of every lane: the Rx
-// spheres (by their grid, or by their hierarchy where they form none), then
+// spheres (by their grid, or by their hierarchy where they form none) and
 // the scene pruned at the sphere hit, visiting BVH nodes until every lane's
 // query has ended; then all lanes handle their hits together and set up their
 // next queries (the next segment, the next pending slot, the next sub-launch,
@@ -893,8 +886,8 @@ struct CurMatrix {
 // of 16,384); the grid needs a row or two.  Bound by instruction fetch: 12 of
 // 32 lanes are active, and short loops run rolled up (unrolled by the
 // compiler they cost 3.1 instead of 2.6 ms on coverage-128).  k_stage1:
-// coverage-128 3.84 -> 2.56 ms, 62k triangles and 256 x 256 Rx 14.8 -> 8.8 ms,
-// the same scene and a 32 x 32 metasurface as Rx 9.6 -> 4.8 ms.
+// coverage-128 3.84 -> 2.07 ms, 62k triangles and 256 x 256 Rx 14.8 -> 8.1 ms,
+// the same scene and a 32 x 32 metasurface as Rx 9.6 -> 4.7 ms.
 
 // warp-aggregated fetch of one launch index per calling lane
 __device__ __forceinline__ long long fetch_launch(unsigned long long *ctr) {
@@ -1237,8 +1230,14 @@ __device__ __forceinline__ bool s1_next(const TraceDev &P, S1Query &q, S1Ray &w,
 
 // 8 CTAs of 128 per SM (64 registers) measured fastest among 4 to 12.
 // LMAX bounds max_reflection: 2^LMAX branch slots (slot indices hold one bit
-// per hit count below L).
-template <int LMAX>
+// per hit count below L).  GRID: the instance for Rx sets that form a grid; the
+// other one visits the nodes of both hierarchies in one loop, so that a lane
+// whose Rx are done goes on with the scene while others still look for theirs
+// (64 x 64 rotated Rx: 4.3 ms, one hierarchy after the other 4.9; in a room of 60
+// triangles 2.1 and 2.4).  Without that code the grid's instance is shorter too
+// (coverage-128: 2.57 -> 2.07 ms).  Both are launched, and the one that the set is
+// not for returns at once (the set is looked at on the device).
+template <int LMAX, bool GRID>
 __global__ void __launch_bounds__(128, 8) k_stage1(const __grid_constant__ TraceDev P) {
   const long long tiles_y = (P.launch_y + 7) / 8;
   const long long n_fetch = (long long)((P.launch_x + 3) / 4) * tiles_y * 32;
@@ -1251,6 +1250,7 @@ __global__ void __launch_bounds__(128, 8) k_stage1(const __grid_constant__ Trace
   if (threadIdx.x < AMS_MAX_L + 2) s_los[threadIdx.x] = -1;
   if (threadIdx.x == 32) s_grid = rx_grid(P);
   __syncthreads();
+  if ((s_grid.ok != 0) != GRID) return;
   int rec[AMS_MAX_RESERVE];  // cell * 8 + hit_cnt of the records kept so far
   Slot slots[1 << LMAX];     // deferred branch slots
   int2 stack[AMS_STACK];     // node, its near distance
@@ -1269,24 +1269,23 @@ __global__ void __launch_bounds__(128, 8) k_stage1(const __grid_constant__ Trace
     ray_setup(q.r, q.r.o, q.r.d);
     q.Dq = unit_dir(q.r);
     q.best.t = AMS_TMAX; q.best.inst = 3; q.best.prim = 0x7fffffff;
-    // ---- Rx spheres
-    if (s_grid.ok) {
-      if (live) rx_by_grid(P, s_grid, q);
-    } else if (live) {
-      q.best = traverse_rx(P, q.r.o, q.r.d, q.best);
-    }
+    // ---- Rx spheres, then the scene, pruned at the sphere hit: node visits
+    // until every lane's query has ended
+    if (GRID && live) rx_by_grid(P, s_grid, q);
     __syncwarp();
-    // ---- scene, pruned at the sphere hit: node visits until every lane's
-    // query has ended
+    if (!GRID && live && P.n_dst == 1) test_prim<2>(P.rx_prims, 0, q.r, q.best, P.dst_r, q.Dq);
     if (live && P.n_tri == 1) test_prim<0>(P.tri_prims, 0, q.r, q.best, 0.0f, q.Dq);
-    bool trav = live && P.n_tri > 1;
+    bool rx = !GRID && P.n_dst > 1;
+    bool trav = live && (rx || P.n_tri > 1);
     int node = 0, sp = 0;
     while (trav) {
-      if ((unsigned)node >= (unsigned)(P.n_tri - 1)) {
+      const int n_prims = rx ? P.n_dst : P.n_tri;
+      const float4 *prims = rx ? P.rx_prims : P.tri_prims;
+      if ((unsigned)node >= (unsigned)(n_prims - 1)) {
         atomicOr(P.err, AMS_DERR_BVH);
         break;
       }
-      const float4 *np = reinterpret_cast<const float4 *>(P.tri_nodes + node);
+      const float4 *np = reinterpret_cast<const float4 *>((rx ? P.rx_nodes : P.tri_nodes) + node);
       const float4 a = __ldg(np), b = __ldg(np + 1), c = __ldg(np + 2);
       const int2 d = __ldg(reinterpret_cast<const int2 *>(np + 3));
       float tn0, tn1;
@@ -1297,14 +1296,16 @@ __global__ void __launch_bounds__(128, 8) k_stage1(const __grid_constant__ Trace
       const int lf1 = (h1 && d.y < 0) ? ~d.y : -1;
       if (lf0 >= 0) h0 = false;
       if (lf1 >= 0) h1 = false;
-      if (lf0 >= P.n_tri || lf1 >= P.n_tri) {
+      if (lf0 >= n_prims || lf1 >= n_prims) {
         atomicOr(P.err, AMS_DERR_BVH);
         break;
       }
 #pragma unroll 1
       for (int k = 0; k < 2; k++) {
         const int lf = k == 0 ? lf0 : lf1;
-        if (lf >= 0) test_prim<0>(P.tri_prims, lf, q.r, q.best, 0.0f, q.Dq);
+        if (lf < 0) continue;
+        if (!GRID && rx) test_prim<2>(prims, lf, q.r, q.best, P.dst_r, q.Dq);
+        else test_prim<0>(prims, lf, q.r, q.best, 0.0f, q.Dq);
       }
       if (h0 && h1) {
         const bool swap = tn1 < tn0;
@@ -1325,6 +1326,11 @@ __global__ void __launch_bounds__(128, 8) k_stage1(const __grid_constant__ Trace
         while (sp > 0) {
           const int2 e = stack[--sp];
           if (__int_as_float(e.y) <= lim) { node = e.x; trav = true; break; }
+        }
+        if (!GRID && !trav && rx) {  // the Rx are done
+          rx = false;
+          trav = P.n_tri > 1;
+          node = 0;
         }
       }
     }
@@ -1983,22 +1989,29 @@ cudaError_t trace_stage1(const TraceDev &P, cudaStream_t st) {
   long long n = (long long)P.launch_x * P.launch_y;
   // the smallest slot array that holds max_reflection's slots
   const int lk = P.L <= 2 ? 0 : (P.L == 3 ? 1 : 2);
-  void (*const kern[3])(TraceDev) = {k_stage1<2>, k_stage1<3>, k_stage1<AMS_MAX_L>};
-  static int per_sm[3][AMS_MAX_DEVICES] = {{0}};
+  void (*const kern[2][3])(TraceDev) = {
+      {k_stage1<2, false>, k_stage1<3, false>, k_stage1<AMS_MAX_L, false>},
+      {k_stage1<2, true>, k_stage1<3, true>, k_stage1<AMS_MAX_L, true>}};
+  static int per_sm[2][3][AMS_MAX_DEVICES] = {{{0}}};
   const int dev = ams_current_device();
   if (dev < 0) return cudaErrorInvalidDevice;
-  if (per_sm[lk][dev] == 0) {
-    int b = 0;
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kern[lk], 128, 0);
+  for (int g = P.n_dst > 1 ? 1 : 0; g >= 0; g--) {  // (one Rx is no grid)
+    int &ps = per_sm[g][lk][dev];
+    if (ps == 0) {
+      int b = 0;
+      cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kern[g][lk], 128, 0);
+      if (e != cudaSuccess) return e;
+      ps = b > 0 ? b : 1;
+    }
+    long long blocks = (long long)ps * ams_device_sms();
+    const long long need = (n + 127) / 128;
+    if (blocks > need) blocks = need;
+    if (blocks < 1) blocks = 1;
+    kern[g][lk]<<<(int)blocks, 128, 0, st>>>(P);
+    cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    per_sm[lk][dev] = b > 0 ? b : 1;
   }
-  long long blocks = (long long)per_sm[lk][dev] * ams_device_sms();
-  const long long need = (n + 127) / 128;
-  if (blocks > need) blocks = need;
-  if (blocks < 1) blocks = 1;
-  kern[lk]<<<(int)blocks, 128, 0, st>>>(P);
-  return cudaGetLastError();
+  return cudaSuccess;
 }
 
 namespace {
