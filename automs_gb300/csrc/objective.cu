@@ -1226,7 +1226,8 @@ __device__ __forceinline__ void cluster_wait() {
 }
 // store into CTA `rank` of the cluster; its mbarrier counts the 8 bytes (no fence
 // and no barrier on either side: a cluster barrier with its release cost about
-// 4 us a tile here)
+// 4 us a tile here).  st.async is an illegal instruction in a kernel that was
+// launched without a cluster dimension.
 __device__ __forceinline__ void cluster_store(uint32_t addr, uint32_t bar, int rank, c2 v) {
   uint32_t a, b;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
@@ -1294,7 +1295,7 @@ constexpr int kMaxClusters = 512;  // partials the scratch holds
 // tile's A: what is older than 2 kLag + 2 tiles has been read everywhere, what
 // is older than kLag + 1 in this CTA.
 constexpr int kSlots = 8, kBufs = 4;
-static_assert(kSlots >= 2 * kLag + 3 && kBufs >= kLag + 2, "buffers");
+static_assert(kSlots >= 2 * kLag + 3 && kSlots <= 8 && kBufs >= kLag + 2, "buffers");
 
 // Warps 0 .. NC - 1 compute (A and C), warps NC .. NC + kLag - 1 form G (the
 // exchange and B), the last warp copies.  The roles meet on mbarriers only, all
@@ -1334,17 +1335,22 @@ __global__ void __launch_bounds__(32 * (kNC + kLag + 1), 1)
   const int hd = (nr + sh.boxR - 1) / sh.boxR * sh.boxR;
   const int used = nd > 0 ? hd + nd : nr;  // stage rows that hold anything
   const int n = cluster < sh.ntiles ? (sh.ntiles - cluster + nclusters - 1) / nclusters : 0;
-  if (t == 0) {
-    for (int i = 0; i < sh.stages; i++) { tc::mbar_init(&full[i], 1); tc::mbar_init(&empty[i], NC); }
-    for (int i = 0; i < kBufs; i++) { tc::mbar_init(&redf[i], NC); tc::mbar_init(&gf[i], 1); }
-    for (int i = 0; i < kSlots; i++) tc::mbar_init(&got[i], 1);
+  if (t < 8) {
+    if (t < sh.stages) { tc::mbar_init(&full[t], 1); tc::mbar_init(&empty[t], NC); }
+    if (t < kBufs) { tc::mbar_init(&redf[t], NC); tc::mbar_init(&gf[t], 1); }
+    if (t < kSlots) tc::mbar_init(&got[t], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   // every CTA of the cluster runs, its barriers set, before anyone stores into
-  // its memory
+  // its memory.  A CTA alone is launched without a cluster and takes no cluster
+  // instruction: S = 4, M = 16, R = 512 12.7 -> 11.8 us, M = 64, R = 1,024 13.0 ->
+  // 12.2 (a CTA without roles per tile of 8 Rx: 11.3 and 12.0, but M = 256, R =
+  // 4,096 16.4 against 14.0)
   __syncthreads();
-  cluster_arrive();
-  cluster_wait();
+  if (sh.CL > 1) {
+    cluster_arrive();
+    cluster_wait();
+  }
 
   if (warp == NC + kLag) {
     // ---- copies
@@ -1377,12 +1383,12 @@ __global__ void __launch_bounds__(32 * (kNC + kLag + 1), 1)
     }
   } else if (warp >= NC) {
     // ---- G of tiles warp - NC, warp - NC + kLag, ...
-    float sum_max = 0.f, sum_sq = 0.f, low_max = 0.f, low_sq = 0.f;
+    double sum_max = 0.0, sum_sq = 0.0;
     const int col = lane & (TR - 1), cs = lane / TR;
     for (int it = warp - NC; it < n; it += kLag) {
       const int bi = it % kBufs, si = it % kSlots;
       if (!warp_wait(&redf[bi], (uint32_t)(it / kBufs) & 1u)) { atomicOr(err, 1u); break; }
-      if (lane == 0)
+      if (lane == 0 && sh.CL > 1)
         tc::mbar_expect_tx(&got[si], (uint32_t)(sh.CL * CB * TR * sizeof(c2)));
       __syncwarp();
       if (cs < CB) {  // the CTA's part of Y, to every CTA of the cluster
@@ -1393,12 +1399,18 @@ __global__ void __launch_bounds__(32 * (kNC + kLag + 1), 1)
         for (int h = NC / 2; h > 0; h /= 2)
 #pragma unroll
           for (int w = 0; w < h; w++) { v[w].x += v[w + h].x; v[w].y += v[w + h].y; }
-        const uint32_t at =
-            smem_addr(ybuf + ((size_t)(si * sh.CL + rank) * CB + cs) * TR + col);
-        const uint32_t bar = smem_addr(&got[si]);
-        for (int r = 0; r < sh.CL; r++) cluster_store(at, bar, r, v[0]);
+        c2 *at = ybuf + ((size_t)(si * sh.CL + rank) * CB + cs) * TR + col;
+        if (sh.CL > 1)
+          for (int r = 0; r < sh.CL; r++)
+            cluster_store(smem_addr(at), smem_addr(&got[si]), r, v[0]);
+        else
+          *at = v[0];
       }
-      if (!warp_wait(&got[si], (uint32_t)(it / kSlots) & 1u)) { atomicOr(err, 1u); break; }
+      __syncwarp();
+      if (sh.CL > 1 && !warp_wait(&got[si], (uint32_t)(it / kSlots) & 1u)) {
+        atomicOr(err, 1u);
+        break;
+      }
       const c2 *yb = ybuf + (size_t)si * sh.CL * CB * TR;
       c2 y[CB], ga[CB], gb[CB];
 #pragma unroll
@@ -1420,21 +1432,25 @@ __global__ void __launch_bounds__(32 * (kNC + kLag + 1), 1)
           gbuf[bi][c][col] = live ? ga[c] : c2{0.f, 0.f};
           if (CB > 1) gbuf[bi][CB + c][col] = live ? gb[c] : c2{0.f, 0.f};
         }
-        if (rank == 0 && live) {
-          add_kept(sum_max, low_max, mx);
-          add_kept(sum_sq, low_sq, sq);
-          if (a.recv_amp)
-#pragma unroll
-            for (int c = 0; c < CB; c++)
-              if (c < a.C) a.recv_amp[(size_t)c * a.R + r] = amp[c];
-        }
       }
       __syncwarp();
       if (lane == 0) tc::mbar_arrive(&gf[bi]);
+      // (what C does not wait for: FP64 sums cost nothing here)
+      if (rank == 0 && live && lane < TR) {
+        sum_max += (double)mx;
+        sum_sq += (double)sq;
+        if (a.recv_amp)
+#pragma unroll
+          for (int c = 0; c < CB; c++)
+            if (c < a.C) a.recv_amp[(size_t)c * a.R + r] = amp[c];
+      }
     }
-    const double x = warp_sum_kept(sum_max, low_max), z = warp_sum_kept(sum_sq, low_sq);
-    // (the cluster barrier below orders the warps' sums)
-    if (lane == 0) { sums[warp - NC][0] = x; sums[warp - NC][1] = z; }
+    for (int o = 16; o > 0; o >>= 1) {
+      sum_max += __shfl_xor_sync(0xffffffffu, sum_max, o);
+      sum_sq += __shfl_xor_sync(0xffffffffu, sum_sq, o);
+    }
+    // (the barrier below orders the warps' sums)
+    if (lane == 0) { sums[warp - NC][0] = sum_max; sums[warp - NC][1] = sum_sq; }
   }
   c2 p1[RPT][CB], p2[RPT][CB];
 #pragma unroll
@@ -1567,8 +1583,12 @@ __global__ void __launch_bounds__(32 * (kNC + kLag + 1), 1)
   }
   // no CTA leaves while another one may still store into its memory
   __syncwarp();
-  cluster_arrive();
-  cluster_wait();
+  if (sh.CL > 1) {
+    cluster_arrive();
+    cluster_wait();
+  } else {
+    __syncthreads();
+  }
   // the tail kernel may launch now; its grid-dependency wait still waits for
   // this grid to complete, with every write below visible
   cudaTriggerProgrammaticLaunchCompletion();
@@ -1727,13 +1747,12 @@ cudaError_t launch_stream_t(const ObjArgs &a, const StreamPlan &pl, const CUtens
   cfg.blockDim = dim3(32 * (kNC + kLag + 1));
   cfg.stream = st;
   cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = (unsigned)pl.sh.CL;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = (unsigned)pl.sh.CL;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
   // clusters resident at once with the most shared memory this kernel takes,
   // looked up once per device and cluster size
   static std::atomic<int> resident[AMS_MAX_DEVICES][3];
@@ -1742,6 +1761,7 @@ cudaError_t launch_stream_t(const ObjArgs &a, const StreamPlan &pl, const CUtens
   const int ci = pl.sh.CL == 1 ? 0 : pl.sh.CL == 2 ? 1 : 2;
   int most = resident[dev][ci].load();
   if (most == 0) {
+    cfg.attrs = attr + 1;
     cfg.numAttrs = 1;
     cfg.gridDim = dim3((unsigned)pl.sh.CL);
     cfg.dynamicSmemBytes = room;
@@ -1750,7 +1770,8 @@ cudaError_t launch_stream_t(const ObjArgs &a, const StreamPlan &pl, const CUtens
     resident[dev][ci].store(most);
   }
   *clusters = std::min(most, pl.sh.ntiles);
-  cfg.numAttrs = 2;
+  cfg.attrs = attr;
+  cfg.numAttrs = pl.sh.CL > 1 ? 2 : 1;
   cfg.gridDim = dim3((unsigned)(*clusters * pl.sh.CL));
   cfg.dynamicSmemBytes = pl.smem;
   return cudaLaunchKernelEx(&cfg, kfn, a, mr, md, pl.sh, U, Ppart, lpart, err);
