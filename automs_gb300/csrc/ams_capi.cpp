@@ -614,8 +614,11 @@ ams_status trace_impl(ams_scene *S, const ams_trace_params *p, const float *src,
       };
       // No round can list more than every path in every cell.  With memory
       // for that, rounds whose stage 2 leaves the chip mostly idle run in
-      // batches without the host looking at their counts.  Where the device has
-      // not got it, every round waits for its count.
+      // batches without the host looking at their counts: 4% of a trace over
+      // the range, stage 2 of coverage-128 2.77 -> 2.37 ms (two rounds a batch
+      // 2.45, eight 2.34, but small traces up to 9% longer), and with a list of
+      // 100 MB (62k triangles, 256 x 256 Rx, 99 rounds) 27.2 -> 25.9 ms.  Where
+      // the device has not got it, every round waits for its count.
       const unsigned long long most = (unsigned long long)ng * n_paths;
       bool batches = !records && most * per_task <= ((size_t)256 << 20);
       constexpr int kBatch = 4;

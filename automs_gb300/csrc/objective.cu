@@ -1297,10 +1297,6 @@ constexpr int kMaxClusters = 512;  // partials the scratch holds
 constexpr int kSlots = 8, kBufs = 4;
 static_assert(kSlots >= 2 * kLag + 3 && kSlots <= 8 && kBufs >= kLag + 2, "buffers");
 
-// Warps 0 .. NC - 1 compute (A and C), warps NC .. NC + kLag - 1 form G (the
-// exchange and B), the last warp copies.  The roles meet on mbarriers only, all
-// waits bounded; a wait that ran out ends its role, the others' waits run out
-// in turn, and the CTAs of the cluster leave together.
 // 16-byte chunk ch of row s in a stage, as the copy's swizzle places it
 template <int TR>
 __device__ __forceinline__ uint32_t tile_chunk(int s, int ch) {
@@ -1308,6 +1304,10 @@ __device__ __forceinline__ uint32_t tile_chunk(int s, int ch) {
                   : (uint32_t)s * 64u + (uint32_t)((ch ^ ((s >> 1) & 3)) << 4);
 }
 
+// Warps 0 .. NC - 1 compute (A and C), warps NC .. NC + kLag - 1 form G (the
+// exchange and B), the last warp copies.  The roles meet on mbarriers only, all
+// waits bounded; a wait that ran out ends its role, the others' waits run out
+// in turn, and the CTAs of the cluster leave together.
 template <int CB, int TR, int RPT>
 __global__ void __launch_bounds__(32 * (kNC + kLag + 1), 1)
     k_obj_stream(const __grid_constant__ ObjArgs a, const __grid_constant__ CUtensorMap mapR,
@@ -1515,7 +1515,7 @@ __global__ void __launch_bounds__(32 * (kNC + kLag + 1), 1)
       }
       if (it < kLag) continue;
       // (C) P += G conj(H) over the columns of the tile kLag before, a thread
-      // per row.  A tile is summed by itself first: a cluster sums 1/38 of the
+      // per row.  A tile is summed by itself first: a cluster sums 1/36 of the
       // Rx, and in one FP32 chain the error of dphi came to 1.1e-6 (M = 2,304,
       // R = 65,536) against 4e-7 of 152 shorter chains
       const int ct = it - kLag, bi = ct % kBufs;

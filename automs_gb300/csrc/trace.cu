@@ -359,7 +359,8 @@ __device__ void traverse(const BvhNode *nodes, const float4 *prims, int n, const
 // visits of wide nodes and 4 to 5 triangle tests for 27 to 32 rays.  Stage-2
 // kernels: 3.1 -> 2.2 ms on coverage-128, 42 -> 25 ms on a 62k-triangle room with
 // 256 x 256 Rx, 90 -> 43 ms with 1,024 metasurface elements as Tx.
-// Bound by instruction issue (66% of the slots) and instruction fetch.
+// Bound by instruction issue (70% of the slots) in large rounds, by a warp's
+// latency in small ones.
 constexpr unsigned kFullWarp = 0xffffffffu;
 
 // n / d by the multiplier of make_fast_div (Granlund and Montgomery 1994)
@@ -883,9 +884,11 @@ struct CurMatrix {
 // exactly what they see in the reference.
 //
 // Half of the node visits were spent on the Rx spheres (13 per query in a tree
-// of 16,384); the grid needs a row or two.  Bound by instruction fetch: 12 of
-// 32 lanes are active, and short loops run rolled up (unrolled by the
-// compiler they cost 3.1 instead of 2.6 ms on coverage-128).  k_stage1:
+// of 16,384); the grid needs a row or two.  Bound by the latency of dependent
+// instructions and node fetches with 14 of 32 lanes active.  Code that is not
+// in the loop any more was worth as much as fewer visits: short loops run
+// rolled up (unrolled by the compiler they cost 3.1 instead of 2.6 ms on
+// coverage-128).  k_stage1:
 // coverage-128 3.84 -> 2.07 ms, 62k triangles and 256 x 256 Rx 14.8 -> 8.1 ms,
 // the same scene and a 32 x 32 metasurface as Rx 9.6 -> 4.7 ms.
 
@@ -2031,8 +2034,8 @@ int stage2_per_sm() {
 int trace_paths_per_item(const TraceDev &P, unsigned long long n_tasks) {
   // several paths per item (fewer atomic adds) only when a round still has
   // about 32 items per resident warp with them: long items at the end of a
-  // smaller round leave the GPU idle (coverage-128's first round: 9 paths
-  // per item, 1.94 ms, against about 1.6 ms one thread per ray)
+  // smaller round leave the GPU idle.  (8 or 128 items per warp: the traces
+  // take the same time, the adds differ.)
   const unsigned long long warps = (unsigned long long)stage2_per_sm() * ams_device_sms() * 8;
   const unsigned long long pairs = (unsigned long long)(P.gs * P.gs) * P.n_src;
   const unsigned long long work = n_tasks * ((pairs + 31) / 32);

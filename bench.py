@@ -142,10 +142,10 @@ def stage1_traffic():
 def kernel_launches(stats, aabbs_given):
     """Kernels of one trace call on the headline workload, at least: the Tx
     hierarchy and the shape of the Tx array, the Rx grid and the Rx hierarchy's
-    seven, stage 1 and its count, the dense path ids and the first list, two per
+    seven, stage 1's two instances and its count, the dense path ids and the first list, two per
     round, the finalize pass (and the AABB kernels when the caller gives
     none)."""
-    n = 3 + 7 + (0 if aabbs_given else 2) + 2
+    n = 3 + 7 + (0 if aabbs_given else 2) + 3
     return n + ((3 + 2 * stats["rounds"] + 1) if stats["fwd_records"] else 0)
 
 
