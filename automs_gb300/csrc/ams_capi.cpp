@@ -479,7 +479,7 @@ ams_status trace_impl(ams_scene *S, const ams_trace_params *p, const float *src,
     need += 3 * al(4 * (size_t)ng * W);
     need += 2 * al(4 * ((size_t)ng + 1)) + al(4 * (size_t)ng) + 2 * al(4 * (size_t)tab_size);
     need += al(16 * (size_t)n_src * n_dst);
-    need += al(kCounterBytes) + al(4 * 16) + al(4 * 8);
+    need += al(kCounterBytes) + al(4 * 16) + al(4 * 9);
     need += 4096;
     CK(S->ws.ensure(need));
     S->ws.reset();
@@ -503,7 +503,7 @@ ams_status trace_impl(ams_scene *S, const ams_trace_params *p, const float *src,
     char *zero = S->ws.take<char>(0);
     char *counters = S->ws.take<char>(kCounterBytes);
     float *tx_info = S->ws.take<float>(16);
-    float *rx_grid = S->ws.take<float>(8);
+    float *rx_grid = S->ws.take<float>(9);
     P.tab_h = S->ws.take<unsigned long long>(tab_size);
     P.tab_key = S->ws.take<int32_t>(14 * (size_t)tab_size);  // 0 = word not written
     P.T = S->ws.take<unsigned>((size_t)ng * W);
@@ -521,7 +521,7 @@ ams_status trace_impl(ams_scene *S, const ams_trace_params *p, const float *src,
     Lbvh tx, rx;
     CK(lbvh_build_spheres(tx, src, src_aabb, n_src, scratch, tx_out, nullptr, st));
     CK(trace_tx_info(src, src_aabb, n_src, tx_info, st));
-    CK(trace_rx_grid(dst, dst_aabb, n0, n1, rx_grid, st));
+    CK(trace_rx_grid(dst, dst_aabb, n0, n1, p->dst_r, rx_grid, st));
     CK(lbvh_build_spheres(rx, dst, dst_aabb, n_dst, scratch, rx_out,
                           reinterpret_cast<const int *>(rx_grid) + 7, st));
     CK(cudaEventRecord(ev[1], st));

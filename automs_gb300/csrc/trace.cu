@@ -227,14 +227,15 @@ __device__ __forceinline__ bool prim_slab(const RayT &r, float4 lo, float4 hi) {
   return tn <= tf && tf >= AMS_TMIN && tn <= AMS_TMAX;
 }
 
+// square of the distance at which a ray meets a sphere
+__device__ __forceinline__ float sphere_acc(float radius) { return fmaxf(5e-5f, radius * radius); }
 // __intersection__sphere, optixPathTracer.cu:419-445; t = closest approach
 // D = d * (1 / |d|) is passed in: the same for every sphere of one query
 __device__ __forceinline__ float sphere_hit(const RayT &r, af3 D, af3 center, float radius) {
   af3 O = sub3(center, r.o);
   float b = dot3(O, D);
   float c = dot3(O, O);
-  float acc = fmaxf(5e-5f, radius * radius);
-  if ((c - b * b < acc) && b > 0.0f && sqrtf(c) > radius) {
+  if ((c - b * b < sphere_acc(radius)) && b > 0.0f && sqrtf(c) > radius) {
     if (b > AMS_TMIN && b < AMS_TMAX) return b;
   }
   return -1.0f;
@@ -918,7 +919,7 @@ struct S1Query {
 // largest deviation of an Rx from its place in the grid along u, v, w; 3-5 the
 // largest extent of a box from its Rx; 6 counts the CTAs of k_rx_grid that are
 // done, whose last one writes 7: 1 where the grid can be used (the hierarchy
-// of the Rx is not built then).
+// of the Rx is not built then); 8 is set where a box is smaller than its sphere.
 struct RxGrid {
   int ok, ua, va, wa;
   float u0, su, iu, v0, sv, iv, w0;  // steps and their inverses, 0 where there is one row
@@ -949,8 +950,14 @@ __device__ __forceinline__ RxGrid rx_grid_axes(const float *dst, int n0, int n1,
   return g;
 }
 __global__ void __launch_bounds__(256) k_rx_grid(const float *dst, const float *aabb, int n0, int n1,
-                                                 float *out) {
+                                                 float radius, float *out) {
   float du, dv;
+  // A sphere's hit lies at the ray's closest approach (sphere_hit).  Only where
+  // the box holds all of the sphere is that always inside the box, and the
+  // nearest hit the same in whichever order the spheres are looked at; with a
+  // smaller box the order of the hierarchy decides.
+  const float need = sqrtf(sphere_acc(radius));
+  bool small = false;
   const RxGrid g = rx_grid_axes(dst, n0, n1, du, dv);
   float m[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   const int ax[3] = {g.ua, g.va, g.wa};
@@ -963,7 +970,10 @@ __global__ void __launch_bounds__(256) k_rx_grid(const float *dst, const float *
       const float x = comp3(p, ax[k]);
       const float dev = fabsf(x - at[k]);
       m[k] = dev < 3.0e38f ? fmaxf(m[k], dev) : 3.0e38f;  // a NaN too
-      m[3 + k] = fmaxf(m[3 + k], fmaxf(fabsf(comp3(hi, ax[k]) - x), fabsf(x - comp3(lo, ax[k]))));
+      const float up = comp3(hi, ax[k]) - x, down = x - comp3(lo, ax[k]);
+      m[3 + k] = fmaxf(m[3 + k], fmaxf(fabsf(up), fabsf(down)));
+      // (the rounding of a box that was made of the radius)
+      small = small || !(fminf(up, down) >= need - (2e-6f + 1e-7f * fabsf(x)));
     }
   }
   for (int k = 0; k < 6; k++) {
@@ -971,6 +981,7 @@ __global__ void __launch_bounds__(256) k_rx_grid(const float *dst, const float *
     if ((threadIdx.x & 31) == 0)
       atomicMax(reinterpret_cast<int *>(out) + k, __float_as_int(v));
   }
+  if (small) reinterpret_cast<int *>(out)[8] = 1;
   __threadfence();
   __syncthreads();
   if (threadIdx.x != 0 ||
@@ -982,7 +993,8 @@ __global__ void __launch_bounds__(256) k_rx_grid(const float *dst, const float *
   // may meet any of them first)
   const bool ok = g.ok && (n0 == 1 || (du != 0.0f && m[0] <= 0.25f * fabsf(du))) &&
                   (n1 == 1 || (dv != 0.0f && m[1] <= 0.25f * fabsf(dv))) && m[2] <= m[5] &&
-                  m[3] < 1e6f && m[4] < 1e6f && m[5] < 1e6f;
+                  m[3] < 1e6f && m[4] < 1e6f && m[5] < 1e6f &&
+                  __ldcg(reinterpret_cast<const int *>(out) + 8) == 0;
   reinterpret_cast<int *>(out)[7] = ok ? 1 : 0;
 }
 __device__ __forceinline__ RxGrid rx_grid(const TraceDev &P) {
@@ -1980,9 +1992,9 @@ cudaError_t trace_tx_info(const float *src, const float *aabb, int n, float *inf
   return cudaGetLastError();
 }
 
-cudaError_t trace_rx_grid(const float *dst, const float *aabb, int n0, int n1, float *out,
-                          cudaStream_t st) {
-  k_rx_grid<<<grid_for((long long)n0 * n1, 256), 256, 0, st>>>(dst, aabb, n0, n1, out);
+cudaError_t trace_rx_grid(const float *dst, const float *aabb, int n0, int n1, float radius,
+                          float *out, cudaStream_t st) {
+  k_rx_grid<<<grid_for((long long)n0 * n1, 256), 256, 0, st>>>(dst, aabb, n0, n1, radius, out);
   return cudaGetLastError();
 }
 

@@ -109,10 +109,10 @@ cudaError_t trace_tri_attr(const float *tris, int n, float4 *attr, cudaStream_t 
 // shape of the Tx array, 16 floats (k_tx_info in trace.cu), zero before
 cudaError_t trace_tx_info(const float *src, const float *aabb, int n, float *info,
                           cudaStream_t st);
-// how the Rx set fits an axis-aligned grid, 8 words (RxGrid in trace.cu), zero
+// how the Rx set fits an axis-aligned grid, 9 words (RxGrid in trace.cu), zero
 // before; word 7 is 1 where it does
-cudaError_t trace_rx_grid(const float *dst, const float *aabb, int n0, int n1, float *out,
-                          cudaStream_t st);
+cudaError_t trace_rx_grid(const float *dst, const float *aabb, int n0, int n1, float radius,
+                          float *out, cudaStream_t st);
 cudaError_t trace_stage1(const TraceDev &P, cudaStream_t st);
 // dense path ids (dense_of [slots], P.slot_of) and the stage-1 bitmap
 // T_slots [ng][w_slots] turned into dense ids in `out` [ng][P.W], zeroed before
