@@ -641,7 +641,13 @@ __device__ __forceinline__ Hit closest_s2(const TraceDev &P, af3 o, af3 d, int s
       }
       if (h.inst != 1) others = P.n_src > 1 && ray_near_tx(P, r);
     }
-    if (others) h = traverse_tx(P, o, d, h);
+    // from the start, as a ray that meets only others: where boxes are smaller than
+    // their spheres the order of the hierarchy decides what comes first, and Tx s
+    // would hide others that lie before it
+    if (others) {
+      h.t = AMS_TMAX; h.inst = 3; h.prim = 0x7fffffff;
+      h = traverse_tx(P, o, d, h);
+    }
     __syncwarp();
   }
   // the rays that the scene is asked for, as beams of close ones
