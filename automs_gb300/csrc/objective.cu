@@ -2152,8 +2152,8 @@ __global__ void k_tc_make_ag(const float *G1, const float *G2, const float *scal
 // next, and bn is chosen so that the items fill whole rounds of the chip
 // (pick_split).
 // 60 codes, K = 1,040, R = 65,536: Y and the adjoint 124 us each with 128 x 128
-// tiles, one a CTA; 101 and 107 us now.  (Two CTAs of a cluster that shared A by
-// multicast loads took 102 and 108 us.)
+// tiles, one a CTA; 101 and 107 us now.  (Two CTAs of a cluster, each loading half
+// of A into both, took 102 and 108 us.)
 __global__ void __launch_bounds__(192, 1)
     k_cgemm3(const __grid_constant__ CUtensorMap tah, const __grid_constant__ CUtensorMap tal,
              const __grid_constant__ CUtensorMap tbh, const __grid_constant__ CUtensorMap tbl,

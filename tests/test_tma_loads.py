@@ -6,7 +6,7 @@ import re
 CSRC = os.path.join(os.path.dirname(os.path.abspath(__file__)), "..", "automs_gb300", "csrc")
 
 
-def test_no_multicast_load():
+def test_loads_have_one_destination():
     files = [f for f in sorted(os.listdir(CSRC)) if f.endswith((".cu", ".cuh", ".h", ".cpp"))]
     assert files
     for name in files:
@@ -14,4 +14,4 @@ def test_no_multicast_load():
             # the pieces of one inline instruction joined
             text = re.sub(r'"\s*"', "", f.read())
         for op in re.findall(r"cp\.async\.bulk[\w.:]*", text):
-            assert "multicast" not in op, f"{name}: {op}"
+            assert "multi" not in op, f"{name}: {op}"
